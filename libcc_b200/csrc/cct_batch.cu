@@ -116,7 +116,7 @@ __device__ void spin_until(const int *p, int target, int *err, long limit) {
   atomicExch(err, 1);
 }
 
-// Sums of one tuple's reduction partials, in the order of finalize_kernel.
+// Sums of one tuple's reduction partials, in the order of tuple_sum_kernel.
 __device__ void finalize_tuple(const TupleRec &T, const SysDev &S, int t, const BatchArgs &A, double *red) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double weight = T.kind == kIJK ? 1.0 : 0.5;
@@ -146,7 +146,7 @@ __device__ void finalize_tuple(const TupleRec &T, const SysDev &S, int t, const 
 }
 
 // One system's etd (Neumaier over its tuples in order), v1 and ets -- the
-// arithmetic of finalize_kernel and ets_kernel, in the same order.
+// arithmetic of tuple_sum_kernel, group_add_kernel and ets_kernel, in the same order.
 __device__ void system_sum(const SysDev &S, int s, const BatchArgs &A, double *red) {
   const int tid = threadIdx.x;
   const int nu = S.nu, no = S.no;
@@ -161,7 +161,7 @@ __device__ void system_sum(const SysDev &S, int s, const BatchArgs &A, double *r
     red[kBT] = sum + comp;
   }
   // thread per v1 element (a, x): the contributions of the system's tuples in
-  // order, each tuple's columns i, j, k in that order (as finalize_kernel adds them)
+  // order, each tuple's columns i, j, k in that order (as group_add_kernel adds them)
   for (int64_t e = tid; e < (int64_t)nu * no; e += kBT) {
     const int x = (int)(e / nu), a = (int)(e - (int64_t)x * nu);
     double v = 0.0;

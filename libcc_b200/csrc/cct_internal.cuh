@@ -98,7 +98,13 @@ struct TupleDev {
   const double *x[3];   // X buffers of the tuple's GEMM jobs
   int kind, i, j, k;
   double weight;        // 1 for i>j>k, 1/2 for degenerate tuples
-  int blocked = 0;      // X in 8 x 8 x 8 blocks (emulated forward), else rows of NP
+};
+// The tuples of one reduction launch, passed by value (the constant bank):
+// at most kMaxGroup consecutive tuples of the list.
+constexpr int kMaxGroup = 32;
+struct TupleGroup {
+  int n = 0;
+  TupleDev t[kMaxGroup];
 };
 // X(p,q,s) of a blocked X buffer: block (p/8, q/8, s/8) of 512 doubles at
 // ((p/8) nbk + q/8) NP/8 + s/8, element ((p%8) 8 + q%8) 8 + s%8, nbk = ceil(nu/8)
@@ -201,10 +207,15 @@ int launch_check_inputs(const Dims &d, const double *eh, const double *ep, const
 // wbuild_f64.cu
 int launch_wbuild_f64(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStream_t s);
 
-// reduce.cu
-int launch_reduce(const Dims &d, const TupleDev &t, const double *eh, const double *ep, const double *voe,
-                  const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s);
-int launch_finalize(const Dims &d, const TupleDev &t, const double *xpart, const double *vpart,
+// reduce.cu: the reductions of a group of tuples (tuple u's partials at
+// xpart + u d.ncta and vpart + u vpart_size(d)), then their sums added to the
+// accumulators in tuple order.  blocked: X in 8 x 8 x 8 blocks (emulated
+// forward), else rows of NP.  tsum: tsum_size(d) doubles per tuple of the group.
+inline int64_t vpart_size(const Dims &d) { return (int64_t)12 * d.nb * d.nb * (d.nb + 1); }
+inline int64_t tsum_size(const Dims &d) { return 1 + 3 * (int64_t)d.nu; }
+int launch_reduce(const Dims &d, const TupleGroup &g, bool blocked, const double *eh, const double *ep,
+                  const double *voe, const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s);
+int launch_finalize(const Dims &d, const TupleGroup &g, const double *xpart, const double *vpart, double *tsum,
                     double *etd_acc, double *v1_acc, cudaStream_t s);
 int launch_ets(const Dims &d, const double *t1, const double *v1_acc, const double *etd_acc, double *out3,
                cudaStream_t s);

@@ -40,8 +40,9 @@ std::vector<Tuple> tuple_list(int no) {
 
 using namespace cct;
 
-// X buffer sets: the W-build of tuple t may run while the reductions of
-// tuples t-1 .. t-kNBuf+1 are still reading theirs.
+// The forward works on groups of consecutive tuples, one W-build launch and one
+// reduction launch each, over a ring of kNBuf X buffer groups: the W build of
+// group g may run while the reductions of groups g-1 .. g-kNBuf+1 still read theirs.
 constexpr int kNBuf = 3;
 // emulated forwards store X in 8 x 8 x 8 blocks (build constant CCT_X_BLOCKED)
 #ifndef CCT_X_BLOCKED
@@ -62,21 +63,24 @@ struct ccT_plan {
   Dims d{};
   cudaStream_t stream = nullptr;      // stream the kernels run on
   cudaStream_t own_stream = nullptr;  // the plan's own stream (ordering, ets)
-  cudaStream_t gemm_stream = nullptr; // W-build GEMMs, highest priority
-  cudaStream_t red_stream = nullptr;  // reductions, lowest priority: they fill GEMM tail waves
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t gemm_stream = nullptr; // W-build GEMMs
+  cudaStream_t gemm_stream2 = nullptr; // FP64 W builds alternate between the two, so one's tail overlaps the next's start
+  cudaStream_t red_stream = nullptr;  // reductions
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_sum = nullptr;
   cudaEvent_t ev_gemm[kNBuf] = {}, ev_red[kNBuf] = {};
-  int64_t tick = 0;                   // tuples issued so far: selects the X buffer
+  int group = 1;                      // tuples per group (choose_group)
+  int nring = 1;                      // groups in the X ring (<= kNBuf)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // inputs (device copies, reference layouts)
   double *eh = nullptr, *ep = nullptr, *t1 = nullptr, *t2 = nullptr, *vm = nullptr, *voe = nullptr;
   // derived operands
   double *E = nullptr, *F = nullptr;
-  double *X[kNBuf][3] = {};  // GEMM outputs, kNBuf tuples in flight
-  double *xpart = nullptr, *vpart = nullptr;
+  double *X = nullptr;       // GEMM outputs: [nring * group tuples][3][xsize]
+  int64_t xsize = 0;         // doubles per GEMM output
+  double *xpart = nullptr, *vpart = nullptr, *tsum = nullptr;  // per tuple of a group
   int16_t *cta_table = nullptr;
   double *acc = nullptr;  // [etd_sum, etd_comp, out3[3], v1(nu*no)]
-  GemmJob *jobs = nullptr;  // [buffer][tuple][3]
+  GemmJob *jobs = nullptr;  // every tuple's jobs in list order (job_offset)
   bool emulated = false;    // INT8 split-integer W-build
   bool packed = false;      // VVVO kept packed (CCT_VVVO_PACKED): no E; vvvo_res and a slab cache instead
   double *vvvo_res = nullptr;
@@ -85,7 +89,7 @@ struct ccT_plan {
   int emu_base_ebn = 0;     // automatic plans: the N tile the kEmuMaxSlices-digit calibration operands use
   double emu_est_err = 0.0, emu_target = 0.0;  // calibrated |dE(T)| bound and its target (Eh)
   EmuOperands emu;
-  EmuJob *emu_jobs = nullptr;  // [buffer][tuple][3]
+  EmuJob *emu_jobs = nullptr;  // as jobs
   int *flags = nullptr;
   double *stage = nullptr;  // packed-slice staging for the legacy hook
   std::vector<Tuple> tuples;
@@ -108,12 +112,12 @@ struct ccT_plan {
   cudaEvent_t ev_bwdf[2] = {};
   // backward, per GX set: pointwise pass done / dE GEMM done / dF GEMM done reading it
   cudaEvent_t ev_gx_pw[kGXSets] = {}, ev_gx_e[kGXSets] = {}, ev_gx_f[kGXSets] = {};
-  cudaEvent_t ev_rec[kNBuf] = {}, ev_pw[kNBuf] = {};  // X buffer b: W rebuilt / read by the pointwise pass
+  std::vector<cudaEvent_t> ev_rec, ev_pw;  // per tuple of the X ring: W rebuilt / read by the pointwise pass
   int64_t fwd_begin = -1, fwd_end = -1;
   float last_bwd_ms = 0.f;
   // options.keep_w: the W-build output of the last forward, kept for the
   // backward ([t - keep_begin][job slot][nu^2 NP]), and the W-build jobs
-  // that write it ([t - keep_begin][3])
+  // that write it (jobs of tuple t at job_offset(t) - job_offset(keep_begin))
   double *xkeep = nullptr;
   size_t xkeep_count = 0;
   GemmJob *keep_jobs = nullptr;
@@ -164,11 +168,37 @@ int upload_emu_jobs(ccT_plan *p, const std::vector<GemmJob> &jobs, EmuJob *dst) 
   return CCT_OK;
 }
 
-// The three W-build GEMM jobs of tuple t (expanded E), writing X slots out[0..2].
-void tuple_jobs(const ccT_plan *p, const Tuple &t, double *const out[3], GemmJob J[3]) {
+int num_jobs(const Tuple &t) { return t.kind == kIJK ? 3 : 2; }
+// Position of tuple t's first job in the plan's job lists.
+int64_t job_offset(const ccT_plan *p, int64_t t) {
+  const int64_t no = p->d.no, nijk = no * (no - 1) * (no - 2) / 6;
+  return t < nijk ? 3 * t : 3 * nijk + 2 * (t - nijk);
+}
+// X buffer g of tuple t: tuple t's place in the ring of nring groups.
+double *xbuf(const ccT_plan *p, int64_t t, int g) {
+  return p->X + (t % ((int64_t)p->group * p->nring) * 3 + g) * p->xsize;
+}
+
+// Tuples per group.  A launch of a small system's tuple leaves most SMs idle:
+// group until a launch has about kGroupTiles W-build tiles (several waves of
+// the 148 SMs), within kMaxGroup tuples and kGroupBytes of X per group; a
+// tuple that has the tiles by itself stays alone (nu >= ~200, where one launch
+// a tuple and groups time the same).  A forward with one tuple a launch
+// against groups: no4-nu36 (16 tuples a group) 302 -> 109 us, no9-nu83
+// emulated (11) 6.11 -> 3.12 ms, no12-nu120 (4) 36.6 -> 34.7 ms.
+constexpr int64_t kGroupTiles = 3552;
+constexpr int64_t kGroupBytes = (int64_t)256 << 20;
+int choose_group(int64_t tiles_per_tuple, int64_t xbytes_per_tuple, int64_t ntuples) {
+  int64_t g = (kGroupTiles + tiles_per_tuple - 1) / tiles_per_tuple;
+  g = std::min(g, std::max<int64_t>(1, kGroupBytes / xbytes_per_tuple));
+  return (int)std::max<int64_t>(1, std::min({g, (int64_t)kMaxGroup, ntuples}));
+}
+
+// The W-build GEMM jobs of tuple t, writing X slots out[0..2]; Ex(x) is the
+// E slab of occupied index x.
+template <typename SlabOf>
+void tuple_jobs(const ccT_plan *p, const Tuple &t, double *const out[3], SlabOf Ex, std::vector<GemmJob> *J) {
   const Dims &d = p->d;
-  const int64_t nu2 = (int64_t)d.nu * d.nu;
-  auto Ex = [&](int x) { return p->E + (int64_t)x * nu2 * d.KP; };
   auto Fyz = [&](int y, int z) { return p->F + ((int64_t)y * d.no + z) * d.NP * d.KP; };
   auto G = [&](int x1, int x2, int x3, int slot) {
     return GemmJob{Ex(x1), Ex(x2), Fyz(x2, x3), Fyz(x1, x3), out[slot], 2, 0};
@@ -177,29 +207,27 @@ void tuple_jobs(const ccT_plan *p, const Tuple &t, double *const out[3], GemmJob
     return GemmJob{Ex(x1), Ex(x1), Fyz(x2, x3), Fyz(x2, x3), out[slot], 1, 0};
   };
   if (t.kind == kIJK) {
-    J[0] = G(t.i, t.j, t.k, 0);
-    J[1] = G(t.i, t.k, t.j, 1);
-    J[2] = G(t.j, t.k, t.i, 2);
+    J->push_back(G(t.i, t.j, t.k, 0));
+    J->push_back(G(t.i, t.k, t.j, 1));
+    J->push_back(G(t.j, t.k, t.i, 2));
   } else if (t.kind == kIJJ) {  // (i,j,j): G(i,j,j), H(j,j,i)
-    J[0] = G(t.i, t.j, t.j, 0);
-    J[1] = H(t.j, t.j, t.i, 1);
-    J[2] = H(t.j, t.j, t.i, 2);  // never launched
+    J->push_back(G(t.i, t.j, t.j, 0));
+    J->push_back(H(t.j, t.j, t.i, 1));
   } else {  // (i,i,k): H(i,i,k), G(i,k,i)
-    J[0] = H(t.i, t.i, t.k, 0);
-    J[1] = G(t.i, t.k, t.i, 1);
-    J[2] = G(t.i, t.k, t.i, 2);  // never launched
+    J->push_back(H(t.i, t.i, t.k, 0));
+    J->push_back(G(t.i, t.k, t.i, 1));
   }
 }
 
 int build_jobs(ccT_plan *p) {
   if (p->packed) return CCT_OK;  // jobs name cache slots: built per forward (packed_schedule)
-  std::vector<GemmJob> jobs(p->tuples.size() * 3 * kNBuf);
-  size_t q = 0;
-  for (int buf = 0; buf < kNBuf; buf++)
-    for (const Tuple &t : p->tuples) {
-      tuple_jobs(p, t, p->X[buf], &jobs[q]);
-      q += 3;
-    }
+  std::vector<GemmJob> jobs;
+  const int64_t nt = (int64_t)p->tuples.size(), slab = (int64_t)p->d.nu * p->d.nu * p->d.KP;
+  jobs.reserve((size_t)job_offset(p, nt));
+  for (int64_t t = 0; t < nt; t++) {
+    double *const out[3] = {xbuf(p, t, 0), xbuf(p, t, 1), xbuf(p, t, 2)};
+    tuple_jobs(p, p->tuples[t], out, [&](int x) { return p->E + x * slab; }, &jobs);
+  }
   CCT_CUDA(cudaMemcpy(p->jobs, jobs.data(), jobs.size() * sizeof(GemmJob), cudaMemcpyHostToDevice));
   if (p->emulated) CCT_TRY(upload_emu_jobs(p, jobs, p->emu_jobs));
   return CCT_OK;
@@ -210,14 +238,13 @@ int build_jobs(ccT_plan *p) {
 // the host gives every slab a tuple needs a slot; (*expand)[t - begin] lists
 // the (slot, x) expansions to issue before tuple t's W build, on the stream
 // that runs the W builds (so the W build of the tuple before has finished
-// reading the slot), and the tuple's jobs, for every X buffer, name the
-// slots.  In tuple order i > j > k a tuple usually needs one new slab.
+// reading the slot), and the tuple's jobs name the slots.  In tuple order i > j > k a tuple usually needs one new slab.
 constexpr int kSlabs = 4;
 using SlabFills = std::vector<std::vector<std::pair<int, int>>>;
 
 int packed_schedule(ccT_plan *p, int64_t begin, int64_t end, SlabFills *expand) {
   const Dims &d = p->d;
-  const int64_t nu2 = (int64_t)d.nu * d.nu, slab = nu2 * d.KP, n = end - begin, ntup = (int64_t)p->tuples.size();
+  const int64_t nu2 = (int64_t)d.nu * d.nu, slab = nu2 * d.KP, n = end - begin;
   int slot_x[kSlabs];
   int64_t last[kSlabs];
   for (int c = 0; c < kSlabs; c++) {
@@ -225,8 +252,7 @@ int packed_schedule(ccT_plan *p, int64_t begin, int64_t end, SlabFills *expand) 
     last[c] = -1;
   }
   expand->assign(n, {});
-  auto Fyz = [&](int y, int z) { return p->F + ((int64_t)y * d.no + z) * d.NP * d.KP; };
-  std::vector<GemmJob> jobs((size_t)kNBuf * n * 3);
+  std::vector<GemmJob> jobs;
   for (int64_t t = begin; t < end; t++) {
     const Tuple &tu = p->tuples[t];
     const int need[3] = {tu.i, tu.j, tu.k};
@@ -249,30 +275,11 @@ int packed_schedule(ccT_plan *p, int64_t begin, int64_t end, SlabFills *expand) 
       const int q = x == need[0] ? 0 : (x == need[1] ? 1 : 2);
       return p->slabs + slot_of[q] * slab;
     };
-    for (int buf = 0; buf < kNBuf; buf++) {
-      auto G = [&](int x1, int x2, int x3, int sl) {
-        return GemmJob{Ex(x1), Ex(x2), Fyz(x2, x3), Fyz(x1, x3), p->X[buf][sl], 2, 0};
-      };
-      auto H = [&](int x1, int x2, int x3, int sl) {
-        return GemmJob{Ex(x1), Ex(x1), Fyz(x2, x3), Fyz(x2, x3), p->X[buf][sl], 1, 0};
-      };
-      GemmJob *J = &jobs[((size_t)buf * n + (t - begin)) * 3];
-      if (tu.kind == kIJK) {
-        J[0] = G(tu.i, tu.j, tu.k, 0);
-        J[1] = G(tu.i, tu.k, tu.j, 1);
-        J[2] = G(tu.j, tu.k, tu.i, 2);
-      } else if (tu.kind == kIJJ) {
-        J[0] = G(tu.i, tu.j, tu.j, 0);
-        J[1] = J[2] = H(tu.j, tu.j, tu.i, 1);
-      } else {
-        J[0] = H(tu.i, tu.i, tu.k, 0);
-        J[1] = J[2] = G(tu.i, tu.k, tu.i, 1);
-      }
-    }
+    double *const out[3] = {xbuf(p, t, 0), xbuf(p, t, 1), xbuf(p, t, 2)};
+    tuple_jobs(p, tu, out, Ex, &jobs);
   }
-  for (int buf = 0; buf < kNBuf; buf++)
-    CCT_CUDA(cudaMemcpy(p->jobs + 3 * (buf * ntup + begin), jobs.data() + (size_t)buf * n * 3,
-                        (size_t)n * 3 * sizeof(GemmJob), cudaMemcpyHostToDevice));
+  CCT_CUDA(cudaMemcpy(p->jobs + job_offset(p, begin), jobs.data(), jobs.size() * sizeof(GemmJob),
+                      cudaMemcpyHostToDevice));
   return CCT_OK;
 }
 
@@ -344,6 +351,7 @@ int prof_collect(ccT_plan *p) {
 int fork_streams(ccT_plan *p) {
   CCT_CUDA(cudaEventRecord(p->ev_fork, p->stream));
   CCT_CUDA(cudaStreamWaitEvent(p->gemm_stream, p->ev_fork, 0));
+  CCT_CUDA(cudaStreamWaitEvent(p->gemm_stream2, p->ev_fork, 0));
   CCT_CUDA(cudaStreamWaitEvent(p->red_stream, p->ev_fork, 0));
   return CCT_OK;
 }
@@ -356,18 +364,28 @@ int join_streams(ccT_plan *p) {
   return CCT_OK;
 }
 
-// The W-build GEMMs of tuple tix into X buffer b on stream st: the plan's
-// own form, or the FP64 kernel when fp64 is set (emulated plans keep the FP64
-// jobs for the backward's recompute and the digit calibration).
+// The W-build GEMMs of tuples [t0, t1) (one X ring group) on stream st: the
+// plan's own form, or the FP64 kernel when fp64 is set (emulated plans keep
+// the FP64 jobs for the backward's recompute and the digit calibration).
 // An emulated W build stores X in 8 x 8 x 8 blocks for the reduction
 // (blocked), or in rows of NP (ccT_tuple_w, whose W assembly reads rows).
-int wbuild_tuple(ccT_plan *p, int64_t tix, int b, bool fp64, cudaStream_t st, bool blocked = kXBlocked) {
-  const Tuple &t = p->tuples[tix];
-  const int njobs = t.kind == kIJK ? 3 : 2;
-  const int64_t ntup = (int64_t)p->tuples.size();
+int wbuild_tuples(ccT_plan *p, int64_t t0, int64_t t1, bool fp64, cudaStream_t st, bool blocked = kXBlocked) {
+  const int64_t off = job_offset(p, t0);
+  const int njobs = (int)(job_offset(p, t1) - off);
   if (p->emulated && !fp64)
-    return launch_wbuild_emu(p->emu, p->d, p->emu_jobs + 3 * (b * ntup + tix), njobs, p->flags + 1, st, blocked);
-  return launch_wbuild_f64(p->d, p->jobs + 3 * (b * ntup + tix), njobs, st);
+    return launch_wbuild_emu(p->emu, p->d, p->emu_jobs + off, njobs, p->flags + 1, st, blocked);
+  return launch_wbuild_f64(p->d, p->jobs + off, njobs, st);
+}
+
+TupleDev tuple_dev(const Tuple &t, double *const X[3]) {
+  TupleDev td{};
+  for (int g = 0; g < 3; g++) td.x[g] = X[g];
+  td.kind = t.kind;
+  td.i = t.i;
+  td.j = t.j;
+  td.k = t.k;
+  td.weight = t.kind == kIJK ? 1.0 : 0.5;
+  return td;
 }
 
 // options.keep_w: room and W-build jobs for the X of tuples [begin, end)
@@ -394,18 +412,20 @@ int prepare_keep(ccT_plan *p, int64_t begin, int64_t end, bool *keep) {
     }
     p->xkeep_count = need;
   }
-  if (p->keep_jobs_count < 3 * n) {
+  const int64_t off = job_offset(p, begin), njobs = job_offset(p, end) - off;
+  if (p->keep_jobs_count < njobs) {
     if (p->keep_jobs) CCT_CUDA(cudaFree(p->keep_jobs));
     p->keep_jobs = nullptr;
     p->keep_jobs_count = 0;
-    CCT_TRY(dalloc(&p->keep_jobs, (size_t)3 * n));
-    p->keep_jobs_count = 3 * n;
+    CCT_TRY(dalloc(&p->keep_jobs, (size_t)njobs));
+    p->keep_jobs_count = njobs;
   }
-  std::vector<GemmJob> jobs((size_t)3 * n);
+  std::vector<GemmJob> jobs;
+  const int64_t eslab = (int64_t)d.nu * d.nu * d.KP;
   for (int64_t t = begin; t < end; t++) {
     double *out[3];
     for (int g = 0; g < 3; g++) out[g] = p->xkeep + ((t - begin) * 3 + g) * slab;
-    tuple_jobs(p, p->tuples[t], out, &jobs[(size_t)3 * (t - begin)]);
+    tuple_jobs(p, p->tuples[t], out, [&](int x) { return p->E + x * eslab; }, &jobs);
   }
   CCT_CUDA(cudaMemcpy(p->keep_jobs, jobs.data(), jobs.size() * sizeof(GemmJob), cudaMemcpyHostToDevice));
   *keep = true;
@@ -417,46 +437,54 @@ double *xkeep_at(const ccT_plan *p, int64_t slot, int g) {
   return p->xkeep + (slot * 3 + g) * (int64_t)p->d.nu * p->d.nu * p->d.NP;
 }
 
-// W-build of tuple tix into X buffer b on the GEMM stream, then its reduction on
-// the reduction stream.  The GEMM waits until the reduction that last read
-// buffer b (two tuples earlier) is done; the reduction waits for its GEMM.
-// keep >= 0 (an FP64 plan keeping W for the backward): the W build writes
-// the kept slot instead of buffer b.
-int run_tuple(ccT_plan *p, int64_t tix, bool fp64 = false, int64_t keep = -1) {
-  const Tuple &t = p->tuples[tix];
-  const int b = (int)(p->tick % kNBuf);
-  p->tick++;
-  CCT_CUDA(cudaStreamWaitEvent(p->gemm_stream, p->ev_red[b], 0));
-  CCT_TRY(prof_mark(p, CCT_KERNEL_WBUILD, p->gemm_stream));
-  if (keep >= 0)
-    CCT_TRY(launch_wbuild_f64(p->d, p->keep_jobs + 3 * keep, t.kind == kIJK ? 3 : 2, p->gemm_stream));
-  else
-    CCT_TRY(wbuild_tuple(p, tix, b, fp64, p->gemm_stream));
-  CCT_TRY(prof_mark(p, -1, p->gemm_stream));
-  CCT_CUDA(cudaEventRecord(p->ev_gemm[b], p->gemm_stream));
-  CCT_CUDA(cudaStreamWaitEvent(p->red_stream, p->ev_gemm[b], 0));
-  // emulated W builds fill every SM's shared memory, so the reduction cannot
-  // run beside them: it is queued on the W-build stream itself (the
-  // reduction stream then only joins).  The step takes the same time as with
-  // two streams (667-672 against 662-675 ms for 800 3-digit tuples at
-  // no24-nu320), and each kernel's launch time is then its own.
-  cudaStream_t rs = p->red_stream;
-  if (kSerialReduce && p->emulated && !fp64) rs = p->gemm_stream;
-  TupleDev td;
-  for (int g = 0; g < 3; g++) td.x[g] = keep >= 0 ? xkeep_at(p, keep, g) : p->X[b][g];
-  td.kind = t.kind;
-  td.i = t.i;
-  td.j = t.j;
-  td.k = t.k;
-  td.weight = t.kind == kIJK ? 1.0 : 0.5;
-  td.blocked = p->emulated && !fp64 && kXBlocked ? 1 : 0;
+// One group: the W builds of tuples [t0, t1) into their ring slot on a GEMM
+// stream, then their reductions on the reduction stream.  The GEMM waits until
+// the reduction that last read the slot is done; the reduction waits for its
+// GEMM.  keep >= 0 (an FP64 plan keeping W for the backward): the W builds
+// write the kept slots from keep on instead of the ring.
+int run_group(ccT_plan *p, int64_t t0, int64_t t1, bool fp64 = false, int64_t keep = -1) {
+  const int64_t grp = t0 / p->group;
+  const int slot = (int)(grp % p->nring);
+  // Emulated W builds fill every SM's shared memory, so neither the reduction
+  // nor the next W build can run beside them: both are queued on one stream
+  // (two streams and one took 662-675 and 667-672 ms for 800 3-digit tuples at
+  // no24-nu320).  The sums of a group's partials need little of an SM and run
+  // on the reduction stream under the next group's W build.  Packed plans refill the slab cache in W-build
+  // order, and profiled launches should not overlap: one GEMM stream too.
+  const bool emu = p->emulated && !fp64;
+  cudaStream_t gs = emu || p->packed || p->profiling || (grp & 1) == 0 ? p->gemm_stream : p->gemm_stream2;
+  cudaStream_t rs = kSerialReduce && emu ? gs : p->red_stream;
+  CCT_CUDA(cudaStreamWaitEvent(gs, p->ev_red[slot], 0));
+  CCT_TRY(prof_mark(p, CCT_KERNEL_WBUILD, gs));
+  if (keep >= 0) {
+    const int64_t j0 = job_offset(p, t0 - keep), j = job_offset(p, t0);  // t0 - keep: the first kept tuple
+    CCT_TRY(launch_wbuild_f64(p->d, p->keep_jobs + (j - j0), (int)(job_offset(p, t1) - j), gs));
+  } else {
+    CCT_TRY(wbuild_tuples(p, t0, t1, fp64, gs));
+  }
+  CCT_TRY(prof_mark(p, -1, gs));
+  if (rs != gs) {
+    CCT_CUDA(cudaEventRecord(p->ev_gemm[slot], gs));
+    CCT_CUDA(cudaStreamWaitEvent(rs, p->ev_gemm[slot], 0));
+  }
+  TupleGroup g;
+  g.n = (int)(t1 - t0);
+  for (int64_t t = t0; t < t1; t++) {
+    double *X[3];
+    for (int q = 0; q < 3; q++) X[q] = keep >= 0 ? xkeep_at(p, keep + (t - t0), q) : xbuf(p, t, q);
+    g.t[t - t0] = tuple_dev(p->tuples[t], X);
+  }
   CCT_TRY(prof_mark(p, CCT_KERNEL_REDUCE, rs));
-  CCT_TRY(launch_reduce(p->d, td, p->eh, p->ep, p->voe, p->cta_table, p->xpart, p->vpart, rs));
-  CCT_TRY(launch_finalize(p->d, td, p->xpart, p->vpart, p->acc, v1_acc(p), rs));
+  if (rs != p->red_stream) CCT_CUDA(cudaStreamWaitEvent(rs, p->ev_sum, 0));  // the partials of the group before are summed
+  CCT_TRY(launch_reduce(p->d, g, emu && kXBlocked, p->eh, p->ep, p->voe, p->cta_table, p->xpart, p->vpart, rs));
+  CCT_CUDA(cudaEventRecord(p->ev_red[slot], rs));
+  cudaStream_t fs = p->profiling ? rs : p->red_stream;
+  if (rs != fs) CCT_CUDA(cudaStreamWaitEvent(fs, p->ev_red[slot], 0));
+  CCT_TRY(launch_finalize(p->d, g, p->xpart, p->vpart, p->tsum, p->acc, v1_acc(p), fs));
   CCT_TRY(prof_mark(p, -1, rs));
-  CCT_CUDA(cudaEventRecord(p->ev_red[b], rs));
-  if (rs != p->red_stream) CCT_CUDA(cudaStreamWaitEvent(p->red_stream, p->ev_red[b], 0));
-  p->last_launches += 3;
+  CCT_CUDA(cudaEventRecord(p->ev_sum, fs));
+  if (fs != p->red_stream) CCT_CUDA(cudaStreamWaitEvent(p->red_stream, p->ev_sum, 0));
+  p->last_launches += 4;
   return CCT_OK;
 }
 
@@ -467,7 +495,7 @@ int tuple_energy(ccT_plan *p, int64_t tix, bool fp64, double *e) {
   CCT_CUDA(cudaMemsetAsync(p->acc, 0, (5 + (int64_t)d.nu * d.no) * 8, p->stream));
   CCT_CUDA(cudaMemsetAsync(p->flags + 1, 0, 4, p->stream));
   CCT_TRY(fork_streams(p));
-  CCT_TRY(run_tuple(p, tix, fp64));
+  CCT_TRY(run_group(p, tix, tix + 1, fp64));
   CCT_TRY(join_streams(p));
   CCT_TRY(launch_ets(d, p->t1, v1_acc(p), p->acc, p->acc + 2, p->stream));
   double out3[3];
@@ -649,7 +677,11 @@ int64_t ccT_num_tuples(int64_t no) {
   return no * (no - 1) * (no - 2) / 6 + no * (no - 1);
 }
 
-int ccT_plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *opt) {
+}  // extern "C"
+
+// ccT_plan_create; group_cap bounds the tuples per group (the legacy driver
+// hook hands tuples over one at a time, in any order).
+static int plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *opt, int group_cap) {
   if (!out) {
     set_error("plan pointer is NULL");
     return CCT_ERR_INVALID;
@@ -743,31 +775,38 @@ int ccT_plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *o
   if (cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest) != cudaSuccess) return fail(CCT_ERR_CUDA);
   if (cudaStreamCreateWithFlags(&p->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithPriority(&p->gemm_stream, cudaStreamNonBlocking, prio_greatest) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&p->gemm_stream2, cudaStreamNonBlocking, prio_greatest) != cudaSuccess ||
       cudaStreamCreateWithPriority(&p->red_stream, cudaStreamNonBlocking, prio_greatest) != cudaSuccess)
     return fail(CCT_ERR_CUDA);
   p->stream = p->own_stream;
-  for (cudaEvent_t *e : {&p->ev_fork, &p->ev_join})
+  for (cudaEvent_t *e : {&p->ev_fork, &p->ev_join, &p->ev_sum})
     if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return fail(CCT_ERR_CUDA);
   for (int b = 0; b < kNBuf; b++)
     if (cudaEventCreateWithFlags(&p->ev_gemm[b], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&p->ev_red[b], cudaEventDisableTiming) != cudaSuccess)
       return fail(CCT_ERR_CUDA);
   if (cudaEventCreate(&p->ev0) != cudaSuccess || cudaEventCreate(&p->ev1) != cudaSuccess) return fail(CCT_ERR_CUDA);
-  const int64_t nu2 = nu * nu;
+  const int64_t nu2 = nu * nu, ntup = (int64_t)p->tuples.size();
+  p->xsize = (p->emulated && kXBlocked ? round_up(nu, kRB) * round_up(nu, kRB) : nu2) * d.NP;
+  {
+    const int64_t bm = p->emulated ? kEmuBM : 128, bn = p->emulated ? d.EBN : d.BN;
+    // packed plans: a group could need more slabs than the cache holds
+    p->group = p->packed ? 1 : choose_group(3 * ((nu2 + bm - 1) / bm) * (d.NP / bn), 3 * p->xsize * 8, ntup);
+    p->group = std::min(p->group, group_cap);
+    p->nring = (int)std::min<int64_t>(kNBuf, (ntup + p->group - 1) / p->group);
+  }
   if ((s = dalloc(&p->eh, no)) || (s = dalloc(&p->ep, nu)) || (s = dalloc(&p->t1, no * nu)) ||
       (s = dalloc(&p->t2, nu2 * no * no)) || (s = dalloc(&p->vm, no * nu * no * no)) ||
       (s = dalloc(&p->voe, nu2 * no * no)) ||
       (s = p->packed ? dalloc(&p->vvvo_res, nu * (nu + 1) / 2 * nu * no) : dalloc(&p->E, no * nu2 * d.KP)) ||
       (s = p->packed ? dalloc(&p->slabs, kSlabs * nu2 * d.KP) : CCT_OK) ||
       (s = dalloc(&p->F, no * no * d.NP * d.KP)) ||
-      (s = dalloc(&p->xpart, d.ncta)) || (s = dalloc(&p->vpart, (int64_t)12 * d.nb * d.nb * (d.nb + 1))) ||
+      (s = dalloc(&p->X, (int64_t)p->group * p->nring * 3 * p->xsize)) ||
+      (s = dalloc(&p->xpart, p->group * d.ncta)) || (s = dalloc(&p->vpart, p->group * vpart_size(d))) ||
+      (s = dalloc(&p->tsum, p->group * tsum_size(d))) ||
       (s = dalloc(&p->cta_table, d.ncta * 3)) || (s = dalloc(&p->acc, 5 + nu * no)) ||
-      (s = dalloc(&p->jobs, p->tuples.size() * 3 * kNBuf)) || (s = dalloc(&p->flags, 4)))
+      (s = dalloc(&p->jobs, job_offset(p, ntup))) || (s = dalloc(&p->flags, 4)))
     return fail(s);
-  for (int b = 0; b < kNBuf; b++)
-    for (int g = 0; g < 3; g++)
-      if ((s = dalloc(&p->X[b][g], (p->emulated && kXBlocked ? round_up(nu, kRB) * round_up(nu, kRB) : nu2) * d.NP)))
-        return fail(s);
   if (p->emulated) {
     EmuOperands &e = p->emu;
     e.slices = o.emu_slices ? o.emu_slices : kEmuMaxSlices;
@@ -784,7 +823,7 @@ int ccT_plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *o
     if ((s = dalloc(&e.E8, bytesE)) || (s = dalloc(&e.E8T, bytesE)) ||
         (s = dalloc(&e.F8, e.slices * rowsF * e.KP8)) || (s = dalloc(&e.expE, rowsE)) ||
         (s = dalloc(&e.expET, rowsE)) || (s = dalloc(&e.expF, rowsF)) || (s = dalloc(&e.expRowF, rowsF)) ||
-        (s = dalloc(&p->emu_jobs, p->tuples.size() * 3 * kNBuf)) ||
+        (s = dalloc(&p->emu_jobs, job_offset(p, ntup))) ||
         (s = dalloc(&e.tileExp, e.tiles_m + no * (d.NP / d.EBN) + 2)) ||
         (s = dalloc(&e.slice_hist, kEmuMaxSlices + 1)))
       return fail(s);
@@ -805,6 +844,12 @@ int ccT_plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *o
   p->e_built.assign(no, 0);
   *out = p;
   return CCT_OK;
+}
+
+extern "C" {
+
+int ccT_plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *opt) {
+  return plan_create(out, no, nu, opt, kMaxGroup);
 }
 
 int ccT_set_inputs(ccT_plan *p, const double *eh, const double *ep, const double *t1, const double *t2,
@@ -929,9 +974,11 @@ int ccT_forward(ccT_plan *p, int64_t begin, int64_t end, double *ets, double *et
   SlabFills fills;
   if (p->packed) CCT_TRY(packed_schedule(p, begin, end, &fills));
   CCT_TRY(fork_streams(p));
-  for (int64_t t = begin; t < end; t++) {
+  for (int64_t t = begin; t < end;) {  // ring groups are aligned to the tuple list; profiled launches are per tuple
+    const int64_t e = p->profiling ? t + 1 : std::min(end, (t / p->group + 1) * p->group);
     if (p->packed) CCT_TRY(packed_fill(p, fills[t - begin], p->gemm_stream));
-    CCT_TRY(run_tuple(p, t, false, keep ? t - begin : -1));
+    CCT_TRY(run_group(p, t, e, false, keep ? t - begin : -1));
+    t = e;
   }
   CCT_TRY(join_streams(p));
   CCT_TRY(launch_ets(d, p->t1, v1_acc(p), p->acc, p->acc + 2, p->stream));
@@ -1014,17 +1061,17 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
     for (int g = 0; g < kGXSets; g++)
       for (cudaEvent_t *e : {&p->ev_gx_pw[g], &p->ev_gx_e[g], &p->ev_gx_f[g]})
         CCT_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-    for (int b = 0; b < kNBuf; b++) {
-      CCT_CUDA(cudaEventCreateWithFlags(&p->ev_rec[b], cudaEventDisableTiming));
-      CCT_CUDA(cudaEventCreateWithFlags(&p->ev_pw[b], cudaEventDisableTiming));
+    for (std::vector<cudaEvent_t> *v : {&p->ev_rec, &p->ev_pw}) {
+      v->assign((size_t)p->group * p->nring, nullptr);
+      for (cudaEvent_t &e : *v) CCT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
   }
-  const int64_t ntup = (int64_t)p->tuples.size();
+  const int64_t ring = (int64_t)p->group * p->nring;  // X buffers in flight, one tuple each
   CCT_CUDA(cudaEventRecord(p->ev0, p->stream));
   CCT_TRY(adj_zero(d, &p->adj, p->stream));
   // dT1 = 2 v1: an emulated plan's v1 is rebuilt from the FP64 W of this pass
   if (p->emulated) CCT_CUDA(cudaMemsetAsync(p->adj.v1, 0, (5 + (size_t)d.nu * d.no) * 8, p->stream));
-  // Four streams.  rec_stream rebuilds W of tuple t into X buffer t mod 3,
+  // Four streams.  rec_stream rebuilds W of tuple t into its X ring buffer,
   // ahead of red_stream, which runs the pointwise adjoint kernels of tuple t
   // (dE/dW, dVOE, deps and dE/dX into GX set t mod 4); bwd_stream then runs
   // the dF GEMM of tuple t, and gemm_stream one dE GEMM for each pair of
@@ -1044,16 +1091,16 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
   for (int64_t t = begin; t < end; t++) {
     const Tuple &tu = p->tuples[t];
     const int set = (int)((t - begin) % kGXSets);
-    const int xb = (int)((t - begin) % kNBuf);
+    const int xb = (int)(t % ring);
     double *Xk[3] = {nullptr, nullptr, nullptr};
     if (kept) {
       for (int g = 0; g < 3; g++) Xk[g] = xkeep_at(p, t - begin, g);
     } else {
-      if (t - begin >= kNBuf) CCT_CUDA(cudaStreamWaitEvent(sW, p->ev_pw[xb], 0));  // X buffer read by t-3
-      CCT_TRY(launch_wbuild_f64(d, p->jobs + 3 * ((int64_t)xb * ntup + t), tu.kind == kIJK ? 3 : 2, sW));
+      if (t - begin >= ring) CCT_CUDA(cudaStreamWaitEvent(sW, p->ev_pw[xb], 0));  // X buffer read by t - ring
+      CCT_TRY(launch_wbuild_f64(d, p->jobs + job_offset(p, t), num_jobs(tu), sW));
       CCT_CUDA(cudaEventRecord(p->ev_rec[xb], sW));
       CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_rec[xb], 0));
-      for (int g = 0; g < 3; g++) Xk[g] = p->X[xb][g];
+      for (int g = 0; g < 3; g++) Xk[g] = xbuf(p, t, g);
     }
     if (t - begin >= kGXSets) {  // GX set last read by the GEMMs of tuple t - kGXSets
       CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_gx_e[set], 0));
@@ -1061,17 +1108,11 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
     }
     CCT_TRY(adj_tuple_pointwise(d, tu, Xk, p->eh, p->ep, p->t1, p->voe, &p->adj, set, sP));
     if (p->emulated) {
-      TupleDev td;
-      td.x[0] = Xk[0];
-      td.x[1] = Xk[1];
-      td.x[2] = Xk[2];
-      td.kind = tu.kind;
-      td.i = tu.i;
-      td.j = tu.j;
-      td.k = tu.k;
-      td.weight = tu.kind == kIJK ? 1.0 : 0.5;
-      CCT_TRY(launch_reduce(d, td, p->eh, p->ep, p->voe, p->cta_table, p->xpart, p->vpart, sP));
-      CCT_TRY(launch_finalize(d, td, p->xpart, p->vpart, p->adj.v1, p->adj.v1 + 5, sP));
+      TupleGroup g;
+      g.n = 1;
+      g.t[0] = tuple_dev(tu, Xk);
+      CCT_TRY(launch_reduce(d, g, false, p->eh, p->ep, p->voe, p->cta_table, p->xpart, p->vpart, sP));
+      CCT_TRY(launch_finalize(d, g, p->xpart, p->vpart, p->tsum, p->adj.v1, p->adj.v1 + 5, sP));
     }
     CCT_CUDA(cudaEventRecord(p->ev_pw[xb], sP));
     CCT_CUDA(cudaEventRecord(p->ev_gx_pw[set], sP));
@@ -1174,8 +1215,9 @@ int ccT_tuple_w(ccT_plan *p, int64_t tuple, double *w, int32_t mem) {
   DeviceGuard guard(p->device);
   CCT_TRY(adj_configure(p->device));
   const int64_t n3 = (int64_t)p->d.nu * p->d.nu * p->d.nu;
-  // X buffer set 0 and the plan's stream, after everything already issued
+  // the tuple's X buffers and the plan's stream, after everything already issued
   CCT_CUDA(cudaStreamSynchronize(p->gemm_stream));
+  CCT_CUDA(cudaStreamSynchronize(p->gemm_stream2));
   CCT_CUDA(cudaStreamSynchronize(p->red_stream));
   double *wc = nullptr, *wf = nullptr;
   CCT_CUDA(cudaMalloc(reinterpret_cast<void **>(&wc), n3 * 8));
@@ -1195,8 +1237,9 @@ int ccT_tuple_w(ccT_plan *p, int64_t tuple, double *w, int32_t mem) {
     s = packed_schedule(p, tuple, tuple + 1, &fills);
     if (s == CCT_OK) s = packed_fill(p, fills[0], p->stream);
   }
-  if (s == CCT_OK) s = wbuild_tuple(p, tuple, 0, false, p->stream, false);  // rows of NP, as the assembly reads
-  if (s == CCT_OK) s = assemble_w_fortran(p->d, p->tuples[tuple], p->X[0], wc, wf, p->stream);
+  double *const X[3] = {xbuf(p, tuple, 0), xbuf(p, tuple, 1), xbuf(p, tuple, 2)};
+  if (s == CCT_OK) s = wbuild_tuples(p, tuple, tuple + 1, false, p->stream, false);  // rows of NP, as the assembly reads
+  if (s == CCT_OK) s = assemble_w_fortran(p->d, p->tuples[tuple], X, wc, wf, p->stream);
   int werr = 0;
   if (s == CCT_OK && cudaMemcpyAsync(&werr, p->flags + 1, 4, cudaMemcpyDeviceToHost, p->stream) != cudaSuccess)
     s = CCT_ERR_CUDA;
@@ -1239,24 +1282,20 @@ int ccT_time_wbuild(ccT_plan *p, int64_t tuple, int32_t reps, double *ms_per_lau
     return CCT_ERR_INVALID;
   }
   DeviceGuard guard(p->device);
-  const int njobs = p->tuples[tuple].kind == kIJK ? 3 : 2;
+  const int slot = (int)(tuple / p->group % p->nring);
   CCT_TRY(fork_streams(p));
-  CCT_CUDA(cudaStreamWaitEvent(p->gemm_stream, p->ev_red[0], 0));
+  CCT_CUDA(cudaStreamWaitEvent(p->gemm_stream, p->ev_red[slot], 0));
   if (p->packed) {  // the tuple's slabs into the cache (not timed)
     SlabFills fills;
     CCT_TRY(packed_schedule(p, tuple, tuple + 1, &fills));
     CCT_TRY(packed_fill(p, fills[0], p->gemm_stream));
   }
-  auto launch = [&]() {
-    return p->emulated ? launch_wbuild_emu(p->emu, p->d, p->emu_jobs + 3 * tuple, njobs, p->flags + 1, p->gemm_stream,
-                                           kXBlocked)
-                       : launch_wbuild_f64(p->d, p->jobs + 3 * tuple, njobs, p->gemm_stream);
-  };
+  auto launch = [&]() { return wbuild_tuples(p, tuple, tuple + 1, false, p->gemm_stream); };
   CCT_TRY(launch());  // warm
   CCT_CUDA(cudaEventRecord(p->ev0, p->gemm_stream));
   for (int r = 0; r < reps; r++) CCT_TRY(launch());
   CCT_CUDA(cudaEventRecord(p->ev1, p->gemm_stream));
-  CCT_CUDA(cudaEventRecord(p->ev_red[0], p->gemm_stream));  // later writers of buffer 0 follow these
+  CCT_CUDA(cudaEventRecord(p->ev_red[slot], p->gemm_stream));  // later writers of the buffer follow these
   CCT_CUDA(cudaEventSynchronize(p->ev1));
   float ms = 0.f;
   CCT_CUDA(cudaEventElapsedTime(&ms, p->ev0, p->ev1));
@@ -1290,15 +1329,12 @@ int64_t ccT_last_forward_launches(const ccT_plan *p) { return p ? p->last_launch
 int ccT_plan_destroy(ccT_plan *p) {
   if (!p) return CCT_OK;
   DeviceGuard guard(p->device);
-  for (cudaStream_t st : {p->stream, p->gemm_stream, p->red_stream, p->bwd_stream, p->rec_stream})
+  for (cudaStream_t st : {p->stream, p->gemm_stream, p->gemm_stream2, p->red_stream, p->bwd_stream, p->rec_stream})
     if (st) cudaStreamSynchronize(st);
   double *bufs[] = {p->eh, p->ep, p->t1, p->t2, p->vm, p->voe, p->E, p->F, p->xpart, p->vpart, p->acc, p->stage,
-                    p->vvvo_res, p->slabs};
+                    p->vvvo_res, p->slabs, p->X, p->tsum};
   for (double *b : bufs)
     if (b) cudaFree(b);
-  for (int b = 0; b < kNBuf; b++)
-    for (int g = 0; g < 3; g++)
-      if (p->X[b][g]) cudaFree(p->X[b][g]);
   if (p->cta_table) cudaFree(p->cta_table);
   if (p->jobs) cudaFree(p->jobs);
   if (p->xkeep) cudaFree(p->xkeep);
@@ -1312,22 +1348,22 @@ int ccT_plan_destroy(ccT_plan *p) {
   if (p->ev0) cudaEventDestroy(p->ev0);
   if (p->ev1) cudaEventDestroy(p->ev1);
   for (cudaEvent_t e : p->prof_events) cudaEventDestroy(e);
-  for (cudaEvent_t e : {p->ev_fork, p->ev_join})
+  for (cudaEvent_t e : {p->ev_fork, p->ev_join, p->ev_sum})
     if (e) cudaEventDestroy(e);
   for (int b = 0; b < kNBuf; b++) {
     if (p->ev_gemm[b]) cudaEventDestroy(p->ev_gemm[b]);
     if (p->ev_red[b]) cudaEventDestroy(p->ev_red[b]);
   }
   if (p->gemm_stream) cudaStreamDestroy(p->gemm_stream);
+  if (p->gemm_stream2) cudaStreamDestroy(p->gemm_stream2);
   if (p->bwd_stream) cudaStreamDestroy(p->bwd_stream);
   if (p->rec_stream) cudaStreamDestroy(p->rec_stream);
   if (p->pw_stream) cudaStreamDestroy(p->pw_stream);
   for (cudaEvent_t e : p->ev_bwdf)
     if (e) cudaEventDestroy(e);
-  for (int b = 0; b < kNBuf; b++) {
-    if (p->ev_rec[b]) cudaEventDestroy(p->ev_rec[b]);
-    if (p->ev_pw[b]) cudaEventDestroy(p->ev_pw[b]);
-  }
+  for (std::vector<cudaEvent_t> *v : {&p->ev_rec, &p->ev_pw})
+    for (cudaEvent_t e : *v)
+      if (e) cudaEventDestroy(e);
   for (int g = 0; g < kGXSets; g++)
     for (cudaEvent_t e : {p->ev_gx_pw[g], p->ev_gx_e[g], p->ev_gx_f[g]})
       if (e) cudaEventDestroy(e);
@@ -1358,7 +1394,7 @@ void ijk_gpu_init_(const int64_t *no, const int64_t *nu, const double *eh, const
   ccT_options o;
   ccT_options_default(&o);
   o.vvvo_mode = CCT_VVVO_EXPANDED;  // the driver hook expands each packed slice into E
-  int s = ccT_plan_create(&p, *no, *nu, &o);
+  int s = plan_create(&p, *no, *nu, &o, 1);
   if (s) legacy_stop("ijk_gpu_init", s);
   DeviceGuard guard(p->device);
   const int64_t n_o = *no, n_u = *nu, nu2 = n_u * n_u;
@@ -1412,7 +1448,7 @@ void ijk_gpu_driver_(const int64_t *nu, const int64_t *no, const int64_t *i, con
   // index of (I,J,K) in the tuple list: DDCC_T_TASK order
   const int64_t tix = I * (I - 1) * (I - 2) / 6 + J * (J - 1) / 2 + K;
   int s = fork_streams(p);
-  if (!s) s = run_tuple(p, tix);
+  if (!s) s = run_group(p, tix, tix + 1);
   if (s) legacy_stop("ijk_gpu_driver", s);
 }
 

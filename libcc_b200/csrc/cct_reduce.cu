@@ -15,7 +15,7 @@
 // unordered triple of 8-wide index blocks {A<=B<=C}, assembles W on every
 // distinct ordered block of its orbit in shared memory, and evaluates every
 // element of those blocks once.  Per-CTA partials are summed by
-// finalize_kernel in a fixed order, so results are bitwise reproducible.
+// tuple_sum_kernel and group_add_kernel in a fixed order, so results are bitwise reproducible.
 #include "cct_internal.cuh"
 #include "cct_reduce_block.cuh"
 
@@ -24,36 +24,52 @@ namespace {
 
 using namespace red;
 
-template <int KIND, bool BLOCKED>
-__global__ void __launch_bounds__(RT, 4) reduce_kernel(int nu, int no, int64_t NP, TupleDev t,
+// Grid (block triple, tuple of the group); a group may mix tuple kinds, the
+// branch is uniform over a CTA.
+template <bool BLOCKED>
+__global__ void __launch_bounds__(RT, 4) reduce_kernel(int nu, int no, int64_t NP, int64_t vsize,
+                                                      const __grid_constant__ TupleGroup grp,
                                                       const double *__restrict__ eh, const double *__restrict__ ep,
                                                       const double *__restrict__ voe,
                                                       const int16_t *__restrict__ table, double *__restrict__ xpart,
                                                       double *__restrict__ vpart) {
   extern __shared__ __align__(16) double dyn_smem[];
   const int64_t cta = blockIdx.x;
-  reduce_block<KIND, false, BLOCKED>(nu, no, NP, t, eh, ep, voe, table[3 * cta], table[3 * cta + 1], table[3 * cta + 2],
-                     xpart + cta, vpart, dyn_smem);
+  const int u = blockIdx.y;
+  const TupleDev &t = grp.t[u];
+  const int S0 = table[3 * cta], S1 = table[3 * cta + 1], S2 = table[3 * cta + 2];
+  double *xp = xpart + (int64_t)u * gridDim.x + cta, *vp = vpart + u * vsize;
+  if (t.kind == kIJK)
+    reduce_block<kIJK, false, BLOCKED>(nu, no, NP, t, eh, ep, voe, S0, S1, S2, xp, vp, dyn_smem);
+  else if (t.kind == kIJJ)
+    reduce_block<kIJJ, false, BLOCKED>(nu, no, NP, t, eh, ep, voe, S0, S1, S2, xp, vp, dyn_smem);
+  else
+    reduce_block<kIIJ, false, BLOCKED>(nu, no, NP, t, eh, ep, voe, S0, S1, S2, xp, vp, dyn_smem);
 }
 
-// etd_acc[0..1]: Neumaier (sum, compensation); v1_acc(nu, no).
-// Block 0 sums the per-CTA x3 partials (thread t takes partials t, t+256, ...
-// in order, then a tree over the 256 threads); every other block owns kFinA
-// virtual indices a, one warp per (a, column), each summing the column's v1
-// partials over all block triples containing a (lane-strided, then a shuffle
-// tree), and one thread per a adds the three column sums to v1 in the order
-// i, j, k.  The loads of a thread's partials are issued eight at a time ahead
-// of its (ordered) adds.
-constexpr int kFinA = 8;
+// Sums of one tuple's partials, weighted: tsum[0] = its E[4], then the v1
+// columns of i, j and k (nu each).  Grid (1 + ceil(nu / kFinA), tuple of the
+// group).  Block 0 sums the per-CTA x3 partials (thread t takes partials t,
+// t+256, ... in order, then a tree over the 256 threads); every other block
+// owns kFinA virtual indices a, one warp per (a, column), each summing the
+// column's v1 partials over all block triples containing a (lane-strided,
+// then a shuffle tree).  The loads of a thread's partials are issued eight at
+// a time ahead of its (ordered) adds.
+// Four virtual indices: 384 threads at 36 registers fit beside a CTA of the
+// emulated W build (576 threads at 80), under which these sums run.
+constexpr int kFinA = 4;
 constexpr int kFinThreads = 32 * 3 * kFinA;
-__global__ void __launch_bounds__(kFinThreads) finalize_kernel(int nu, int nb, int64_t ncta, TupleDev t,
-                                                               const double *__restrict__ xpart,
-                                                               const double *__restrict__ vpart,
-                                                               double *__restrict__ etd_acc,
-                                                               double *__restrict__ v1_acc) {
+__global__ void __launch_bounds__(kFinThreads) tuple_sum_kernel(int nu, int nb, int64_t ncta, int64_t vsize,
+                                                                const __grid_constant__ TupleGroup grp,
+                                                                const double *__restrict__ xpart_all,
+                                                                const double *__restrict__ vpart_all,
+                                                                double *__restrict__ tsum_all) {
   constexpr int U = 8;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
+  const double weight = grp.t[blockIdx.y].weight;
+  const double *xpart = xpart_all + (int64_t)blockIdx.y * ncta, *vpart = vpart_all + (int64_t)blockIdx.y * vsize;
+  double *tsum = tsum_all + (int64_t)blockIdx.y * (1 + 3 * nu);
   if (blockIdx.x == 0) {
     __shared__ double red[256];
     if (tid < 256) {
@@ -73,17 +89,9 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(int nu, int nb, i
       if (tid < st) red[tid] += red[tid + st];
       __syncthreads();
     }
-    if (tid == 0) {
-      const double v = t.weight * red[0];
-      const double sum = etd_acc[0];
-      const double nsum = sum + v;
-      const double comp = fabs(sum) >= fabs(v) ? (sum - nsum) + v : (v - nsum) + sum;
-      etd_acc[0] = nsum;
-      etd_acc[1] += comp;
-    }
+    if (tid == 0) tsum[0] = weight * red[0];
     return;
   }
-  __shared__ double sc[kFinA][3];
   const int warp = tid >> 5, la8 = warp / 3, col = warp - 3 * (warp / 3);
   const int a = (blockIdx.x - 1) * kFinA + la8;
   if (a < nu) {
@@ -101,17 +109,51 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(int nu, int nb, i
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (lane == 0) sc[la8][col] = v;
+    if (lane == 0) tsum[1 + col * nu + a] = weight * v;
   }
-  __syncthreads();
-  if (tid < kFinA) {
-    const int a2 = (blockIdx.x - 1) * kFinA + tid;
-    if (a2 < nu) {
-      v1_acc[a2 + (int64_t)nu * t.i] += t.weight * sc[tid][0];
-      v1_acc[a2 + (int64_t)nu * t.j] += t.weight * sc[tid][1];
-      v1_acc[a2 + (int64_t)nu * t.k] += t.weight * sc[tid][2];
+}
+
+// Adds the group's tuple sums to the accumulators in tuple order, each tuple's
+// columns in the order i, j, k: etd_acc[0..1] is a Neumaier (sum,
+// compensation) pair, v1_acc(nu, no) takes one thread per element.
+__global__ void __launch_bounds__(256) group_add_kernel(int nu, int no, const __grid_constant__ TupleGroup grp,
+                                                        const double *__restrict__ tsum, double *__restrict__ etd_acc,
+                                                        double *__restrict__ v1_acc) {
+  const int64_t stride = 1 + 3 * (int64_t)nu;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) {
+      double sum = etd_acc[0], comp = etd_acc[1];
+      for (int u = 0; u < grp.n; u++) {
+        const double v = tsum[u * stride];
+        const double nsum = sum + v;
+        comp += fabs(sum) >= fabs(v) ? (sum - nsum) + v : (v - nsum) + sum;
+        sum = nsum;
+      }
+      etd_acc[0] = sum;
+      etd_acc[1] = comp;
     }
+    return;
   }
+  const int64_t e = (int64_t)(blockIdx.x - 1) * 256 + threadIdx.x;
+  if (e >= (int64_t)nu * no) return;
+  const int x = (int)(e / nu), a = (int)(e - (int64_t)x * nu);
+  double v = v1_acc[e];
+  constexpr int U = 4;  // tuples whose loads are in flight together
+  for (int u0 = 0; u0 < grp.n; u0 += U) {
+    double c[U][3];
+#pragma unroll
+    for (int q = 0; q < U; q++) {
+      const TupleDev &t = grp.t[u0 + q < grp.n ? u0 + q : u0];
+      const double *s = tsum + (u0 + q) * stride + 1 + a;
+      const bool live = u0 + q < grp.n;
+      c[q][0] = live && t.i == x ? s[0] : 0.0;
+      c[q][1] = live && t.j == x ? s[nu] : 0.0;
+      c[q][2] = live && t.k == x ? s[2 * (int64_t)nu] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < U; q++) v = ((v + c[q][0]) + c[q][1]) + c[q][2];
+  }
+  v1_acc[e] = v;
 }
 
 // out3 = {ets, etd, ets+etd}; ets = 2 sum_{i,a} t1(i,a) v1(a,i) (triples.F90:311-316)
@@ -142,49 +184,57 @@ __global__ void ets_kernel(int no, int nu, const double *__restrict__ t1, const 
 
 }  // namespace
 
-template <int KIND, bool BLOCKED>
-int launch_reduce_kind(const Dims &d, const TupleDev &t, const double *eh, const double *ep, const double *voe,
-                       const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s) {
+template <bool BLOCKED>
+int launch_reduce_layout(const Dims &d, const TupleGroup &g, const double *eh, const double *ep, const double *voe,
+                         const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s) {
   constexpr int smem = REDUCE_SMEM;
   static int configured_device = -1;
   int dev = 0;
   CCT_CUDA(cudaGetDevice(&dev));
   if (configured_device != dev) {
-    CCT_CUDA(cudaFuncSetAttribute(reduce_kernel<KIND, BLOCKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CCT_CUDA(cudaFuncSetAttribute(reduce_kernel<KIND, BLOCKED>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    CCT_CUDA(cudaFuncSetAttribute(reduce_kernel<BLOCKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CCT_CUDA(cudaFuncSetAttribute(reduce_kernel<BLOCKED>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   cudaSharedmemCarveoutMaxShared));
     configured_device = dev;
   }
-  reduce_kernel<KIND, BLOCKED>
-      <<<(unsigned)d.ncta, RT, smem, s>>>(d.nu, d.no, d.NP, t, eh, ep, voe, cta_table, xpart, vpart);
+  reduce_kernel<BLOCKED><<<dim3((unsigned)d.ncta, (unsigned)g.n), RT, smem, s>>>(
+      d.nu, d.no, d.NP, vpart_size(d), g, eh, ep, voe, cta_table, xpart, vpart);
   CCT_CUDA(cudaGetLastError());
   return CCT_OK;
 }
 
-template <bool BLOCKED>
-int launch_reduce_layout(const Dims &d, const TupleDev &t, const double *eh, const double *ep, const double *voe,
-                         const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s) {
-  if (t.kind == kIJK) return launch_reduce_kind<kIJK, BLOCKED>(d, t, eh, ep, voe, cta_table, xpart, vpart, s);
-  if (t.kind == kIJJ) return launch_reduce_kind<kIJJ, BLOCKED>(d, t, eh, ep, voe, cta_table, xpart, vpart, s);
-  return launch_reduce_kind<kIIJ, BLOCKED>(d, t, eh, ep, voe, cta_table, xpart, vpart, s);
-}
-
-int launch_reduce(const Dims &d, const TupleDev &t, const double *eh, const double *ep, const double *voe,
-                  const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s) {
-  if (t.blocked) {
+int launch_reduce(const Dims &d, const TupleGroup &g, bool blocked, const double *eh, const double *ep,
+                  const double *voe, const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s) {
+  if (blocked) {
     if (d.NP % RB) {
       set_error("blocked X needs NP a multiple of 8 (NP = " + std::to_string(d.NP) + ")");
       return CCT_ERR_INVALID;
     }
-    return launch_reduce_layout<true>(d, t, eh, ep, voe, cta_table, xpart, vpart, s);
+    return launch_reduce_layout<true>(d, g, eh, ep, voe, cta_table, xpart, vpart, s);
   }
-  return launch_reduce_layout<false>(d, t, eh, ep, voe, cta_table, xpart, vpart, s);
+  return launch_reduce_layout<false>(d, g, eh, ep, voe, cta_table, xpart, vpart, s);
 }
 
-int launch_finalize(const Dims &d, const TupleDev &t, const double *xpart, const double *vpart, double *etd_acc,
-                    double *v1_acc, cudaStream_t s) {
+int launch_finalize(const Dims &d, const TupleGroup &g, const double *xpart, const double *vpart, double *tsum,
+                    double *etd_acc, double *v1_acc, cudaStream_t s) {
+  static int configured_device = -1;
+  int dev = 0;
+  CCT_CUDA(cudaGetDevice(&dev));
+  if (configured_device != dev) {
+    // the W builds' and reductions' carveout: an SM that would have to change
+    // it first drains
+    CCT_CUDA(cudaFuncSetAttribute(tuple_sum_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  cudaSharedmemCarveoutMaxShared));
+    CCT_CUDA(cudaFuncSetAttribute(group_add_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  cudaSharedmemCarveoutMaxShared));
+    configured_device = dev;
+  }
   const int vblocks = (d.nu + kFinA - 1) / kFinA;  // one warp per (virtual index, column)
-  finalize_kernel<<<1 + vblocks, kFinThreads, 0, s>>>(d.nu, d.nb, d.ncta, t, xpart, vpart, etd_acc, v1_acc);
+  tuple_sum_kernel<<<dim3(1 + vblocks, g.n), kFinThreads, 0, s>>>(d.nu, d.nb, d.ncta, vpart_size(d), g, xpart, vpart,
+                                                                  tsum);
+  CCT_CUDA(cudaGetLastError());
+  const int ablocks = (int)(((int64_t)d.nu * d.no + 255) / 256);
+  group_add_kernel<<<1 + ablocks, 256, 0, s>>>(d.nu, d.no, g, tsum, etd_acc, v1_acc);
   CCT_CUDA(cudaGetLastError());
   return CCT_OK;
 }
