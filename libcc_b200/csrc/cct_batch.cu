@@ -71,7 +71,7 @@ constexpr int kBatchBN[] = {0, 32, 48, 64};
 struct SysDev {
   int no, nu, nb, tiles_m, tiles_n;
   int64_t KP, NP, ncta;
-  const double *eh, *ep, *t1, *voe;
+  const double *eh, *ep, *t1, *vb;
   const int16_t *cta_table;
   int64_t tuple_begin, ntuples;  // the system's tuples, consecutive, in reference order
   double *v1;                    // (nu, no) result
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
         spin_until(group_rd + (T.group - kRing), A.group_rd_items[T.group - kRing], A.err, A.spin_limit);
       __syncthreads();
       const int tile_m = it.w / S.tiles_n, tile_n = it.w - tile_m * S.tiles_n;
-      wb::wbuild_tile<BN, kBTM>(A.jobs[(int64_t)t * 3 + it.z], S.nu, S.KP, S.nu + S.no, S.NP, tile_m, tile_n, smem);
+      wb::wbuild_tile<BN, kBTM>(A.jobs[(int64_t)t * 3 + it.z], S.nu, S.KP, S.nu + S.no, S.NP, tile_m, tile_n, false, smem);
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) atomicAdd(wb_done + t, 1);
@@ -246,11 +246,14 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
       const int S0 = S.cta_table[3 * c], S1 = S.cta_table[3 * c + 1], S2 = S.cta_table[3 * c + 2];
       double *dsm = reinterpret_cast<double *>(smem);
       if (T.kind == kIJK)
-        red::reduce_block<kIJK, true>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.voe, S0, S1, S2, T.xpart + c, T.vpart, dsm);
+        red::reduce_block<kIJK, red::kRowsCoherent>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c,
+                                                      T.vpart, dsm, A.err);
       else if (T.kind == kIJJ)
-        red::reduce_block<kIJJ, true>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.voe, S0, S1, S2, T.xpart + c, T.vpart, dsm);
+        red::reduce_block<kIJJ, red::kRowsCoherent>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c,
+                                                      T.vpart, dsm, A.err);
       else
-        red::reduce_block<kIIJ, true>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.voe, S0, S1, S2, T.xpart + c, T.vpart, dsm);
+        red::reduce_block<kIIJ, red::kRowsCoherent>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c,
+                                                      T.vpart, dsm, A.err);
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -285,7 +288,7 @@ __global__ void __launch_bounds__(wb::NT, 3) batch_wb_kernel(const BatchArgs A, 
   const TupleRec &T = A.tuples[it.y];
   const SysDev &S = A.sys[T.sys];
   const int tile_m = it.w / S.tiles_n, tile_n = it.w - tile_m * S.tiles_n;
-  wb::wbuild_tile<BN, wb::BM>(A.jobs[(int64_t)it.y * 3 + it.z], S.nu, S.KP, S.nu + S.no, S.NP, tile_m, tile_n, smem);
+  wb::wbuild_tile<BN, wb::BM>(A.jobs[(int64_t)it.y * 3 + it.z], S.nu, S.KP, S.nu + S.no, S.NP, tile_m, tile_n, true, smem);
 }
 
 __global__ void __launch_bounds__(kBT, 2) batch_rd_kernel(const BatchArgs A, int64_t item0) {
@@ -310,11 +313,14 @@ __global__ void __launch_bounds__(kBT, 2) batch_rd_kernel(const BatchArgs A, int
   const int c = it.z;
   const int S0 = S.cta_table[3 * c], S1 = S.cta_table[3 * c + 1], S2 = S.cta_table[3 * c + 2];
   if (T.kind == kIJK)
-    red::reduce_block<kIJK>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.voe, S0, S1, S2, T.xpart + c, T.vpart, dsm);
+    red::reduce_block<kIJK, red::kBulk>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c, T.vpart, dsm,
+                                          A.err);
   else if (T.kind == kIJJ)
-    red::reduce_block<kIJJ>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.voe, S0, S1, S2, T.xpart + c, T.vpart, dsm);
+    red::reduce_block<kIJJ, red::kBulk>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c, T.vpart, dsm,
+                                          A.err);
   else
-    red::reduce_block<kIIJ>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.voe, S0, S1, S2, T.xpart + c, T.vpart, dsm);
+    red::reduce_block<kIIJ, red::kBulk>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c, T.vpart, dsm,
+                                          A.err);
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) s_flag = atomicAdd(rd_done + t, 1) == T.rd_items - 1;
@@ -347,7 +353,7 @@ struct BatchSystemHost {
   int no = 0, nu = 0;
   Dims d{};
   double *eh = nullptr, *ep = nullptr, *t1 = nullptr, *t2 = nullptr, *vm = nullptr, *voe = nullptr,
-         *vvvo = nullptr, *E = nullptr, *F = nullptr, *v1 = nullptr;
+         *vvvo = nullptr, *E = nullptr, *F = nullptr, *v1 = nullptr, *vb = nullptr;
   int16_t *cta_table = nullptr;
   int64_t f_np = 0;  // the N padding F was built for
   bool ready = false;
@@ -464,7 +470,7 @@ int build_schedule(ccT_batch *b) {
   struct TH {
     int sys, kind, i, j, k, njobs, group;
     double cost;
-    int64_t scratch, x_off, xpart_off, vpart_off;
+    int64_t scratch, xsize, x_off, xpart_off, vpart_off;
     int wb_items, rd_items;
   };
   std::vector<TH> th;
@@ -503,10 +509,12 @@ int build_schedule(ccT_batch *b) {
       h.j = t.j;
       h.k = t.k;
       h.njobs = t.kind == kIJK ? 3 : 2;
+      const int64_t xs = b->mode == 0 ? nu2 * d.NP : round_up(S.nu, kRB) * round_up(S.nu, kRB) * d.NP;  // X: rows / blocks
+      h.xsize = xs;
       h.cost = (double)h.njobs * nu2 * d.NP * d.KP;
       // X, then the reduction partials; rounded to 256 B so every X buffer of
       // the next tuple stays 16-byte aligned (the W-build stores double2)
-      h.scratch = round_up(h.njobs * nu2 * d.NP * 8, 256);  // rounded: X buffers stay 16-byte aligned
+      h.scratch = round_up(h.njobs * xs * 8, 256);  // rounded: X buffers stay 16-byte aligned
       h.xpart_off = round_up(d.ncta + (int64_t)d.nb * kRB * 3 * npairs, 32);  // partial doubles (offset later)
       h.wb_items = b->mode == 2 ? 0 : h.njobs * tiles_m * tiles_n;
       h.rd_items = (int)d.ncta;
@@ -563,7 +571,7 @@ int build_schedule(ccT_batch *b) {
     r.group = h.group;
     r.wb_items = h.wb_items + (u == b->stall_tuple ? 1 : 0);
     r.rd_items = h.rd_items;
-    for (int g = 0; g < 3; g++) r.x[g] = base + (int64_t)std::min(g, h.njobs - 1) * nu2 * d.NP;
+    for (int g = 0; g < 3; g++) r.x[g] = base + (int64_t)std::min(g, h.njobs - 1) * h.xsize;
     r.xpart = partials + h.xpart_off;
     r.vpart = r.xpart + d.ncta;
     rec[u] = r;
@@ -691,7 +699,7 @@ int build_schedule(ccT_batch *b) {
     v.eh = S.eh;
     v.ep = S.ep;
     v.t1 = S.t1;
-    v.voe = S.voe;
+    v.vb = S.vb;
     v.cta_table = S.cta_table;
     v.tuple_begin = sys_begin[s];
     v.ntuples = sys_count[s];
@@ -786,7 +794,7 @@ int launch_grouped(ccT_batch *b) {
     if (g >= kRing) CCT_CUDA(cudaStreamWaitEvent(b->stream, b->ev_ring[slot], 0));
     for (const ccT_batch::EmuLaunch &L : b->grp_emu[g]) {  // mode 2: one emulated launch per system
       const ccT_plan *P = b->emu_plans[L.sys];
-      CCT_TRY(launch_wbuild_emu(plan_emu(P), plan_dims(P), b->emu_jobs + L.off, (int)L.njobs, b->err, b->stream));
+      CCT_TRY(launch_wbuild_emu(plan_emu(P), plan_dims(P), b->emu_jobs + L.off, (int)L.njobs, b->err, b->stream, true));
     }
     for (const ccT_batch::WbRange &r : b->grp_wb[g]) {
       switch (r.bn) {
@@ -958,7 +966,7 @@ int ccT_batch_create(ccT_batch **out, int64_t nsys, const int64_t *no, const int
     const int64_t n = S.no, v = S.nu, v2 = v * v;
     if ((st = dmalloc(&S.eh, n)) || (st = dmalloc(&S.ep, v)) || (st = dmalloc(&S.t1, n * v)) ||
         (st = dmalloc(&S.t2, v2 * n * n)) || (st = dmalloc(&S.vm, n * v * n * n)) ||
-        (st = dmalloc(&S.voe, v2 * n * n)) || (st = dmalloc(&S.vvvo, v * (v + 1) / 2 * v * n)) ||
+        (st = dmalloc(&S.voe, v2 * n * n)) || (st = dmalloc(&S.vb, vb_size(S.d))) || (st = dmalloc(&S.vvvo, v * (v + 1) / 2 * v * n)) ||
         (st = dmalloc(&S.E, n * v2 * S.d.KP)) || (st = dmalloc(&S.v1, v * n)) ||
         (st = dmalloc(&S.cta_table, S.d.ncta * 3)))
       return fail(st);
@@ -1015,6 +1023,7 @@ int ccT_batch_set_inputs(ccT_batch *b, int64_t s, const double *eh, const double
   CCT_CUDA(cudaMemcpyAsync(S.voe, voe, v2 * n * n * 8, kind, b->stream));
   CCT_CUDA(cudaMemcpyAsync(S.vvvo, vvvo_packed, v * (v + 1) / 2 * v * n * 8, kind, b->stream));
   CCT_TRY(launch_build_e(S.d, S.vvvo, S.t2, S.E, 0, S.no, b->stream));  // E depends on KP alone
+  CCT_TRY(launch_build_vb(S.d, S.voe, S.vb, b->stream));
   CCT_CUDA(cudaStreamSynchronize(b->stream));
   free_schedule(b);  // the next forward rebuilds F (for its N tile) and the graph
   S.ready = true;
@@ -1181,7 +1190,7 @@ int ccT_batch_destroy(ccT_batch *b) {
     if (p) ccT_plan_destroy(p);
   for (BatchSystemHost &S : b->sys)
     for (void *q : {(void *)S.eh, (void *)S.ep, (void *)S.t1, (void *)S.t2, (void *)S.vm, (void *)S.voe,
-                    (void *)S.vvvo, (void *)S.E, (void *)S.F, (void *)S.v1, (void *)S.cta_table})
+                    (void *)S.vvvo, (void *)S.E, (void *)S.F, (void *)S.v1, (void *)S.cta_table, (void *)S.vb})
       if (q) cudaFree(q);
   for (cudaEvent_t e : {b->ev0, b->ev1, b->ev_fork, b->ev_join})
     if (e) cudaEventDestroy(e);

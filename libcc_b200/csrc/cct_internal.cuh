@@ -106,7 +106,7 @@ struct TupleGroup {
   int n = 0;
   TupleDev t[kMaxGroup];
 };
-// X(p,q,s) of a blocked X buffer: block (p/8, q/8, s/8) of 512 doubles at
+// X(p,q,s) of a blocked X buffer (the forward's; the backward reads rows of NP): block (p/8, q/8, s/8) of 512 doubles at
 // ((p/8) nbk + q/8) NP/8 + s/8, element ((p%8) 8 + q%8) 8 + s%8, nbk = ceil(nu/8)
 __host__ __device__ __forceinline__ int64_t xblock_base(int64_t P, int64_t Q, int64_t S, int nu, int64_t NP) {
   return ((P * ((nu + 7) / 8) + Q) * (NP / 8) + S) * 512;
@@ -205,16 +205,22 @@ int launch_check_inputs(const Dims &d, const double *eh, const double *ep, const
                         const double *vm, const double *voe, const double *vvvo, int *flags, cudaStream_t s);
 
 // wbuild_f64.cu
-int launch_wbuild_f64(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStream_t s);
+// blocked: X in 8 x 8 x 8 blocks, else rows of NP
+int launch_wbuild_f64(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStream_t s, bool blocked = false);
 
 // reduce.cu: the reductions of a group of tuples (tuple u's partials at
 // xpart + u d.ncta and vpart + u vpart_size(d)), then their sums added to the
-// accumulators in tuple order.  blocked: X in 8 x 8 x 8 blocks (emulated
-// forward), else rows of NP.  tsum: tsum_size(d) doubles per tuple of the group.
+// accumulators in tuple order.  blocked: X in 8 x 8 x 8 blocks, else rows of
+// NP.  vb: the combined VOE tiles of launch_build_vb; err is set when a bounded
+// wait runs out.  tsum: tsum_size(d) doubles per tuple of the group.
 inline int64_t vpart_size(const Dims &d) { return (int64_t)12 * d.nb * d.nb * (d.nb + 1); }
 inline int64_t tsum_size(const Dims &d) { return 1 + 3 * (int64_t)d.nu; }
 int launch_reduce(const Dims &d, const TupleGroup &g, bool blocked, const double *eh, const double *ep,
-                  const double *voe, const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s);
+                  const double *vb, const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s);
+// 2 VOE(a,b,y,z) - VOE(a,b,z,y) in 8 x 8 tiles, [y][z][nb][nb][64], entry
+// (8 A + u, 8 B + v) of tile (A, B) at u + 8 v; zero past nu.
+inline int64_t vb_size(const Dims &d) { return (int64_t)d.no * d.no * d.nb * d.nb * 64; }
+int launch_build_vb(const Dims &d, const double *voe, double *vb, cudaStream_t s);
 int launch_finalize(const Dims &d, const TupleGroup &g, const double *xpart, const double *vpart, double *tsum,
                     double *etd_acc, double *v1_acc, cudaStream_t s);
 int launch_ets(const Dims &d, const double *t1, const double *v1_acc, const double *etd_acc, double *out3,

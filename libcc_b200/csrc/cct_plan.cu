@@ -44,11 +44,6 @@ using namespace cct;
 // reduction launch each, over a ring of kNBuf X buffer groups: the W build of
 // group g may run while the reductions of groups g-1 .. g-kNBuf+1 still read theirs.
 constexpr int kNBuf = 3;
-// emulated forwards store X in 8 x 8 x 8 blocks (build constant CCT_X_BLOCKED)
-#ifndef CCT_X_BLOCKED
-#define CCT_X_BLOCKED 1
-#endif
-constexpr bool kXBlocked = CCT_X_BLOCKED != 0;
 #ifndef CCT_SERIAL_REDUCE
 #define CCT_SERIAL_REDUCE 1
 #endif
@@ -74,7 +69,7 @@ struct ccT_plan {
   // inputs (device copies, reference layouts)
   double *eh = nullptr, *ep = nullptr, *t1 = nullptr, *t2 = nullptr, *vm = nullptr, *voe = nullptr;
   // derived operands
-  double *E = nullptr, *F = nullptr;
+  double *E = nullptr, *F = nullptr, *vb = nullptr;
   double *X = nullptr;       // GEMM outputs: [nring * group tuples][3][xsize]
   int64_t xsize = 0;         // doubles per GEMM output
   double *xpart = nullptr, *vpart = nullptr, *tsum = nullptr;  // per tuple of a group
@@ -367,14 +362,14 @@ int join_streams(ccT_plan *p) {
 // The W-build GEMMs of tuples [t0, t1) (one X ring group) on stream st: the
 // plan's own form, or the FP64 kernel when fp64 is set (emulated plans keep
 // the FP64 jobs for the backward's recompute and the digit calibration).
-// An emulated W build stores X in 8 x 8 x 8 blocks for the reduction
-// (blocked), or in rows of NP (ccT_tuple_w, whose W assembly reads rows).
-int wbuild_tuples(ccT_plan *p, int64_t t0, int64_t t1, bool fp64, cudaStream_t st, bool blocked = kXBlocked) {
+// X goes to 8 x 8 x 8 blocks for the reduction (blocked), or to rows of NP
+// (ccT_tuple_w and the backward, which read rows).
+int wbuild_tuples(ccT_plan *p, int64_t t0, int64_t t1, bool fp64, cudaStream_t st, bool blocked = true) {
   const int64_t off = job_offset(p, t0);
   const int njobs = (int)(job_offset(p, t1) - off);
   if (p->emulated && !fp64)
     return launch_wbuild_emu(p->emu, p->d, p->emu_jobs + off, njobs, p->flags + 1, st, blocked);
-  return launch_wbuild_f64(p->d, p->jobs + off, njobs, st);
+  return launch_wbuild_f64(p->d, p->jobs + off, njobs, st, blocked);
 }
 
 TupleDev tuple_dev(const Tuple &t, double *const X[3]) {
@@ -476,7 +471,7 @@ int run_group(ccT_plan *p, int64_t t0, int64_t t1, bool fp64 = false, int64_t ke
   }
   CCT_TRY(prof_mark(p, CCT_KERNEL_REDUCE, rs));
   if (rs != p->red_stream) CCT_CUDA(cudaStreamWaitEvent(rs, p->ev_sum, 0));  // the partials of the group before are summed
-  CCT_TRY(launch_reduce(p->d, g, emu && kXBlocked, p->eh, p->ep, p->voe, p->cta_table, p->xpart, p->vpart, rs));
+  CCT_TRY(launch_reduce(p->d, g, keep < 0, p->eh, p->ep, p->vb, p->cta_table, p->xpart, p->vpart, p->flags + 1, rs));
   CCT_CUDA(cudaEventRecord(p->ev_red[slot], rs));
   cudaStream_t fs = p->profiling ? rs : p->red_stream;
   if (rs != fs) CCT_CUDA(cudaStreamWaitEvent(fs, p->ev_red[slot], 0));
@@ -504,7 +499,7 @@ int tuple_energy(ccT_plan *p, int64_t tix, bool fp64, double *e) {
   CCT_CUDA(cudaMemcpyAsync(out3, p->acc + 2, 3 * 8, cudaMemcpyDeviceToHost, p->stream));
   CCT_CUDA(cudaStreamSynchronize(p->stream));
   if (werr) {
-    set_error("an emulated W-build kernel ran out its bounded wait and unwound");
+    set_error("a kernel ran out its bounded wait and unwound");
     return CCT_ERR_TIMEOUT;
   }
   *e = out3[0] + out3[1];
@@ -787,7 +782,7 @@ static int plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options
       return fail(CCT_ERR_CUDA);
   if (cudaEventCreate(&p->ev0) != cudaSuccess || cudaEventCreate(&p->ev1) != cudaSuccess) return fail(CCT_ERR_CUDA);
   const int64_t nu2 = nu * nu, ntup = (int64_t)p->tuples.size();
-  p->xsize = (p->emulated && kXBlocked ? round_up(nu, kRB) * round_up(nu, kRB) : nu2) * d.NP;
+  p->xsize = round_up(nu, kRB) * round_up(nu, kRB) * d.NP;  // blocked; rows of NP fit
   {
     const int64_t bm = p->emulated ? kEmuBM : 128, bn = p->emulated ? d.EBN : d.BN;
     // packed plans: a group could need more slabs than the cache holds
@@ -797,7 +792,7 @@ static int plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options
   }
   if ((s = dalloc(&p->eh, no)) || (s = dalloc(&p->ep, nu)) || (s = dalloc(&p->t1, no * nu)) ||
       (s = dalloc(&p->t2, nu2 * no * no)) || (s = dalloc(&p->vm, no * nu * no * no)) ||
-      (s = dalloc(&p->voe, nu2 * no * no)) ||
+      (s = dalloc(&p->voe, nu2 * no * no)) || (s = dalloc(&p->vb, vb_size(d))) ||
       (s = p->packed ? dalloc(&p->vvvo_res, nu * (nu + 1) / 2 * nu * no) : dalloc(&p->E, no * nu2 * d.KP)) ||
       (s = p->packed ? dalloc(&p->slabs, kSlabs * nu2 * d.KP) : CCT_OK) ||
       (s = dalloc(&p->F, no * no * d.NP * d.KP)) ||
@@ -913,6 +908,7 @@ int ccT_set_inputs(ccT_plan *p, const double *eh, const double *ep, const double
   }
   if (s == CCT_OK && !p->packed) s = launch_build_e(d, vvvo_dev, p->t2, p->E, 0, d.no, p->stream);
   if (s == CCT_OK) s = launch_build_f(d, p->t2, p->vm, p->F, p->stream);
+  if (s == CCT_OK) s = launch_build_vb(d, p->voe, p->vb, p->stream);
   // an automatic plan builds its digit operands during the calibration
   if (s == CCT_OK && p->emulated && !p->emu_auto) s = emu_build_operands(d, p->E, p->F, &p->emu, p->stream);
   if (staged) {
@@ -997,7 +993,7 @@ int ccT_forward(ccT_plan *p, int64_t begin, int64_t end, double *ets, double *et
   if (etd) *etd = out3[1];
   p->fwd_begin = p->fwd_end = -1;
   if (werr) {
-    set_error("an emulated W-build kernel ran out its bounded wait and unwound");
+    set_error("a kernel ran out its bounded wait and unwound");
     return CCT_ERR_TIMEOUT;
   }
   if (!std::isfinite(out3[0]) || !std::isfinite(out3[1])) {
@@ -1111,7 +1107,7 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
       TupleGroup g;
       g.n = 1;
       g.t[0] = tuple_dev(tu, Xk);
-      CCT_TRY(launch_reduce(d, g, false, p->eh, p->ep, p->voe, p->cta_table, p->xpart, p->vpart, sP));
+      CCT_TRY(launch_reduce(d, g, false, p->eh, p->ep, p->vb, p->cta_table, p->xpart, p->vpart, p->flags + 1, sP));
       CCT_TRY(launch_finalize(d, g, p->xpart, p->vpart, p->tsum, p->adj.v1, p->adj.v1 + 5, sP));
     }
     CCT_CUDA(cudaEventRecord(p->ev_pw[xb], sP));
@@ -1251,7 +1247,7 @@ int ccT_tuple_w(ccT_plan *p, int64_t tuple, double *w, int32_t mem) {
   cudaFree(wc);
   if (mem == CCT_MEM_HOST && wf) cudaFree(wf);
   if (s == CCT_OK && werr) {
-    set_error("an emulated W-build kernel ran out its bounded wait and unwound");
+    set_error("a kernel ran out its bounded wait and unwound");
     s = CCT_ERR_TIMEOUT;
   }
   return s;
@@ -1332,7 +1328,7 @@ int ccT_plan_destroy(ccT_plan *p) {
   for (cudaStream_t st : {p->stream, p->gemm_stream, p->gemm_stream2, p->red_stream, p->bwd_stream, p->rec_stream})
     if (st) cudaStreamSynchronize(st);
   double *bufs[] = {p->eh, p->ep, p->t1, p->t2, p->vm, p->voe, p->E, p->F, p->xpart, p->vpart, p->acc, p->stage,
-                    p->vvvo_res, p->slabs, p->X, p->tsum};
+                    p->vvvo_res, p->slabs, p->X, p->tsum, p->vb};
   for (double *b : bufs)
     if (b) cudaFree(b);
   if (p->cta_table) cudaFree(p->cta_table);
@@ -1407,6 +1403,7 @@ void ijk_gpu_init_(const int64_t *no, const int64_t *nu, const double *eh, const
   up(p->vm, vm, n_o * n_u * n_o * n_o);
   up(p->voe, voe, nu2 * n_o * n_o);
   if ((s = launch_build_f(p->d, p->t2, p->vm, p->F, p->stream))) legacy_stop("ijk_gpu_init", s);
+  if ((s = launch_build_vb(p->d, p->voe, p->vb, p->stream))) legacy_stop("ijk_gpu_init", s);
   if ((s = dalloc(&p->stage, n_u * (n_u + 1) / 2 * n_u))) legacy_stop("ijk_gpu_init", s);
   if (cudaMemsetAsync(p->acc, 0, (5 + n_u * n_o) * 8, p->stream) != cudaSuccess) legacy_stop("ijk_gpu_init", CCT_ERR_CUDA);
   p->host_eh.assign(eh, eh + n_o);

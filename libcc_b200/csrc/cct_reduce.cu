@@ -12,10 +12,12 @@
 //
 // The twelve terms arrive as the three GEMM outputs X_g (cct_wbuild_f64.cu),
 // so W at all six index permutations is assembled on chip: one CTA owns an
-// unordered triple of 8-wide index blocks {A<=B<=C}, assembles W on every
-// distinct ordered block of its orbit in shared memory, and evaluates every
-// element of those blocks once.  Per-CTA partials are summed by
+// unordered triple of 8-wide index blocks {A<=B<=C}, brings the X blocks of
+// its orbit into shared memory, and evaluates every element of those blocks
+// once.  Per-CTA partials are summed by
 // tuple_sum_kernel and group_add_kernel in a fixed order, so results are bitwise reproducible.
+#include <algorithm>
+
 #include "cct_internal.cuh"
 #include "cct_reduce_block.cuh"
 
@@ -26,13 +28,13 @@ using namespace red;
 
 // Grid (block triple, tuple of the group); a group may mix tuple kinds, the
 // branch is uniform over a CTA.
-template <bool BLOCKED>
-__global__ void __launch_bounds__(RT, 4) reduce_kernel(int nu, int no, int64_t NP, int64_t vsize,
+template <Fill FILL>
+__global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t NP, int64_t vsize,
                                                       const __grid_constant__ TupleGroup grp,
                                                       const double *__restrict__ eh, const double *__restrict__ ep,
-                                                      const double *__restrict__ voe,
+                                                      const double *__restrict__ vb,
                                                       const int16_t *__restrict__ table, double *__restrict__ xpart,
-                                                      double *__restrict__ vpart) {
+                                                      double *__restrict__ vpart, int *err) {
   extern __shared__ __align__(16) double dyn_smem[];
   const int64_t cta = blockIdx.x;
   const int u = blockIdx.y;
@@ -40,11 +42,11 @@ __global__ void __launch_bounds__(RT, 4) reduce_kernel(int nu, int no, int64_t N
   const int S0 = table[3 * cta], S1 = table[3 * cta + 1], S2 = table[3 * cta + 2];
   double *xp = xpart + (int64_t)u * gridDim.x + cta, *vp = vpart + u * vsize;
   if (t.kind == kIJK)
-    reduce_block<kIJK, false, BLOCKED>(nu, no, NP, t, eh, ep, voe, S0, S1, S2, xp, vp, dyn_smem);
+    reduce_block<kIJK, FILL>(nu, no, NP, t, eh, ep, vb, S0, S1, S2, xp, vp, dyn_smem, err);
   else if (t.kind == kIJJ)
-    reduce_block<kIJJ, false, BLOCKED>(nu, no, NP, t, eh, ep, voe, S0, S1, S2, xp, vp, dyn_smem);
+    reduce_block<kIJJ, FILL>(nu, no, NP, t, eh, ep, vb, S0, S1, S2, xp, vp, dyn_smem, err);
   else
-    reduce_block<kIIJ, false, BLOCKED>(nu, no, NP, t, eh, ep, voe, S0, S1, S2, xp, vp, dyn_smem);
+    reduce_block<kIIJ, FILL>(nu, no, NP, t, eh, ep, vb, S0, S1, S2, xp, vp, dyn_smem, err);
 }
 
 // Sums of one tuple's partials, weighted: tsum[0] = its E[4], then the v1
@@ -182,37 +184,58 @@ __global__ void ets_kernel(int no, int nu, const double *__restrict__ t1, const 
   }
 }
 
+// One thread per entry of a tile (launch_build_vb).
+__global__ void build_vb_kernel(int no, int nu, int nb, const double *__restrict__ voe, double *__restrict__ vb) {
+  const int64_t n = (int64_t)no * no * nb * nb * VTILE, nu2 = (int64_t)nu * nu;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t tile = e / VTILE, yz = tile / ((int64_t)nb * nb), AB = tile - yz * nb * nb;
+    const int64_t A = AB / nb, B = AB - A * nb, y = yz / no, z = yz - y * no;
+    const int64_t f = RB * A + (e & 7), s = RB * B + ((e >> 3) & 7);
+    double v = 0.0;
+    if (f < nu && s < nu)
+      v = fma(2.0, voe[(z * no + y) * nu2 + f + nu * s], -voe[(y * no + z) * nu2 + f + nu * s]);
+    vb[e] = v;
+  }
+}
+
 }  // namespace
 
-template <bool BLOCKED>
-int launch_reduce_layout(const Dims &d, const TupleGroup &g, const double *eh, const double *ep, const double *voe,
-                         const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s) {
+int launch_build_vb(const Dims &d, const double *voe, double *vb, cudaStream_t s) {
+  const int64_t blocks = (vb_size(d) + 255) / 256;
+  build_vb_kernel<<<(unsigned)std::min<int64_t>(blocks, 148 * 64), 256, 0, s>>>(d.no, d.nu, d.nb, voe, vb);
+  CCT_CUDA(cudaGetLastError());
+  return CCT_OK;
+}
+
+template <Fill FILL>
+int launch_reduce_fill(const Dims &d, const TupleGroup &g, const double *eh, const double *ep, const double *vb,
+                       const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s) {
   constexpr int smem = REDUCE_SMEM;
   static int configured_device = -1;
   int dev = 0;
   CCT_CUDA(cudaGetDevice(&dev));
   if (configured_device != dev) {
-    CCT_CUDA(cudaFuncSetAttribute(reduce_kernel<BLOCKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CCT_CUDA(cudaFuncSetAttribute(reduce_kernel<BLOCKED>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    CCT_CUDA(cudaFuncSetAttribute(reduce_kernel<FILL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CCT_CUDA(cudaFuncSetAttribute(reduce_kernel<FILL>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   cudaSharedmemCarveoutMaxShared));
     configured_device = dev;
   }
-  reduce_kernel<BLOCKED><<<dim3((unsigned)d.ncta, (unsigned)g.n), RT, smem, s>>>(
-      d.nu, d.no, d.NP, vpart_size(d), g, eh, ep, voe, cta_table, xpart, vpart);
+  reduce_kernel<FILL><<<dim3((unsigned)d.ncta, (unsigned)g.n), RT, smem, s>>>(
+      d.nu, d.no, d.NP, vpart_size(d), g, eh, ep, vb, cta_table, xpart, vpart, err);
   CCT_CUDA(cudaGetLastError());
   return CCT_OK;
 }
 
 int launch_reduce(const Dims &d, const TupleGroup &g, bool blocked, const double *eh, const double *ep,
-                  const double *voe, const int16_t *cta_table, double *xpart, double *vpart, cudaStream_t s) {
+                  const double *vb, const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s) {
   if (blocked) {
     if (d.NP % RB) {
       set_error("blocked X needs NP a multiple of 8 (NP = " + std::to_string(d.NP) + ")");
       return CCT_ERR_INVALID;
     }
-    return launch_reduce_layout<true>(d, g, eh, ep, voe, cta_table, xpart, vpart, s);
+    return launch_reduce_fill<kBulk>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s);
   }
-  return launch_reduce_layout<false>(d, g, eh, ep, voe, cta_table, xpart, vpart, s);
+  return launch_reduce_fill<kRows>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s);
 }
 
 int launch_finalize(const Dims &d, const TupleGroup &g, const double *xpart, const double *vpart, double *tsum,

@@ -26,14 +26,14 @@ using namespace wb;
 
 template <int BN>
 __global__ void __launch_bounds__(NT, 3) wbuild_f64_kernel(const GemmJob *__restrict__ jobs, int nu, int64_t KP,
-                                                           int64_t KV, int64_t NP, int tiles_n) {
+                                                           int64_t KV, int64_t NP, int tiles_n, bool blocked) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tile_m = blockIdx.x / tiles_n, tile_n = blockIdx.x - tile_m * tiles_n;
-  wbuild_tile<BN>(jobs[blockIdx.y], nu, KP, KV, NP, tile_m, tile_n, smem_raw);
+  wbuild_tile<BN>(jobs[blockIdx.y], nu, KP, KV, NP, tile_m, tile_n, blocked, smem_raw);
 }
 
 template <int BN>
-int launch_bn(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStream_t s) {
+int launch_bn(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStream_t s, bool blocked) {
   constexpr int smem = smem_bytes<BN>();
   static int configured_device = -1;
   int dev = 0;
@@ -46,21 +46,21 @@ int launch_bn(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStream_t s)
   const int tiles_m = (int)((M + BM - 1) / BM);
   const int tiles_n = (int)(d.NP / BN);
   dim3 grid(tiles_m * tiles_n, njobs);
-  wbuild_f64_kernel<BN><<<grid, NT, smem, s>>>(jobs_dev, d.nu, d.KP, d.nu + d.no, d.NP, tiles_n);
+  wbuild_f64_kernel<BN><<<grid, NT, smem, s>>>(jobs_dev, d.nu, d.KP, d.nu + d.no, d.NP, tiles_n, blocked);
   CCT_CUDA(cudaGetLastError());
   return CCT_OK;
 }
 
 }  // namespace
 
-int launch_wbuild_f64(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStream_t s) {
+int launch_wbuild_f64(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStream_t s, bool blocked) {
   switch (d.BN) {
-    case 64: return launch_bn<64>(d, jobs_dev, njobs, s);
-    case 56: return launch_bn<56>(d, jobs_dev, njobs, s);
-    case 48: return launch_bn<48>(d, jobs_dev, njobs, s);
-    case 40: return launch_bn<40>(d, jobs_dev, njobs, s);
-    case 32: return launch_bn<32>(d, jobs_dev, njobs, s);
-    case 24: return launch_bn<24>(d, jobs_dev, njobs, s);  // the CCSD terms' X_j GEMM (N = no)
+    case 64: return launch_bn<64>(d, jobs_dev, njobs, s, blocked);
+    case 56: return launch_bn<56>(d, jobs_dev, njobs, s, blocked);
+    case 48: return launch_bn<48>(d, jobs_dev, njobs, s, blocked);
+    case 40: return launch_bn<40>(d, jobs_dev, njobs, s, blocked);
+    case 32: return launch_bn<32>(d, jobs_dev, njobs, s, blocked);
+    case 24: return launch_bn<24>(d, jobs_dev, njobs, s, blocked);  // the CCSD terms' X_j GEMM (N = no)
     default:
       set_error("unsupported W-build N tile " + std::to_string(d.BN));
       return CCT_ERR_INVALID;

@@ -51,10 +51,11 @@ __device__ __forceinline__ void dmma_16x8x4(double *d, double a0, double a1, dou
 // KP-long half of the contraction holds KV = nu + no columns and zero
 // padding, whose k4 steps are skipped.  smem_raw holds smem_bytes<BN, TM>().
 // It starts with a barrier, so a persistent CTA can call it for consecutive
-// tiles on the same shared memory.
+// tiles on the same shared memory.  blocked: X in 8 x 8 x 8 blocks
+// (xblock_base; four lanes write one 64-byte row of a block, as in rows of NP).
 template <int BN, int TM = BM>
 __device__ __forceinline__ void wbuild_tile(const GemmJob &job, int nu, int64_t KP, int64_t KV, int64_t NP,
-                                            int tile_m, int tile_n, unsigned char *smem_raw) {
+                                            int tile_m, int tile_n, bool blocked, unsigned char *smem_raw) {
   constexpr int BM = TM, NT = TM;
   constexpr int NF = BN / 8;
   double *As = reinterpret_cast<double *>(smem_raw);
@@ -185,7 +186,7 @@ __device__ __forceinline__ void wbuild_tile(const GemmJob &job, int nu, int64_t 
   }
   cp_async_wait<0>();
 
-  // epilogue: X[(p*nu+q)*NP + s]
+  // epilogue: X[(p*nu+q)*NP + s], or its place in the blocks
 #pragma unroll
   for (int i = 0; i < MF; i++) {
 #pragma unroll
@@ -193,10 +194,16 @@ __device__ __forceinline__ void wbuild_tile(const GemmJob &job, int nu, int64_t 
       const int64_t m = m0 + warp * WM + i * 16 + g + half * 8;
       if (m >= M) continue;
       double *orow = job.out + m * NP + n0 + 2 * t;
+      int64_t step = 8;
+      if (blocked) {
+        const int r = warp * WM + i * 16 + g + half * 8, p = rowpq[2 * r], q = rowpq[2 * r + 1];
+        orow = job.out + xblock_base(p >> 3, q >> 3, n0 >> 3, nu, NP) + ((p & 7) * 8 + (q & 7)) * 8 + 2 * t;
+        step = 512;
+      }
 #pragma unroll
       for (int j = 0; j < NF; j++) {
         double2 v = make_double2(acc[i][j][2 * half], acc[i][j][2 * half + 1]);
-        *reinterpret_cast<double2 *>(orow + j * 8) = v;
+        *reinterpret_cast<double2 *>(orow + j * step) = v;
       }
     }
   }
