@@ -89,7 +89,7 @@ constexpr int A_BLK = kEmuABlk;
 #define CCT_EMU_DRAIN_WARPS 16
 #endif
 #ifndef CCT_EMU_MAXNREG
-#define CCT_EMU_MAXNREG 80
+#define CCT_EMU_MAXNREG 96
 #endif
 // Ring budget: 200 KB gives a 3-digit, 80-column tile five stages (2% faster
 // than four) and 5 digits three (5% faster than two); the reduction CTA that
@@ -121,9 +121,6 @@ __device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvt
 __device__ __forceinline__ void mbar_init(uint64_t *b, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(b)), "r"(count));
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(b)), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive(uint64_t *b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
 }
@@ -135,6 +132,38 @@ __device__ __forceinline__ bool mbar_test(uint64_t *b, uint32_t parity) {
       : "r"(su32(b)), "r"(parity)
       : "memory");
   return ok != 0;
+}
+// One poll that never suspends the thread.
+__device__ __forceinline__ bool mbar_poll(uint64_t *b, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+      : "=r"(ok)
+      : "r"(su32(b)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// The same operations on barrier addresses a loop steps through.
+__device__ __forceinline__ bool mbar_test_at(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_poll_at(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
 }
 // Bounded wait on a phase parity.  Returns false when another role of the CTA
 // aborted, or when the limit runs out (then the error word and the abort flag
@@ -154,10 +183,13 @@ __device__ __forceinline__ void mbar_settle(uint64_t *b, uint32_t parity, int *e
     if (mbar_test(b, parity)) return;
   atomicExch(err, 1);
 }
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+__device__ __forceinline__ void mbar_expect_tx_at(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load_at(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(su32(dst)),
-      "l"(src), "r"(bytes), "r"(su32(bar))
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
 // K-major, no swizzle: 8-row x 16-byte core matrices; the two K halves of a
@@ -208,16 +240,53 @@ struct EmuArgs {
 
 constexpr int kNoRowExp = -30000;  // exponent of an all-zero row: never the maximum
 
-// Digits of work item (row tile tm, column tile tn of job z = x3).
-template <int S>
-__device__ __forceinline__ int item_slices(const EmuArgs &a, int tm, int tn, int z) {
-  if (!a.tileExp) return S;
-  const int ea = a.tileExp[tm], eb = a.tileExp[a.tiles_m + z * a.tiles_n + tn];
-  const int top = a.tileExp[a.tiles_m + a.no * a.tiles_n] + a.tileExp[a.tiles_m + a.no * a.tiles_n + 1];
-  if (ea <= kNoRowExp || eb <= kNoRowExp) return 1;  // all-zero rows or columns: X is zero
-  const int s = S - (top - (ea + eb)) / 7;
-  return s < 1 ? 1 : (s > S ? S : s);
-}
+// A CTA's work items, one after the other: (job, row tile, column tile), the
+// column tile fastest, every gridDim.x-th.
+struct ItemCursor {
+  int jb, tm, tn, step_m, step_n;
+  __device__ __forceinline__ explicit ItemCursor(const EmuArgs &a) {
+    step_m = (int)gridDim.x / a.tiles_n;
+    step_n = (int)gridDim.x - step_m * a.tiles_n;
+    tm = (int)blockIdx.x / a.tiles_n;
+    tn = (int)blockIdx.x - tm * a.tiles_n;
+    jb = tm / a.tiles_m;
+    tm -= jb * a.tiles_m;
+  }
+  __device__ __forceinline__ bool valid(const EmuArgs &a) const { return jb < a.njobs; }
+  __device__ __forceinline__ void next(const EmuArgs &a) {
+    tn += step_n;
+    tm += step_m;
+    if (tn >= a.tiles_n) {
+      tn -= a.tiles_n;
+      tm++;
+    }
+    while (tm >= a.tiles_m) {
+      tm -= a.tiles_m;
+      jb++;
+    }
+  }
+};
+
+// Digits of a work item of an adaptive plan, from its tiles' exponents; load()
+// only issues the loads, so they can be in flight while the item before runs.
+struct ItemDigits {
+  int ea = 0, eb = 0, top = 0;
+  __device__ __forceinline__ explicit ItemDigits(const EmuArgs &a) {
+    if (a.tileExp) top = a.tileExp[a.tiles_m + a.no * a.tiles_n] + a.tileExp[a.tiles_m + a.no * a.tiles_n + 1];
+  }
+  __device__ __forceinline__ void load(const EmuArgs &a, const ItemCursor &c, int z) {  // z = x3 of the item's job
+    if (!a.tileExp) return;
+    ea = a.tileExp[c.tm];
+    eb = a.tileExp[a.tiles_m + z * a.tiles_n + c.tn];
+  }
+  template <int S>
+  __device__ __forceinline__ int digits(const EmuArgs &a) const {
+    if (!a.tileExp) return S;
+    if (ea <= kNoRowExp || eb <= kNoRowExp) return 1;  // all-zero rows or columns: X is zero
+    const int s = S - (top - (ea + eb)) / 7;
+    return s < 1 ? 1 : (s > S ? S : s);
+  }
+};
 
 __device__ __forceinline__ double pow2(int e) {
   // exact 2^e for normal exponents; ldexp covers the subnormal range
@@ -246,8 +315,6 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t M = (int64_t)args.nu * args.nu;
-  const int per_job = args.tiles_m * args.tiles_n;
-  const int64_t nitems = (int64_t)args.njobs * per_job;
   const int KC = args.kchunks;
   const int64_t GA = (int64_t)args.sop * A_BLK, GB = (int64_t)args.sop * B_BLK;  // bytes of one K chunk in HBM
   const int64_t aslab = (int64_t)args.tiles_m * KC * GA;  // bytes per occupied index
@@ -279,154 +346,220 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
 
   if (warp == 0) {
     if (lane == 0) {  // ---------------- producer
-      uint32_t g = 0;
-      bool ok = true;
-      for (int64_t it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
-        const int jb = (int)(it / per_job);
-        const int rem = (int)(it - (int64_t)jb * per_job);
-        const int tm = rem / args.tiles_n, tn = rem - tm * args.tiles_n;
-        const EmuJob job = args.jobs[jb];
-        const int sl = item_slices<S>(args, tm, tn, job.x3);
+      const uint32_t full0 = su32(full), empty0 = su32(empty), a0 = su32(sA), b0 = su32(sB);
+      int st = 0;
+      uint32_t ph = 1;  // a slot's first use finds the phase before the first complete
+      bool ok = true, wrapped = false;
+      // Every role reads an item's job one item ahead and what the job's
+      // values address one item ahead of its use, so no item starts by
+      // waiting for a chain of loads (that chain, with 64-bit divisions for
+      // the item's place, took some 2 us an item in each role): CCT_EMU_ITEM
+      ItemCursor cur(args), nxt = cur;
+      ItemDigits dig(args);
+      EmuJob job{}, job1{};
+      int sl = S;
+      if (cur.valid(args)) {
+        job = args.jobs[cur.jb];
+        dig.load(args, cur, job.x3);
+        sl = dig.digits<S>(args);
+        nxt.next(args);
+        if (nxt.valid(args)) job1 = args.jobs[nxt.jb];
+      }
+      while (cur.valid(args) && ok) {
+        const int tm = cur.tm, tn = cur.tn;
+        ItemCursor nx2 = nxt;
+        EmuJob job2{};
+        if (nxt.valid(args)) {
+          dig.load(args, nxt, job1.x3);
+          nx2.next(args);
+          if (nx2.valid(args)) job2 = args.jobs[nx2.jb];
+        }
+        const bool run = sl == S && whole;  // a stage's chunks are one contiguous run per operand
         for (int h = 0; h < job.nhalves && ok; h++) {
           const int8_t *A = (h == 0 ? args.E8 + job.x1 * aslab : args.E8T + job.x2 * aslab) + (int64_t)tm * KC * GA;
           const int8_t *B = args.F8 + job.fyz[h] * bslab + (int64_t)tn * KC * GB;
-          for (int kc = 0; kc < KC; kc += KS, g++) {
-            const int st = (int)(g % ST);
-            const uint32_t nch = KC - kc < KS ? (uint32_t)(KC - kc) : (uint32_t)KS;  // the last stage may be short
-            if (g >= (uint32_t)ST && !mbar_wait(&empty[st], ((g / ST) - 1) & 1, args.err, abort_flag)) {
+          for (int left = KC; left > 0; left -= KS) {
+            const uint32_t nch = left < KS ? (uint32_t)left : (uint32_t)KS;  // the last stage may be short
+            if (!mbar_test_at(empty0 + 8 * st, ph) && !mbar_wait(&empty[st], ph, args.err, abort_flag)) {
               ok = false;
               break;
             }
-            if (sl == S && whole) {  // all digits: the stage's chunks are one contiguous run per operand
-              mbar_expect_tx(&full[st], nch * (CA + CB));
-              bulk_load(sA + st * SA, A + (int64_t)kc * GA, nch * CA, &full[st]);
-              bulk_load(sB + st * SB, B + (int64_t)kc * GB, nch * CB, &full[st]);
+            const uint32_t bar = full0 + 8 * st, da = a0 + st * SA, db = b0 + st * SB;
+            if (run) {
+              mbar_expect_tx_at(bar, nch * (CA + CB));
+              bulk_load_at(da, A, nch * CA, bar);
+              bulk_load_at(db, B, nch * CB, bar);
             } else {  // the leading sl digit slices of each chunk
-              mbar_expect_tx(&full[st], nch * (uint32_t)sl * (A_BLK + B_BLK));
+              mbar_expect_tx_at(bar, nch * (uint32_t)sl * (A_BLK + B_BLK));
               for (uint32_t c = 0; c < nch; c++) {
-                bulk_load(sA + st * SA + c * CA, A + (int64_t)(kc + c) * GA, (uint32_t)sl * A_BLK, &full[st]);
-                bulk_load(sB + st * SB + c * CB, B + (int64_t)(kc + c) * GB, (uint32_t)sl * B_BLK, &full[st]);
+                bulk_load_at(da + c * CA, A + c * GA, (uint32_t)sl * A_BLK, bar);
+                bulk_load_at(db + c * CB, B + c * GB, (uint32_t)sl * B_BLK, bar);
               }
+            }
+            A += KS * GA;
+            B += KS * GB;
+            if (++st == ST) {
+              st = 0;
+              ph ^= 1;
+              wrapped = true;
             }
           }
         }
+        sl = dig.digits<S>(args);
+        cur = nxt;
+        nxt = nx2;
+        job = job1;
+        job1 = job2;
       }
       // let every copy still in flight land before the CTA can exit
-      for (uint32_t q = g > (uint32_t)ST ? g - ST : 0; q < g; q++) mbar_settle(&full[q % ST], (q / ST) & 1, args.err);
+      // (slots before st hold this round's copies, the others the round before's)
+      const uint32_t round = ph ^ 1;
+      for (int q = 0; q < ST; q++) {
+        if (q < st)
+          mbar_settle(&full[q], round, args.err);
+        else if (wrapped)
+          mbar_settle(&full[q], round ^ 1, args.err);
+      }
     }
   } else if (warp == 1) {
     if (lane == 0) {  // ---------------- MMA issuer
       // kind::i8, D s32, A/B s8, K-major, M = 128; N (bits 17-22, N >> 3) per MMA
       const uint32_t idesc0 = (2u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
       const uint64_t dA0 = desc_kmajor(sA), dB0 = desc_kmajor(sB);
-      uint32_t g = 0, n = 0;
+      uint32_t n = 0;
       bool ok = true;
-      // halves and digit count of an item (global loads: the issuer fetches
-      // them one item ahead, so they are not between two items' MMAs)
-      auto item_info = [&](int64_t item, int *nhalves, int *slices) {
-        const int jb = (int)(item / per_job);
-        const int rem = (int)(item - (int64_t)jb * per_job);
-        const int tm = rem / args.tiles_n, tn = rem - tm * args.tiles_n;
-        const EmuJob &job = args.jobs[jb];
-        *nhalves = job.nhalves;
-        *slices = item_slices<S>(args, tm, tn, job.x3);
-      };
-      int nh_next = 0, sl_next = 0;
-      if (blockIdx.x < nitems) item_info(blockIdx.x, &nh_next, &sl_next);
-      for (int64_t it = blockIdx.x; it < nitems && ok; it += gridDim.x, n++) {
+      // The tensor pipe holds only a few MMAs ahead of the one it runs, so the
+      // issuer's own work idles it unless long MMAs are queued meanwhile.  So:
+      // the next stage's barrier is polled, and its place in the ring worked
+      // out, before a stage's last and widest MMA; a stage's slot is handed
+      // back (the commit) only after the first MMAs of the stage after it; a
+      // chunk ends with its widest row (t = 0) except an item's first, whose
+      // t = 0 row initialises the accumulators; the next item's job is read in
+      // the middle of an item.  Of some 560 clocks a 3-digit 80-column chunk
+      // takes (616 before), its MMAs need 244 back to back; reading a barrier
+      // still waits for the MMAs queued before it.
+      const uint32_t full0 = su32(full), empty0 = su32(empty);
+      const uint32_t hiA = (uint32_t)(dA0 >> 32), hiB = (uint32_t)(dB0 >> 32);  // constant: only the start address moves
+      const uint32_t loA0 = (uint32_t)dA0, loB0 = (uint32_t)dB0;
+      int st = 0;
+      uint32_t ph = 0;            // parity of full[st]'s current phase
+      bool ready = false;         // full[st] has been seen complete
+      uint32_t pending = 0;       // barrier of the slot the next commit hands back
+      ItemCursor cur(args), nxt = cur;
+      ItemDigits dig(args);
+      int sl = S, nh = 0, nh1 = 0, z1 = 0;  // the item's, and the next item's halves and x3
+      if (cur.valid(args)) {
+        nh = args.jobs[cur.jb].nhalves;
+        dig.load(args, cur, args.jobs[cur.jb].x3);
+        sl = dig.digits<S>(args);
+        nxt.next(args);
+        if (nxt.valid(args)) {
+          nh1 = args.jobs[nxt.jb].nhalves;
+          z1 = args.jobs[nxt.jb].x3;
+        }
+      }
+      constexpr bool kLate = ST > 3;  // rings of two or three stages need the slot back at once
+      bool acc_free = true;  // the accumulator set of the item has been seen free
+      for (; cur.valid(args) && ok; n++) {
         // item n uses accumulator set ab; the drain of the item that used it
         // last (use - 1 uses ago) has read it
         const int ab = NB == 2 ? (int)(n & 1) : 0;
         const uint32_t use = NB == 2 ? (n >> 1) : n;
         const uint32_t acc = tmem + (uint32_t)(ab * S * EBN);
-        if (use > 0 && !mbar_wait(&tmem_empty[ab], (use - 1) & 1, args.err, abort_flag)) {
+        if (!acc_free && !mbar_wait(&tmem_empty[ab], (use - 1) & 1, args.err, abort_flag)) {
           ok = false;
           break;
         }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const int nh = nh_next, sl = sl_next;
-        // the next item's job and digit count, loaded while this item's MMAs issue
-        if (it + gridDim.x < nitems) item_info(it + gridDim.x, &nh_next, &sl_next);
-        if (args.slice_hist) atomicAdd(args.slice_hist + sl, 1ull);
-        for (int h = 0; h < nh && ok; h++) {
-          for (int kc = 0; kc < KC; kc += KS, g++) {
-            const int st = (int)(g % ST);
-            const int nch = KC - kc < KS ? KC - kc : KS;
-            if (!mbar_wait(&full[st], (g / ST) & 1, args.err, abort_flag)) {
+        ItemCursor nx2 = nxt;
+        int nh2 = 0, z2 = 0;
+        // A slice t against B slices u0 .. u0+cnt-1 (one operand of cnt
+        // EBN rows) into diagonals t+u0 .. t+u0+cnt-1
+        auto mma = [&](uint32_t loA, uint32_t loB, int t, int u0, int cnt, uint32_t accumulate) {
+          const uint32_t idesc = idesc0 | ((uint32_t)((cnt * EBN) >> 3) << 17);
+          asm volatile(
+              "{ .reg .pred p; .reg .b64 a, b; setp.ne.b32 p, %6, 0; mov.b64 a, {%1, %2}; mov.b64 b, {%3, %4}; "
+              "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %5, p; }" ::"r"(acc + (uint32_t)((t + u0) * EBN)),
+              "r"(loA + (uint32_t)(t * (A_BLK >> 4))), "r"(hiA), "r"(loB + (uint32_t)(u0 * (B_BLK >> 4))), "r"(hiB),
+              "r"(idesc), "r"(accumulate));
+        };
+        // A slice t meets n = s - t B slices, taken as MMAs of at most MPS
+        // slices whose sizes differ by one.
+        auto row = [&](uint32_t loA, uint32_t loB, int s, int t, uint32_t accumulate) {
+          const int n = s - t;
+          const int parts = (n + MPS - 1) / MPS;
+          const int base = n / parts, extra = n - base * parts;
+#pragma unroll
+          for (int q = 0; q < parts; q++)
+            mma(loA, loB, t, q * base + (q < extra ? q : extra), base + (q < extra ? 1 : 0), accumulate);
+        };
+        const int stages = (KC + KS - 1) / KS * nh;
+        // The stages of the item at a digit count fixed at compile time:
+        // straight-line MMAs with constant shapes and offsets.
+        auto run_item = [&](auto slc) {
+          constexpr int SLC = decltype(slc)::value;
+          int left = KC;  // chunks of the half
+          for (int q = 0; q < stages; q++) {
+            if (!ready && !mbar_wait(&full[st], ph, args.err, abort_flag)) {
               ok = false;
-              break;
+              return;
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint32_t loA = loA0 + st * (SA >> 4), loB = loB0 + st * (SB >> 4);  // 16-byte units
+            const uint32_t slot = empty0 + 8 * st;
+            if (++st == ST) {
+              st = 0;
+              ph ^= 1;
+            }
+            ready = mbar_poll_at(full0 + 8 * st, ph);  // read at the next stage
+            const bool two = KS > 1 && left > 1;       // the last stage of a half may hold one chunk
+            left -= KS;
+            if (left <= 0) left = KC;
+            if (q == 0) {  // the item's first chunk: t = 0 initialises every diagonal
 #pragma unroll
-            for (int c = 0; c < KS; c++) {
-              if (c >= nch) break;
-              // descriptor start addresses are linear in 16-byte units
-              const uint64_t dA = dA0 + (uint64_t)((st * SA + c * CA) >> 4);
-              const uint64_t dB = dB0 + (uint64_t)((st * SB + c * CB) >> 4);
-              const uint32_t first = (h == 0 && kc == 0 && c == 0) ? 0u : 1u;  // accumulate flag of the t = 0 row
-              // A slice t against B slices u0 .. u0+cnt-1 (one operand of cnt
-              // EBN rows) into diagonals t+u0 .. t+u0+cnt-1
-              auto mma = [&](int t, int u0, int cnt) {
-                const uint32_t idesc = idesc0 | ((uint32_t)((cnt * EBN) >> 3) << 17);
-                asm volatile(
-                    "{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p; "
-                    "}" ::"r"(acc + (uint32_t)((t + u0) * EBN)),
-                    "l"(dA + (uint64_t)(t * (A_BLK >> 4))), "l"(dB + (uint64_t)(u0 * (B_BLK >> 4))), "r"(idesc),
-                    "r"(t > 0 ? 1u : first));
-              };
-              // t = 0 first: with the accumulate flag clear it initialises
-              // every diagonal of the item; later rows add into them.  Each
-              // digit count has a schedule fixed at compile time:
-              // straight-line MMAs with constant shapes and offsets, so the
-              // single issuing thread spends no time on the partition
-              // arithmetic between MMAs.  A slice t meets n = s - t B slices,
-              // taken as MMAs of at most MPS slices whose sizes differ by one.
-              auto schedule = [&](auto slc) {
-                constexpr int SLC = decltype(slc)::value;
-#pragma unroll
-                for (int t = 0; t < SLC; t++) {
-                  const int n = SLC - t;
-                  const int parts = (n + MPS - 1) / MPS;
-                  const int base = n / parts, extra = n - base * parts;
-#pragma unroll
-                  for (int q = 0; q < parts; q++) mma(t, q * base + (q < extra ? q : extra), base + (q < extra ? 1 : 0));
-                }
-              };
-              if constexpr (EBN <= 80) {
-                switch (sl) {
-                  case 1: schedule(std::integral_constant<int, 1>{}); break;
-                  case 2: if constexpr (S >= 2) schedule(std::integral_constant<int, 2>{}); break;
-                  case 3: if constexpr (S >= 3) schedule(std::integral_constant<int, 3>{}); break;
-                  case 4: if constexpr (S >= 4) schedule(std::integral_constant<int, 4>{}); break;
-                  case 5: if constexpr (S >= 5) schedule(std::integral_constant<int, 5>{}); break;
-                  case 6: if constexpr (S >= 6) schedule(std::integral_constant<int, 6>{}); break;
-                  default: if constexpr (S >= 7) schedule(std::integral_constant<int, 7>{}); break;
-                }
-              } else if (sl == S) {  // the 96-column tile: one fixed schedule (more would spill)
-                schedule(std::integral_constant<int, S>{});
-              } else {
-#pragma unroll
-                for (int t = 0; t < S; t++) {
-                  if (t >= sl) break;
-                  const int n = sl - t;
-                  const int parts = (n + MPS - 1) / MPS;
-                  const int base = n / parts, extra = n - base * parts;
-                  int u0 = 0;
-                  for (int q = 0; q < parts; q++) {
-                    const int cnt = base + (q < extra ? 1 : 0);
-                    mma(t, u0, cnt);
-                    u0 += cnt;
-                  }
+              for (int t = 0; t < SLC; t++) row(loA, loB, SLC, t, t > 0 ? 1u : 0u);
+              if (nxt.valid(args)) {  // the next item's exponents, the job after it
+                dig.load(args, nxt, z1);
+                nx2.next(args);
+                if (nx2.valid(args)) {
+                  nh2 = args.jobs[nx2.jb].nhalves;
+                  z2 = args.jobs[nx2.jb].x3;
                 }
               }
+            } else {
+#pragma unroll
+              for (int t = SLC - 1; t >= 0; t--) row(loA, loB, SLC, t, 1u);
+              if (kLate) mma_commit(pending);
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                su32(&empty[st])));
+            pending = slot;
+            if (q == stages - 1) {
+              const uint32_t u1 = NB == 2 ? (n + 1) >> 1 : n + 1;  // the next item's use of its set
+              acc_free = u1 == 0 || (NB == 2 && mbar_poll(&tmem_empty[(n + 1) & 1], (u1 - 1) & 1));
+            }
+            if (two) {
+#pragma unroll
+              for (int t = SLC - 1; t >= 0; t--) row(loA + (CA >> 4), loB + (CB >> 4), SLC, t, 1u);
+            }
+            if (!kLate) mma_commit(slot);
           }
+        };
+        switch (sl) {
+          case 1: run_item(std::integral_constant<int, 1>{}); break;
+          case 2: if constexpr (S >= 2) run_item(std::integral_constant<int, 2>{}); break;
+          case 3: if constexpr (S >= 3) run_item(std::integral_constant<int, 3>{}); break;
+          case 4: if constexpr (S >= 4) run_item(std::integral_constant<int, 4>{}); break;
+          case 5: if constexpr (S >= 5) run_item(std::integral_constant<int, 5>{}); break;
+          case 6: if constexpr (S >= 6) run_item(std::integral_constant<int, 6>{}); break;
+          default: if constexpr (S >= 7) run_item(std::integral_constant<int, 7>{}); break;
         }
         if (!ok) break;
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            su32(&acc_full[ab])));
+        mma_commit(su32(&acc_full[ab]));
+        if (kLate) mma_commit(pending);
+        sl = dig.digits<S>(args);
+        nh = nh1;
+        nh1 = nh2;
+        z1 = z2;
+        cur = nxt;
+        nxt = nx2;
       }
       // every MMA issued has completed before the tensor memory is freed
       asm volatile(
@@ -435,70 +568,112 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
     }
   } else {  // ---------------- drain: warp w owns TMEM lane quarter w % 4
     constexpr int CW = EBN / (NDW / 4);  // columns per drain warp
-    static_assert(CW % 4 == 0, "the drain stores X four columns at a time");
+    static_assert(CW % 4 == 0 && CW <= 32, "the drain stores X four columns at a time, a column scale per lane");
     const int q = warp & 3;
     const int row = q * 32 + lane;
     const int cbase = ((warp - 2) / 4) * CW;
-    // diagonal d = t + u (0-based digits) carries 2^(-7(d+2)), times 2^2 for
-    // the two operand scales 2^(e+1)
-    double cd[S];
-#pragma unroll
-    for (int d = 0; d < S; d++) cd[d] = pow2(2 - 7 * (d + 2));
     uint32_t n = 0;
-    for (int64_t it = blockIdx.x; it < nitems; it += gridDim.x, n++) {
-      // everything that does not depend on the MMAs is fetched before the wait
-      const int jb = (int)(it / per_job);
-      const int rem = (int)(it - (int64_t)jb * per_job);
-      const int tm = rem / args.tiles_n, tn = rem - tm * args.tiles_n;
-      const EmuJob job = args.jobs[jb];
-      const int64_t m = (int64_t)tm * EBM + row;
-      const bool live = m < M;
-      const int eA = live ? args.expE[m] : 0;
-      const int n0 = tn * EBN + cbase;
-      const int sl = item_slices<S>(args, tm, tn, job.x3);
+    ItemCursor cur(args), nxt = cur;
+    ItemDigits dig(args);
+    int sl = S, z1 = 0, eA1 = 0, eB1 = 0;
+    double *out = nullptr, *out1 = nullptr;
+    // exponents of an item's row of this thread, and of column n0 + lane
+    auto load_exps = [&](const ItemCursor &c, int z, int *eA, int *eB) {
+      const uint32_t m = (uint32_t)c.tm * EBM + row;  // nu^2 < 2^31
+      *eA = m < (uint32_t)M ? args.expE[m] : 0;
+      *eB = lane < CW ? args.expF[(int64_t)z * args.NPe + c.tn * EBN + cbase + lane] : 0;
+    };
+    if (cur.valid(args)) {
+      const EmuJob &job = args.jobs[cur.jb];
+      out = job.out;
+      dig.load(args, cur, job.x3);
+      load_exps(cur, job.x3, &eA1, &eB1);
+      sl = dig.digits<S>(args);
+      nxt.next(args);
+      if (nxt.valid(args)) {
+        out1 = args.jobs[nxt.jb].out;
+        z1 = args.jobs[nxt.jb].x3;
+      }
+    }
+    for (; cur.valid(args); n++) {
+      const uint32_t m = (uint32_t)cur.tm * EBM + row;
+      const bool live = m < (uint32_t)M;
+      const int n0 = cur.tn * EBN + cbase;
+      // The diagonals are summed exactly in int64, acc = sum_d D_d 2^(7(sl-1-d)): |D_d| <= 2 (d+1) K 64^2, so below 2^63 for six
+      // digits and K <= 32000; a seventh is added in FP64.  One conversion
+      // and one power-of-two scaling per element follow.
+      const int e0 = eA1 + 2 - 7 * (sl + 1);
+      const int eBl = eB1;
+      const int emin = e0 + __reduce_min_sync(0xffffffffu, eBl), emax = e0 + __reduce_max_sync(0xffffffffu, eBl);
+      const bool normal = __all_sync(0xffffffffu, emin >= -1022 && emax <= 1023);
+      double *xrow = out;
+      if (args.xblocked) {
+        const uint32_t pp = m / (uint32_t)args.nu, qq = m - pp * (uint32_t)args.nu;
+        xrow += xblock_base(pp >> 3, qq >> 3, 0, args.nu, args.NP) + ((pp & 7) * 8 + (qq & 7)) * 8;
+      } else {
+        xrow += (int64_t)m * args.NP;
+      }
+      // the next item's exponents and the job after it, loaded while this item's MMAs run
+      ItemCursor nx2 = nxt;
+      double *out2 = nullptr;
+      int z2 = 0;
+      ItemDigits dig1 = dig;
+      if (nxt.valid(args)) {
+        dig1.load(args, nxt, z1);
+        load_exps(nxt, z1, &eA1, &eB1);
+        nx2.next(args);
+        if (nx2.valid(args)) {
+          out2 = args.jobs[nx2.jb].out;
+          z2 = args.jobs[nx2.jb].x3;
+        }
+      }
+      if (args.slice_hist && threadIdx.x == 64) atomicAdd(args.slice_hist + sl, 1ull);
       const int ab = NB == 2 ? (int)(n & 1) : 0;
       const uint32_t use = NB == 2 ? (n >> 1) : n;
       // warp-uniform decision: the tcgen05.ld below are .sync.aligned
       if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[ab], use & 1, args.err, abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
-      // Up to five digits the diagonals are summed exactly in int64 by
-      // Horner's rule, acc = sum_d D_d 2^(7(sl-1-d)) (|D_d| < 2^31: below
-      // 2^60), and converted once; 6- and 7-digit launches, and the 96-column
-      // tile (whose int64 sums would spill at 80 registers), sum in FP64.
-      // acc holds the int64 sum, or the FP64 bits of the FP64 sum.
-      constexpr int H = S <= 5 && EBN <= 80 ? S : 0;
-      auto cvt = [](long long x) {
-        if constexpr (S <= 3) {  // |x| < 2^46: exact through the 2^52 + 2^51 bias
-          return __longlong_as_double(x + 0x4338000000000000LL) - 6755399441055744.0;
-        } else {
-          return __ll2double_rn(x);
-        }
-      };
+      // Pairs of diagonals first, D_d 128 + D_d+1 (one widening multiply-add
+      // each), then the pairs.  (Loading every diagonal before one wait, to
+      // hold the tensor memory for less, spilled at 96 registers: 7 digits
+      // 1.32 -> 1.39 ms a tuple at no24-nu320.)
       long long acc[CW];
 #pragma unroll
       for (int c0 = 0; c0 < CW; c0 += 16) {
         const int w = CW - c0 >= 16 ? 16 : (CW - c0 >= 8 ? 8 : 4);  // chunk widths 16, then 8 or 4
-#pragma unroll
-        for (int d0 = 0; d0 < S; d0++) {
-          if (d0 >= sl) break;  // diagonals past the item's digit count were not written
-          uint32_t v[16];
-          const uint32_t addr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((ab * S + d0) * EBN + cbase + c0);
+        uint32_t v[2][16];
+        auto load = [&](int d) {
+          const uint32_t addr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((ab * S + d) * EBN + cbase + c0);
           if (w == 16)
-            tmem_ld16(addr, v);
+            tmem_ld16(addr, v[d & 1]);
           else if (w == 8)
-            tmem_ld8(addr, v);
+            tmem_ld8(addr, v[d & 1]);
           else
-            tmem_ld4(addr, v);
-          asm volatile("tcgen05.wait::ld.sync.aligned;");
+            tmem_ld4(addr, v[d & 1]);
+        };
 #pragma unroll
-          for (int j = 0; j < 16; j++) {
-            if (j >= w) continue;
-            const long long dv = (long long)(int32_t)v[j];
-            if constexpr (H > 0) {
-              acc[c0 + j] = d0 == 0 ? dv : (acc[c0 + j] << 7) + dv;
-            } else {
-              const double a = d0 == 0 ? 0.0 : __longlong_as_double(acc[c0 + j]);
-              acc[c0 + j] = __double_as_longlong(fma((double)dv, cd[d0], a));
+        for (int d = 0; d < S; d += 2) {
+          if (d >= sl) break;  // diagonals past the item's digit count were not written
+          const bool pair = d + 1 < S && d + 1 < sl;
+          load(d);
+          if (pair) load(d + 1);
+          asm volatile("tcgen05.wait::ld.sync.aligned;");
+          if (pair) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+              if (j >= w) continue;
+              const long long p = (long long)(int)v[0][j] * 128 + (int)v[1][j];
+              acc[c0 + j] = d == 0 ? p : (acc[c0 + j] << 14) + p;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+              if (j >= w) continue;
+              const int dv = (int)v[0][j];
+              long long &x = acc[c0 + j];
+              x = d == 0 ? (long long)dv
+                  : d < 6 ? (x << 7) + dv
+                          : __double_as_longlong(fma(__ll2double_rn(x), 128.0, (double)dv));
             }
           }
         }
@@ -508,30 +683,39 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[ab]);
-      if (live) {
-        const int16_t *eB = args.expF + (int64_t)job.x3 * args.NPe + n0;
-        const int e0 = eA + (H > 0 ? 2 - 7 * (sl + 1) : 0);
-        auto val = [&](int j) { return (H > 0 ? cvt(acc[j]) : __longlong_as_double(acc[j])) * pow2(e0 + eB[j]); };
-        // one 32-byte sector per store (a thread owns a row, so 16-byte
-        // stores wrote half a sector each and doubled the write traffic)
-        if (args.xblocked) {  // a quad of columns (s % 4 == 0) stays inside one block
-          const int64_t pp = m / args.nu, qq = m - pp * args.nu;
-          double *xb = job.out + xblock_base(pp >> 3, qq >> 3, 0, args.nu, args.NP) + ((pp & 7) * 8 + (qq & 7)) * 8;
-#pragma unroll
-          for (int j = 0; j < CW; j += 4) {
-            const int64_t sc = n0 + j;
-            if (sc >= args.NP) break;
-            st_global_v4(xb + (sc >> 3) * 512 + (sc & 7), val(j), val(j + 1), val(j + 2), val(j + 3));
-          }
+      auto value = [&](int j) {
+        if constexpr (S <= 3) {  // |x| < 2^46: exact through the 2^52 + 2^51 bias
+          return __longlong_as_double(acc[j] + 0x4338000000000000LL) - 6755399441055744.0;
         } else {
-          double *xrow = job.out + m * args.NP + n0;
-#pragma unroll
-          for (int j = 0; j < CW; j += 4) {
-            if (n0 + j >= args.NP) break;  // NP is a multiple of 4: a quad is stored whole or not at all
-            st_global_v4(xrow + j, val(j), val(j + 1), val(j + 2), val(j + 3));
-          }
+          return S == 7 && sl == 7 ? __longlong_as_double(acc[j]) : __ll2double_rn(acc[j]);
         }
-      }
+      };
+      // One 32-byte sector per store (a thread owns a row, so 16-byte stores
+      // wrote half a sector each and doubled the write traffic); a quad of
+      // columns stays inside one block.  NP is a multiple of 4: a quad is
+      // stored whole or not at all.
+      auto store = [&](auto scale) {
+#pragma unroll
+        for (int j = 0; j < CW; j += 4) {
+          double x[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) x[u] = value(j + u) * scale(__shfl_sync(0xffffffffu, eBl, j + u));
+          const int sc = n0 + j;
+          if (live && sc < (int)args.NP)
+            st_global_v4(xrow + (args.xblocked ? (sc >> 3) * 512 + (sc & 7) : sc), x[0], x[1], x[2], x[3]);
+        }
+      };
+      if (normal)
+        store([&](int e) { return __hiloint2double((e0 + 1023 + e) << 20, 0); });
+      else
+        store([&](int e) { return pow2(e0 + e); });
+      dig = dig1;
+      sl = dig.digits<S>(args);
+      out = out1;
+      out1 = out2;
+      z1 = z2;
+      cur = nxt;
+      nxt = nx2;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -769,6 +953,10 @@ int launch_emu_s(const EmuOperands &o, const Dims &d, const EmuJob *jobs_dev, in
   }
   a.err = err;
   const int64_t items = (int64_t)njobs * a.tiles_m * a.tiles_n;
+  if (items > 0x7fffffff) {
+    set_error("too many W-build tiles in one launch");
+    return CCT_ERR_INVALID;
+  }
   const int grid = (int)(items < g_num_sms[dev] ? items : g_num_sms[dev]);
   wbuild_emu_kernel<S, EBN><<<grid, EMU_THREADS, smem, s>>>(a);
   CCT_CUDA(cudaGetLastError());

@@ -51,15 +51,15 @@ __global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t N
 
 // Sums of one tuple's partials, weighted: tsum[0] = its E[4], then the v1
 // columns of i, j and k (nu each).  Grid (1 + ceil(nu / kFinA), tuple of the
-// group).  Block 0 sums the per-CTA x3 partials (thread t takes partials t,
-// t+256, ... in order, then a tree over the 256 threads); every other block
+// group).  Block 0 sums the per-CTA x3 partials (sum t takes partials t, t+256, ...
+// in order, then a tree over the 256 sums); every other block
 // owns kFinA virtual indices a, one warp per (a, column), each summing the
 // column's v1 partials over all block triples containing a (lane-strided,
 // then a shuffle tree).  The loads of a thread's partials are issued eight at
 // a time ahead of its (ordered) adds.
-// Four virtual indices: 384 threads at 36 registers fit beside a CTA of the
-// emulated W build (576 threads at 80), under which these sums run.
-constexpr int kFinA = 4;
+// Two virtual indices: 192 threads at 40 registers fit beside a CTA of the
+// emulated W build (576 threads at 96), under which these sums run.
+constexpr int kFinA = 2;
 constexpr int kFinThreads = 32 * 3 * kFinA;
 __global__ void __launch_bounds__(kFinThreads) tuple_sum_kernel(int nu, int nb, int64_t ncta, int64_t vsize,
                                                                 const __grid_constant__ TupleGroup grp,
@@ -74,9 +74,9 @@ __global__ void __launch_bounds__(kFinThreads) tuple_sum_kernel(int nu, int nb, 
   double *tsum = tsum_all + (int64_t)blockIdx.y * (1 + 3 * nu);
   if (blockIdx.x == 0) {
     __shared__ double red[256];
-    if (tid < 256) {
+    for (int q = tid; q < 256; q += kFinThreads) {  // 256 partial sums, whatever the threads
       double s = 0.0;
-      for (int64_t c0 = tid; c0 < ncta; c0 += 256 * U) {
+      for (int64_t c0 = q; c0 < ncta; c0 += 256 * U) {
         double v[U];
 #pragma unroll
         for (int u = 0; u < U; u++) v[u] = c0 + 256 * u < ncta ? xpart[c0 + 256 * u] : 0.0;
@@ -84,11 +84,11 @@ __global__ void __launch_bounds__(kFinThreads) tuple_sum_kernel(int nu, int nb, 
         for (int u = 0; u < U; u++)
           if (c0 + 256 * u < ncta) s += v[u];
       }
-      red[tid] = s;
+      red[q] = s;
     }
     __syncthreads();
     for (int st = 128; st > 0; st >>= 1) {
-      if (tid < st) red[tid] += red[tid + st];
+      for (int q = tid; q < st; q += kFinThreads) red[q] += red[q + st];
       __syncthreads();
     }
     if (tid == 0) tsum[0] = weight * red[0];
