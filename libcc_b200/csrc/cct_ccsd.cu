@@ -13,12 +13,11 @@
 //   T2(i,y,z,j) += X_j(y,z,i) - sum_k O1(k,z) P_j(i,k,y) - sum_k O1(k,y) Q_j(i,z,k),
 //   X_j(p,q,i) = sum_x (x q|p j) O1(i,x),   P_j(i,k,y) = sum_x O1(i,x) VL(k,x,y,j),
 //   Q_j(i,z,k) = sum_x O1(i,x) VR(z,k,x,j).
-// X_j for all j is one launch of the FP64 W-build tile with its row operand
-// gathered from the packed triangle (the packed-VVVO path: row (p,q) of
-// occupied j at k is (k q|p j)) against O1 as the column operand: 2 no^2 nu^3
-// flops on the tensor pipe instead of 6 no^2 nu^3 on the FP64 units, and the
-// packed slices read once instead of an expanded nu^3 slice written and read
-// per j.  P and Q (no^2 nu per j) and the combination are small kernels.
+// X_j is 2 no^2 nu^3 flops on the tensor pipe instead of 6 no^2 nu^3, read from
+// the packed slices without expanding them.  For no <= 32 one kernel forms
+// X_j and P_j for a (y, j) and adds both to T2 (f4_x_kernel), a second one Q_j
+// and its product for eight z (f4_qt_kernel); larger no runs the W-build tile on
+// gathered rows and element-wise kernels.
 //
 // terms_32_33_34_35:
 //   t2 <- t2^T as an (nou x nou) matrix                            (TRANSQ)
@@ -79,153 +78,339 @@ __global__ void f4_pq_kernel(int no, int nu, const double *__restrict__ o1, cons
   }
 }
 
-// The same steps for no <= kNoTile, staged in shared memory so that global
-// accesses are coalesced runs.
+// ---- no <= kNoTile: the products with O1 on the FP64 tensor pipe
+// (mma.sync.m16n8k4), NT = ceil(no / 8) column fragments.
 constexpr int kNoTile = 32;
-// P[j][y][.][.] for one (y, j) per CTA: the contiguous VL(., ., y, j) slab and
-// O1 pass through shared memory 32 virtual indices x at a time.
-__global__ void __launch_bounds__(256) f4_p_tiled_kernel(int no, int nu, const double *__restrict__ o1,
-                                                         const double *__restrict__ vl, double *__restrict__ P) {
-  constexpr int XC = 32;
-  __shared__ double vs[XC][kNoTile], os[XC][kNoTile];
-  const int y = blockIdx.x, j = blockIdx.y, tid = threadIdx.x;
-  const int i = tid & 31, kq = tid >> 5;
-  const double *slab = vl + (int64_t)no * nu * (y + (int64_t)nu * j);  // VL(k, x, y, j) = slab[k + no x]
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int x0 = 0; x0 < nu; x0 += XC) {
-    __syncthreads();
-    for (int e = tid; e < XC * kNoTile; e += 256) {
-      const int x = e / kNoTile, c = e % kNoTile;
-      const bool ok = x0 + x < nu && c < no;
-      vs[x][c] = ok ? slab[c + (int64_t)no * (x0 + x)] : 0.0;
-      os[x][c] = ok ? o1[c + (int64_t)no * (x0 + x)] : 0.0;
+
+__device__ __forceinline__ void cp8(double *smem, const double *gmem, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
+               "l"(gmem), "r"(ok ? 8 : 0));
+}
+
+// O1 in fragment order, so a warp's fragment is one contiguous 256-byte load:
+//   ob[x / 4][j][lane] = O1(8 j + lane / 4, x + lane % 4)      column operand, K = x
+//   oa[y / 16][k / 4][h][lane] = O1(k + lane % 4, y + 8 h + lane / 4)  row operand, K = k
+// zero past (no, nu); x runs to a multiple of 16.
+__global__ void f4_o1frag_kernel(int no, int nu, int nt, int k4, int64_t nob, int64_t noa,
+                                 const double *__restrict__ o1, double *__restrict__ ob, double *__restrict__ oa) {
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nob + noa;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const bool b = e < nob;
+    const int64_t r = b ? e : e - nob;
+    const int lane = (int)(r & 31), g = lane >> 2, t = lane & 3;
+    const int64_t f = r >> 5;
+    int64_t i, x;
+    if (b) {
+      i = 8 * (f % nt) + g;
+      x = 4 * (f / nt) + t;
+    } else {
+      i = 4 * ((f / 2) % k4) + t;
+      x = 16 * (f / 2 / k4) + 8 * (f & 1) + g;
     }
-    __syncthreads();
-#pragma unroll 8
-    for (int x = 0; x < XC; x++) {
-      const double o = os[x][i];
-#pragma unroll
-      for (int u = 0; u < 4; u++) acc[u] = fma(vs[x][kq + 8 * u], o, acc[u]);
-    }
-  }
-  double *pj = P + ((int64_t)j * nu + y) * no * no;
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    const int k = kq + 8 * u;
-    if (k < no && i < no) pj[(int64_t)k * no + i] = acc[u];
+    const double v = i < no && x < nu ? o1[i + (int64_t)no * x] : 0.0;
+    (b ? ob : oa)[r] = v;
   }
 }
 
-// Q[j][z][.][.] for eight consecutive z and one j per CTA: VR(z..z+7, k, x, j)
-// are 64-byte runs, staged 16 x at a time.
-__global__ void __launch_bounds__(256) f4_q_tiled_kernel(int no, int nu, const double *__restrict__ o1,
-                                                         const double *__restrict__ vr, double *__restrict__ Q) {
-  constexpr int XC = 16, ZT = 8;
-  __shared__ double vs[XC][kNoTile][ZT], os[XC][kNoTile];
-  const int z0 = blockIdx.x * ZT, j = blockIdx.y, tid = threadIdx.x;
-  const int i = tid & 31, zz = tid >> 5;
+// X_j(p, q, i) = sum_x (x q|p j) O1(i, x) for one (p, j) per CTA; T2 form (t2
+// set): T2(i,p,q,j) += X_j(p,q,i) - sum_k O1(k,q) P(i,k), P(i,k) = sum_x O1(i,x)
+// VL(k,x,p,j); else X goes to X[(j nu^2 + p nu + q) np + i].
+//
+// The packed triangle of (p, j) holds (x q) once, row max(x,q).  A warp owns 32
+// rows q, two 16-row blocks; per 16 x each block is 16 rows of the triangle's
+// 128-byte runs whichever side of the diagonal it lies on (rows q right of
+// it, rows x left of it, kept transposed in shared memory), so every global read
+// is coalesced; blocks on the diagonal are read element by element.  Element
+// (r, c) of a block lies at 16 r + (c ^ 4 (r & 3)), r the triangle row: the
+// fragment reads hit sixteen bank pairs either way.  Runs start on any 8-byte
+// boundary, hence 8-byte copies.  Warps share nothing in the main loop, so there is no
+// barrier in it; ten warps and two CTAs on an SM keep the packed slices of a
+// whole wave (2 x 148 of 0.4 MB at nu = 320) near the size of L2, where the second
+// of an element's two reads finds it.
+// Bound: the FP64 tensor pipe (3.8e10 flop at no24-nu320: 1.0 ms).  There the
+// X GEMM on rows gathered through the triangle index, P and the T2 pass took 4.07 ms, this
+// kernel 1.99 ms.
+constexpr int kXW = 10;        // warps
+constexpr int kXStages = 2;    // 16-x chunks in flight per warp
+constexpr int kXSmem = kXW * kXStages * 2 * 256 * 8;
+static_assert(kXStages * 2 * 256 >= kNoTile * kNoTile, "the warps' sums of P fit");
+template <int NT>
+__global__ void __launch_bounds__(kXW * 32, 2)
+    f4_x_kernel(int no, uint32_t nu, int k4, const double *__restrict__ vvvo, const double *__restrict__ ob,
+                const double *__restrict__ oa, const double *__restrict__ vl, double *__restrict__ t2,
+                double *__restrict__ X, int64_t np) {
+  extern __shared__ __align__(16) double xsm[];
+  __shared__ double ps[kNoTile][NT * 8];  // -P(i, k) at [k][i]
+  const int p = blockIdx.x, j = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nk = (nu + 15) / 16;  // x chunks
+  const double *tri = vvvo + ((int64_t)j * nu + p) * ((int64_t)nu * (nu + 1) / 2);
+  if (t2) {
+    // P: every warp takes each tenth four of the x, all (k, i); the warps'
+    // sums are added in order.  (A (16 k, 8 i) tile per warp over every x
+    // left ten warps waiting on six chains of loads: 0.6 ms of the launch.)
+    const double *slab = vl + (int64_t)no * nu * (p + (int64_t)nu * j);  // VL(k, x, p, j) = slab[k + no x]
+    double acc[2][NT][4];
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+      for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int r = 0; r < 4; r++) acc[m][n][r] = 0.0;
+#pragma unroll 2
+    for (int ks = warp; ks < 4 * nk; ks += kXW) {
+      const int x = 4 * ks + t;
+      double a[4], bf[NT];
+#pragma unroll
+      for (int q = 0; q < 4; q++) a[q] = 8 * q + g < no && x < nu ? slab[8 * q + g + (int64_t)no * x] : 0.0;
+#pragma unroll
+      for (int n = 0; n < NT; n++) bf[n] = __ldg(ob + ((int64_t)ks * NT + n) * 32 + lane);
+#pragma unroll
+      for (int n = 0; n < NT; n++) {
+        wb::dmma_16x8x4(acc[0][n], a[0], a[1], bf[n]);
+        if (NT > 2) wb::dmma_16x8x4(acc[1][n], a[2], a[3], bf[n]);
+      }
+    }
+    double *part = xsm + warp * (kNoTile * NT * 8);
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+      for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          part[(16 * m + g + 8 * (r >> 1)) * (NT * 8) + 8 * n + 2 * t + (r & 1)] = acc[m][n][r];
+    __syncthreads();
+    for (int e = threadIdx.x; e < kNoTile * NT * 8; e += kXW * 32) {
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < kXW; w++) v += xsm[w * (kNoTile * NT * 8) + e];
+      (&ps[0][0])[e] = -v;
+    }
+    __syncthreads();
+  }
+  double *mine = xsm + warp * (kXStages * 2 * 256);
+  const int lr = lane >> 4, lc = lane & 15;
+  for (int qb = 32 * warp; qb < nu; qb += 32 * kXW) {
+    double acc[2][NT][4];
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+      for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int r = 0; r < 4; r++) acc[m][n][r] = 0.0;
+    auto load = [&](int c) {  // chunk c into its ring slot
+      const int x0 = 16 * c;
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        double *dst = mine + ((c & (kXStages - 1)) * 2 + m) * 256;
+        const int q0 = qb + 16 * m;
+        if (x0 == q0) {  // the diagonal block, rows q
+#pragma unroll
+          for (int it = 0; it < 8; it++) {
+            const int r = lr + 2 * it, q = q0 + r, x = x0 + lc;
+            const uint32_t hi = max(q, x), lo = min(q, x);  // nu <= 4096: triangle offsets below 2^24
+            cp8(dst + 16 * r + (lc ^ ((r & 3) << 2)), tri + (hi < nu ? hi * (hi + 1) / 2 + lo : 0), hi < nu);
+          }
+        } else {  // rows of the triangle R0 .., columns C0 .. < R0
+          const int R0 = max(x0, q0), C = min(x0, q0) + lc;
+#pragma unroll
+          for (int it = 0; it < 8; it++) {
+            const uint32_t r = lr + 2 * it, row = R0 + r;
+            cp8(dst + 16 * r + (lc ^ ((r & 3) << 2)), tri + (row < nu ? row * (row + 1) / 2 + C : 0), row < nu);
+          }
+        }
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < kXStages - 1; c++) {
+      if (c < nk) load(c);
+      wb::cp_async_commit();
+    }
+    for (int c = 0; c < nk; c++) {
+      if (c + kXStages - 1 < nk) load(c + kXStages - 1);
+      wb::cp_async_commit();
+      wb::cp_async_wait<kXStages - 1>();
+      __syncwarp();
+      const double *src = mine + (c & (kXStages - 1)) * 512;
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++) {
+        double b[NT];
+#pragma unroll
+        for (int n = 0; n < NT; n++) b[n] = __ldg(ob + ((int64_t)(4 * c + kk) * NT + n) * 32 + lane);
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+          const double *blk = src + m * 256;
+          const int x = 4 * kk + t;
+          double a0, a1;
+          if (16 * c > qb + 16 * m) {  // rows x: the block is kept transposed
+            a0 = blk[16 * x + (g ^ ((x & 3) << 2))];
+            a1 = blk[16 * x + ((g + 8) ^ ((x & 3) << 2))];
+          } else {
+            a0 = blk[16 * g + (x ^ ((g & 3) << 2))];
+            a1 = blk[16 * (g + 8) + (x ^ ((g & 3) << 2))];
+          }
+#pragma unroll
+          for (int n = 0; n < NT; n++) wb::dmma_16x8x4(acc[m][n], a0, a1, b[n]);
+        }
+      }
+      __syncwarp();  // the slot is refilled by the next iteration's load
+    }
+    wb::cp_async_wait<0>();
+    if (t2) {
+      for (int kk = 0; kk < k4; kk++) {
+        double b[NT];
+#pragma unroll
+        for (int n = 0; n < NT; n++) b[n] = ps[4 * kk + t][8 * n + g];
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+          const int64_t yt = qb / 16 + m;
+          if (16 * yt >= nu) continue;
+          const double *a = oa + ((yt * k4 + kk) * 2) * 32 + lane;
+          const double a0 = __ldg(a), a1 = __ldg(a + 32);
+#pragma unroll
+          for (int n = 0; n < NT; n++) wb::dmma_16x8x4(acc[m][n], a0, a1, b[n]);
+        }
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int q = qb + 16 * m + g + 8 * h;
+        if (q >= nu) continue;
+        double *row = t2 ? t2 + (int64_t)no * (p + (int64_t)nu * (q + (int64_t)nu * j))
+                         : X + (((int64_t)j * nu + p) * nu + q) * np;
+        double old[NT][2];
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            const int i = 8 * n + 2 * t + r;
+            old[n][r] = t2 && i < no ? row[i] : 0.0;
+          }
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            const int i = 8 * n + 2 * t + r;
+            if (i < no) row[i] = old[n][r] + acc[m][n][2 * h + r];
+          }
+      }
+  }
+}
+
+// T2(i,y,z,j) -= sum_k O1(k,y) Q(i,z,k), Q(i,z,k) = sum_x O1(i,x) VR(z,k,x,j),
+// for eight z and one j per CTA, one z per warp: VR(z .. z+7, k, x, j) are
+// 64-byte runs, staged 8 x at a time; the warp's Q then is the column operand
+// of its z's T2 slab, which is one contiguous run over (i, y).  Element (z, k)
+// of an x lies at 33 z + k, an x every 268 doubles: fragment reads (k = 0..3 by x
+// = 0..3) hit sixteen bank pairs, the copies at most two to a pair.
+// Bound: HBM, VR once and T2 read and written (1.4 GB at no24-nu320: 0.21 ms).  0.52 ms
+// there; Q and the T2 pass as two kernels took 1.91 ms.
+constexpr int kQX = 8, kQPitch = 268, kQStages = 3;
+constexpr int kQSmem = 8 * kNoTile * kNoTile * 8;  // the ring, later the warps' Q
+static_assert(kQStages * kQX * kQPitch <= 8 * kNoTile * kNoTile, "the ring fits");
+template <int NT>
+__global__ void __launch_bounds__(256, 2)
+    f4_qt_kernel(int no, int nu, int k4, const double *__restrict__ ob, const double *__restrict__ oa,
+                 const double *__restrict__ vr, double *__restrict__ t2) {
+  extern __shared__ __align__(16) double qsm[];
+  const int z0 = blockIdx.x * 8, j = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nc = (nu + kQX - 1) / kQX;
   const int64_t nuno = (int64_t)nu * no;
-  double acc[kNoTile];
-#pragma unroll
-  for (int k = 0; k < kNoTile; k++) acc[k] = 0.0;
-  for (int x0 = 0; x0 < nu; x0 += XC) {
-    __syncthreads();
-    for (int e = tid; e < XC * kNoTile * ZT; e += 256) {
-      const int z = e % ZT, k = (e / ZT) % kNoTile, x = e / (ZT * kNoTile);
-      const bool ok = x0 + x < nu && k < no && z0 + z < nu;
-      vs[x][k][z] = ok ? vr[(z0 + z) + (int64_t)nu * k + nuno * (x0 + x) + nuno * nu * j] : 0.0;
+  const double *src = vr + nuno * nu * j;
+  auto load = [&](int c) {
+    double *dst = qsm + (c % kQStages) * (kQX * kQPitch);
+    for (int e = threadIdx.x; e < kQX * kNoTile * 8; e += 256) {
+      const int z = e & 7, k = (e >> 3) & (kNoTile - 1), xl = e >> 8, x = c * kQX + xl;
+      if (k >= no) continue;  // (rows past no of a fragment are never stored)
+      const bool ok = x < nu && z0 + z < nu;
+      cp8(dst + xl * kQPitch + 33 * z + k, src + (ok ? (z0 + z) + (int64_t)nu * k + nuno * x : 0), ok);
     }
-    for (int e = tid; e < XC * kNoTile; e += 256) {
-      const int x = e / kNoTile, c = e % kNoTile;
-      os[x][c] = (x0 + x < nu && c < no) ? o1[c + (int64_t)no * (x0 + x)] : 0.0;
-    }
-    __syncthreads();
-    for (int x = 0; x < XC; x++) {
-      const double o = os[x][i];
+  };
+  double acc[2][NT][4];
 #pragma unroll
-      for (int k = 0; k < kNoTile; k++) acc[k] = fma(vs[x][k][zz], o, acc[k]);
-    }
-  }
-  const int z = z0 + zz;
-  if (z < nu && i < no) {
-    double *qz = Q + ((int64_t)j * nu + z) * no * no;
+  for (int m = 0; m < 2; m++)
 #pragma unroll
-    for (int k = 0; k < kNoTile; k++)
-      if (k < no) qz[(int64_t)k * no + i] = acc[k];
-  }
-}
-
-// T2(i,y,z,j) += X_j(y,z,i) - sum_k O1(k,z) P[j][y][k][i] for one (y, j) per
-// CTA and every z (P[j][y] in shared memory, O1(., z) through the read-only
-// cache: a warp reads one z's column); four z at a time, so their loads are
-// in flight together.
-__global__ void __launch_bounds__(256) f4_t2p_tiled_kernel(int no, int nu, int64_t np,
-                                                           const double *__restrict__ o1,
-                                                           const double *__restrict__ X,
-                                                           const double *__restrict__ P, double *__restrict__ t2) {
-  __shared__ double ps[kNoTile][kNoTile];
-  const int y = blockIdx.x, j = blockIdx.y, tid = threadIdx.x;
-  const int i = tid & 31, zg = tid >> 5;
-  const double *pj = P + ((int64_t)j * nu + y) * no * no;
-  for (int e = tid; e < kNoTile * kNoTile; e += 256) {
-    const int k = e / kNoTile, c = e % kNoTile;
-    ps[k][c] = (k < no && c < no) ? pj[(int64_t)k * no + c] : 0.0;
-  }
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) acc[m][n][r] = 0.0;
+  for (int e = threadIdx.x; e < kQStages * kQX * kQPitch; e += 256) qsm[e] = 0.0;  // k >= no
   __syncthreads();
-  if (i >= no) return;
-  const int64_t nu2 = (int64_t)nu * nu;
-  constexpr int U = 4;
-  for (int zb = zg; zb < nu; zb += 8 * U) {
-    double v[U], t[U];
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int z = zb + 8 * u;
-      v[u] = z < nu ? X[((int64_t)j * nu2 + (int64_t)y * nu + z) * np + i] : 0.0;
-      t[u] = z < nu ? t2[i + (int64_t)no * (y + (int64_t)nu * (z + (int64_t)nu * j))] : 0.0;
-    }
+  for (int c = 0; c < kQStages - 1; c++) {
+    if (c < nc) load(c);
+    wb::cp_async_commit();
+  }
+  for (int c = 0; c < nc; c++) {
+    wb::cp_async_wait<kQStages - 2>();
+    __syncthreads();
+    if (c + kQStages - 1 < nc) load(c + kQStages - 1);
+    wb::cp_async_commit();
+    const double *buf = qsm + (c % kQStages) * (kQX * kQPitch) + 33 * warp;
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int z = zb + 8 * u;
-      if (z >= nu) break;
-      const double *oz = o1 + (int64_t)no * z;
-      for (int k = 0; k < no; k++) v[u] -= __ldg(oz + k) * ps[k][i];
-      t2[i + (int64_t)no * (y + (int64_t)nu * (z + (int64_t)nu * j))] = t[u] + v[u];
+    for (int kk = 0; kk < kQX / 4; kk++) {
+      double b[NT];
+#pragma unroll
+      for (int n = 0; n < NT; n++) b[n] = __ldg(ob + ((int64_t)(c * (kQX / 4) + kk) * NT + n) * 32 + lane);
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        if (m == 1 && NT <= 2) continue;  // no <= 16
+        const double *a = buf + (4 * kk + t) * kQPitch + 16 * m + g;
+        const double a0 = a[0], a1 = a[8];
+#pragma unroll
+        for (int n = 0; n < NT; n++) wb::dmma_16x8x4(acc[m][n], a0, a1, b[n]);
+      }
     }
   }
-}
-
-// T2(i,y,z,j) -= sum_k O1(k,y) Q[j][z][k][i] for one (z, j) per CTA and every
-// y; T2(., ., z, j) over (i, y) is one contiguous run.
-__global__ void __launch_bounds__(256) f4_t2q_tiled_kernel(int no, int nu, const double *__restrict__ o1,
-                                                           const double *__restrict__ Q, double *__restrict__ t2) {
-  __shared__ double qs[kNoTile][kNoTile];
-  const int z = blockIdx.x, j = blockIdx.y, tid = threadIdx.x;
-  const int i = tid & 31, yg = tid >> 5;
-  const double *qz = Q + ((int64_t)j * nu + z) * no * no;
-  for (int e = tid; e < kNoTile * kNoTile; e += 256) {
-    const int k = e / kNoTile, c = e % kNoTile;
-    qs[k][c] = (k < no && c < no) ? qz[(int64_t)k * no + c] : 0.0;
-  }
-  __syncthreads();
-  if (i >= no) return;
-  double *tz = t2 + (int64_t)no * nu * (z + (int64_t)nu * j);
-  constexpr int U = 4;
-  for (int yb = yg; yb < nu; yb += 8 * U) {
-    double t[U];
+  wb::cp_async_wait<0>();
+  __syncthreads();  // every warp is done with the ring
+  const int z = z0 + warp;
+  if (z >= nu) return;
+  // -Q(i, z, k) at [k][i], the warp's own
+  double *qz = qsm + warp * (kNoTile * kNoTile);
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int y = yb + 8 * u;
-      t[u] = y < nu ? tz[i + (int64_t)no * y] : 0.0;
+  for (int m = 0; m < 2; m++)
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+        qz[(16 * m + g + 8 * (r >> 1)) * kNoTile + 8 * n + 2 * t + (r & 1)] = -acc[m][n][r];
+  __syncwarp();
+  double b[2 * NT][NT];
+#pragma unroll
+  for (int kk = 0; kk < 2 * NT; kk++)
+#pragma unroll
+    for (int n = 0; n < NT; n++) b[kk][n] = qz[(4 * kk + t) * kNoTile + 8 * n + g];
+  double *slab = t2 + nuno * (z + (int64_t)nu * j);
+  const int ny = (nu + 15) / 16;
+  for (int yt = 0; yt < ny; yt++) {
+    // the product is summed on its own and T2 rounded once
+    double c[NT][4], old[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const int y = 16 * yt + g + 8 * (r >> 1), i = 8 * n + 2 * t + (r & 1);
+        old[n][r] = y < nu && i < no ? slab[i + (int64_t)no * y] : 0.0;
+        c[n][r] = 0.0;
+      }
+#pragma unroll
+    for (int kk = 0; kk < 2 * NT; kk++) {
+      if (kk >= k4) break;
+      const double *a = oa + (((int64_t)yt * k4 + kk) * 2) * 32 + lane;
+      const double a0 = __ldg(a), a1 = __ldg(a + 32);
+#pragma unroll
+      for (int n = 0; n < NT; n++) wb::dmma_16x8x4(c[n], a0, a1, b[kk][n]);
     }
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int y = yb + 8 * u;
-      if (y >= nu) break;
-      const double *oy = o1 + (int64_t)no * y;
-      double s = 0.0;
-      for (int k = 0; k < no; k++) s = fma(__ldg(oy + k), qs[k][i], s);
-      tz[i + (int64_t)no * y] = t[u] - s;
-    }
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const int y = 16 * yt + g + 8 * (r >> 1), i = 8 * n + 2 * t + (r & 1);
+        if (y < nu && i < no) slab[i + (int64_t)no * y] = old[n][r] + c[n][r];
+      }
   }
 }
 
@@ -374,18 +559,68 @@ struct DevBuf {  // device copies of host arrays (or the caller's device arrays)
   int tmp(double **dst, int64_t n) { return alloc(reinterpret_cast<void **>(dst), (size_t)n * 8); }
 };
 
+// O1 in fragment order (f4_o1frag_kernel), no <= kNoTile.
+struct O1Frag {
+  int nt, k4;
+  double *ob, *oa;
+};
+int o1_fragments(int64_t no, int64_t nu, const double *d_o1, DevBuf &b, O1Frag *f, cudaStream_t s) {
+  f->nt = (int)((no + 7) / 8);
+  f->k4 = (int)((no + 3) / 4);
+  const int64_t chunks = (nu + 15) / 16, nob = 4 * chunks * f->nt * 32, noa = chunks * f->k4 * 64;
+  CCT_TRY(b.tmp(&f->ob, nob));
+  CCT_TRY(b.tmp(&f->oa, noa));
+  f4_o1frag_kernel<<<grid_of(nob + noa), 256, 0, s>>>((int)no, (int)nu, f->nt, f->k4, nob, noa, d_o1, f->ob, f->oa);
+  CCT_CUDA(cudaGetLastError());
+  return CCT_OK;
+}
+
+template <int NT>
+int launch_x(int64_t no, int64_t nu, const O1Frag &f, const double *vvvo, const double *vl, double *t2, double *X,
+             int64_t np, cudaStream_t s) {
+  CCT_CUDA(cudaFuncSetAttribute(f4_x_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem));
+  f4_x_kernel<NT><<<dim3((unsigned)nu, (unsigned)no), kXW * 32, kXSmem, s>>>((int)no, (int)nu, f.k4, vvvo, f.ob, f.oa,
+                                                                            vl, t2, X, np);
+  CCT_CUDA(cudaGetLastError());
+  return CCT_OK;
+}
+// vl and t2 set: the T2 update; else X (rows of np doubles).
+int launch_x(int64_t no, int64_t nu, const O1Frag &f, const double *vvvo, const double *vl, double *t2, double *X,
+             int64_t np, cudaStream_t s) {
+  switch (f.nt) {
+    case 1: return launch_x<1>(no, nu, f, vvvo, vl, t2, X, np, s);
+    case 2: return launch_x<2>(no, nu, f, vvvo, vl, t2, X, np, s);
+    case 3: return launch_x<3>(no, nu, f, vvvo, vl, t2, X, np, s);
+    default: return launch_x<4>(no, nu, f, vvvo, vl, t2, X, np, s);
+  }
+}
+template <int NT>
+int launch_qt(int64_t no, int64_t nu, const O1Frag &f, const double *vr, double *t2, cudaStream_t s) {
+  CCT_CUDA(cudaFuncSetAttribute(f4_qt_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQSmem));
+  f4_qt_kernel<NT><<<dim3((unsigned)((nu + 7) / 8), (unsigned)no), 256, kQSmem, s>>>((int)no, (int)nu, f.k4, f.ob,
+                                                                                     f.oa, vr, t2);
+  CCT_CUDA(cudaGetLastError());
+  return CCT_OK;
+}
+
 // X_j(p,q,i) = sum_x (x q|p j) O1(i,x) for every occupied j, X_j at x + j nu^2 np,
-// row (p,q) at (p nu + q) np: the W-build tile, one packed-row job per j.
+// row (p,q) at (p nu + q) np: f4_x_kernel, or for no > kNoTile the W-build
+// tile, one packed-row job per j.
 int packed_o1_gemm(int64_t no, int64_t nu, const double *d_o1, const double *d_vvvo, DevBuf &b, double **X,
                    int64_t *np_out, cudaStream_t s) {
   const int64_t nutr = nu * (nu + 1) / 2;
+  if (no <= kNoTile) {
+    O1Frag f;
+    CCT_TRY(o1_fragments(no, nu, d_o1, b, &f, s));
+    *np_out = 8 * f.nt;
+    CCT_TRY(b.tmp(X, no * nu * nu * *np_out));
+    return launch_x(no, nu, f, d_vvvo, nullptr, nullptr, *X, *np_out, s);
+  }
   Dims g{};
   g.nu = (int)nu;                  // M = nu^2 rows (p, q)
   g.no = 0;                        // K = nu (the packed part of a row alone)
   g.KP = round_up(nu, kKB);
-  // N = no: a 24-column tile when no pads to 24 (no waste at no = 24, where
-  // the smallest plan tile, 32, computes a quarter of padding)
-  g.BN = round_up(no, 8) == 24 ? 24 : choose_bn((int)no);
+  g.BN = choose_bn((int)no);
   g.NP = round_up(no, g.BN);
   double *o1pad;
   CCT_TRY(b.tmp(&o1pad, g.NP * g.KP));
@@ -434,21 +669,22 @@ extern "C" int ccT_ccsd_terms_29_31(int64_t no, int64_t nu, const double *o1, do
   CCT_TRY(b.get(&d_vl, vl, no * nu2 * no, mem, true, s));
   CCT_TRY(b.get(&d_vr, vr, nu * no * nu * no, mem, true, s));
   CCT_TRY(b.get(&d_vvvo, vvvo, nutr * nu * no, mem, true, s));
-  double *X, *P, *Q;
-  int64_t np = 0;
-  CCT_TRY(packed_o1_gemm(no, nu, d_o1, d_vvvo, b, &X, &np, s));
-  CCT_TRY(b.tmp(&P, no * no * nu * no));
-  CCT_TRY(b.tmp(&Q, no * no * nu * no));
   if (no <= kNoTile) {
-    f4_p_tiled_kernel<<<dim3((unsigned)nu, (unsigned)no), 256, 0, s>>>((int)no, (int)nu, d_o1, d_vl, P);
-    CCT_CUDA(cudaGetLastError());
-    f4_q_tiled_kernel<<<dim3((unsigned)((nu + 7) / 8), (unsigned)no), 256, 0, s>>>((int)no, (int)nu, d_o1, d_vr, Q);
-    CCT_CUDA(cudaGetLastError());
-    f4_t2p_tiled_kernel<<<dim3((unsigned)nu, (unsigned)no), 256, 0, s>>>((int)no, (int)nu, np, d_o1, X, P, d_t2);
-    CCT_CUDA(cudaGetLastError());
-    f4_t2q_tiled_kernel<<<dim3((unsigned)nu, (unsigned)no), 256, 0, s>>>((int)no, (int)nu, d_o1, Q, d_t2);
-    CCT_CUDA(cudaGetLastError());
+    O1Frag f;
+    CCT_TRY(o1_fragments(no, nu, d_o1, b, &f, s));
+    CCT_TRY(launch_x(no, nu, f, d_vvvo, d_vl, d_t2, nullptr, 0, s));
+    switch (f.nt) {
+      case 1: CCT_TRY(launch_qt<1>(no, nu, f, d_vr, d_t2, s)); break;
+      case 2: CCT_TRY(launch_qt<2>(no, nu, f, d_vr, d_t2, s)); break;
+      case 3: CCT_TRY(launch_qt<3>(no, nu, f, d_vr, d_t2, s)); break;
+      default: CCT_TRY(launch_qt<4>(no, nu, f, d_vr, d_t2, s)); break;
+    }
   } else {
+    double *X, *P, *Q;
+    int64_t np = 0;
+    CCT_TRY(packed_o1_gemm(no, nu, d_o1, d_vvvo, b, &X, &np, s));
+    CCT_TRY(b.tmp(&P, no * no * nu * no));
+    CCT_TRY(b.tmp(&Q, no * no * nu * no));
     f4_pq_kernel<<<grid_of(2 * no * no * nu * no), 256, 0, s>>>((int)no, (int)nu, d_o1, d_vl, d_vr, P, Q);
     CCT_CUDA(cudaGetLastError());
     f4_t2_kernel<<<grid_of(no * nu2 * no), 256, 0, s>>>((int)no, (int)nu, np, d_o1, X, P, Q, d_t2);
@@ -527,8 +763,16 @@ extern "C" int ccT_ccsd_terms_32_35(int64_t no, int64_t nu, const double *o1, do
   CCT_TRY(b.tmp(&bpad, nsplit * g.NP * g.KP));
   CCT_TRY(b.tmp(&t, nsplit * no * no * g.NP));
   CCT_CUDA(cudaMemcpyAsync(o2in, d_o2, (size_t)n4 * 8, cudaMemcpyDeviceToDevice, s));
-  CCT_CUDA(cudaMemsetAsync(apad, 0, (size_t)nsplit * no * no * g.KP * 8, s));
-  CCT_CUDA(cudaMemsetAsync(bpad, 0, (size_t)nsplit * g.NP * g.KP * 8, s));
+  // zero the padding: columns of a split past nu^2, rows past nu no
+  for (int z = 0; z < nsplit; z++) {
+    const int64_t left = nu2 - z * g.KP, used = left < 0 ? 0 : (left < g.KP ? left : g.KP);
+    double *az = apad + (int64_t)z * no * no * g.KP, *bz = bpad + (int64_t)z * g.NP * g.KP;
+    if (used < g.KP) {
+      CCT_CUDA(cudaMemset2DAsync(az + used, (size_t)g.KP * 8, 0, (size_t)(g.KP - used) * 8, (size_t)(no * no), s));
+      CCT_CUDA(cudaMemset2DAsync(bz + used, (size_t)g.KP * 8, 0, (size_t)(g.KP - used) * 8, (size_t)nou, s));
+    }
+    if (g.NP > nou) CCT_CUDA(cudaMemsetAsync(bz + nou * g.KP, 0, (size_t)(g.NP - nou) * g.KP * 8, s));
+  }
   f4_o2_kernel<<<grid_of(n4), 256, 0, s>>>((int)no, (int)nu, g.KP, o2in, d_o2, apad);
   CCT_CUDA(cudaGetLastError());
   {
