@@ -74,7 +74,9 @@ struct ccT_plan {
   int64_t xsize = 0;         // doubles per GEMM output
   double *xpart = nullptr, *vpart = nullptr, *tsum = nullptr;  // per tuple of a group
   int16_t *cta_table = nullptr;
-  double *acc = nullptr;  // [etd_sum, etd_comp, out3[3], v1(nu*no)]
+  double *acc = nullptr;  // [etd_sum, etd_comp, out3[3], v1(nu*no)], then flags (16 B) and slice_hist: one block
+  std::vector<double> host_out;  // out3, v1 and flags, as the forward reads them back
+  void *arena = nullptr;         // every buffer of plan_create, one allocation
   GemmJob *jobs = nullptr;  // every tuple's jobs in list order (job_offset)
   bool emulated = false;    // INT8 split-integer W-build
   bool packed = false;      // VVVO kept packed (CCT_VVVO_PACKED): no E; vvvo_res and a slab cache instead
@@ -141,6 +143,44 @@ int dalloc(T **p, size_t count) {
 
 double *v1_acc(ccT_plan *p) { return p->acc + 5; }
 
+// Device buffers collected first and then cut from one allocation (256-byte
+// aligned pieces): some twenty cudaMalloc / cudaFree pairs took most of a small
+// plan's life (no8-nu72: create and destroy 5.0 ms, 1.6 ms as one).
+struct Arena {
+  std::vector<std::pair<void **, size_t>> parts;
+  size_t bytes = 0;
+  template <typename T>
+  void add(T **p, int64_t count) {
+    parts.push_back({reinterpret_cast<void **>(p), bytes});
+    bytes += (std::max<size_t>((size_t)count * sizeof(T), 1) + 255) / 256 * 256;
+  }
+  int allocate(void **block) {
+    CCT_CUDA(cudaMalloc(block, bytes));
+    for (auto &q : parts) *q.first = static_cast<char *>(*block) + q.second;
+    return CCT_OK;
+  }
+};
+
+// The accumulators, flags and digit histogram of a forward, zeroed.
+int clear_results(ccT_plan *p) {
+  const size_t n = 5 + (size_t)p->d.nu * p->d.no;
+  CCT_CUDA(cudaMemsetAsync(p->acc, 0, n * 8 + 16 + (p->emulated ? (kEmuMaxSlices + 1) * 8 : 0), p->stream));
+  return CCT_OK;
+}
+// out3, v1 and flags in one copy; waits for p->stream.
+int read_results(ccT_plan *p, double out3[3], double *v1_out, int *werr) {
+  const size_t n = (size_t)p->d.nu * p->d.no;
+  p->host_out.resize(3 + n + 2);
+  CCT_CUDA(cudaMemcpyAsync(p->host_out.data(), p->acc + 2, (3 + n + 2) * 8, cudaMemcpyDeviceToHost, p->stream));
+  CCT_CUDA(cudaStreamSynchronize(p->stream));
+  std::memcpy(out3, p->host_out.data(), 3 * 8);
+  if (v1_out) std::memcpy(v1_out, p->host_out.data() + 3, n * 8);
+  int hflags[4];
+  std::memcpy(hflags, p->host_out.data() + 3 + n, 16);
+  *werr = hflags[1];
+  return CCT_OK;
+}
+
 // The FP64 jobs as split-integer jobs: half 0 E[x1] x F[x2][x3], half 1
 // E^T[x2] x F[x1][x3], by occupied index instead of by pointer.
 int upload_emu_jobs(ccT_plan *p, const std::vector<GemmJob> &jobs, EmuJob *dst) {
@@ -175,8 +215,9 @@ double *xbuf(const ccT_plan *p, int64_t t, int g) {
 }
 
 // Tuples per group.  A launch of a small system's tuple leaves most SMs idle:
-// group until a launch has about kGroupTiles W-build tiles (several waves of
-// the 148 SMs), within kMaxGroup tuples and kGroupBytes of X per group; a
+// group until a launch has about kGroupTiles W-build tiles (eight waves of
+// three FP64 CTAs, or 24 tiles of an emulated CTA, on 148 SMs; four FP64 waves
+// took 32.2 ms where eight take 31.2, at no12-nu120), within kMaxGroup tuples and kGroupBytes of X per group; a
 // tuple that has the tiles by itself stays alone (nu >= ~200, where one launch
 // a tuple and groups time the same).  A forward with one tuple a launch
 // against groups: no4-nu36 (16 tuples a group) 302 -> 109 us, no9-nu83
@@ -487,17 +528,14 @@ int run_group(ccT_plan *p, int64_t t0, int64_t t1, bool fp64 = false, int64_t ke
 // the FP64 one.  Leaves the plan's accumulators holding that tuple only.
 int tuple_energy(ccT_plan *p, int64_t tix, bool fp64, double *e) {
   const Dims &d = p->d;
-  CCT_CUDA(cudaMemsetAsync(p->acc, 0, (5 + (int64_t)d.nu * d.no) * 8, p->stream));
-  CCT_CUDA(cudaMemsetAsync(p->flags + 1, 0, 4, p->stream));
+  CCT_TRY(clear_results(p));
   CCT_TRY(fork_streams(p));
   CCT_TRY(run_group(p, tix, tix + 1, fp64));
   CCT_TRY(join_streams(p));
   CCT_TRY(launch_ets(d, p->t1, v1_acc(p), p->acc, p->acc + 2, p->stream));
   double out3[3];
   int werr = 0;
-  CCT_CUDA(cudaMemcpyAsync(&werr, p->flags + 1, 4, cudaMemcpyDeviceToHost, p->stream));
-  CCT_CUDA(cudaMemcpyAsync(out3, p->acc + 2, 3 * 8, cudaMemcpyDeviceToHost, p->stream));
-  CCT_CUDA(cudaStreamSynchronize(p->stream));
+  CCT_TRY(read_results(p, out3, nullptr, &werr));
   if (werr) {
     set_error("a kernel ran out its bounded wait and unwound");
     return CCT_ERR_TIMEOUT;
@@ -786,22 +824,33 @@ static int plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options
   {
     const int64_t bm = p->emulated ? kEmuBM : 128, bn = p->emulated ? d.EBN : d.BN;
     // packed plans: a group could need more slabs than the cache holds
-    p->group = p->packed ? 1 : choose_group(3 * ((nu2 + bm - 1) / bm) * (d.NP / bn), 3 * p->xsize * 8, ntup);
+    p->group = p->packed ? 1
+                         : choose_group(3 * ((nu2 + bm - 1) / bm) * (d.NP / bn), 3 * p->xsize * 8, ntup);
     p->group = std::min(p->group, group_cap);
     p->nring = (int)std::min<int64_t>(kNBuf, (ntup + p->group - 1) / p->group);
   }
-  if ((s = dalloc(&p->eh, no)) || (s = dalloc(&p->ep, nu)) || (s = dalloc(&p->t1, no * nu)) ||
-      (s = dalloc(&p->t2, nu2 * no * no)) || (s = dalloc(&p->vm, no * nu * no * no)) ||
-      (s = dalloc(&p->voe, nu2 * no * no)) || (s = dalloc(&p->vb, vb_size(d))) ||
-      (s = p->packed ? dalloc(&p->vvvo_res, nu * (nu + 1) / 2 * nu * no) : dalloc(&p->E, no * nu2 * d.KP)) ||
-      (s = p->packed ? dalloc(&p->slabs, kSlabs * nu2 * d.KP) : CCT_OK) ||
-      (s = dalloc(&p->F, no * no * d.NP * d.KP)) ||
-      (s = dalloc(&p->X, (int64_t)p->group * p->nring * 3 * p->xsize)) ||
-      (s = dalloc(&p->xpart, p->group * d.ncta)) || (s = dalloc(&p->vpart, p->group * vpart_size(d))) ||
-      (s = dalloc(&p->tsum, p->group * tsum_size(d))) ||
-      (s = dalloc(&p->cta_table, d.ncta * 3)) || (s = dalloc(&p->acc, 5 + nu * no)) ||
-      (s = dalloc(&p->jobs, job_offset(p, ntup))) || (s = dalloc(&p->flags, 4)))
-    return fail(s);
+  Arena mem;
+  mem.add(&p->eh, no);
+  mem.add(&p->ep, nu);
+  mem.add(&p->t1, no * nu);
+  mem.add(&p->t2, nu2 * no * no);
+  mem.add(&p->vm, no * nu * no * no);
+  mem.add(&p->voe, nu2 * no * no);
+  mem.add(&p->vb, vb_size(d));
+  if (p->packed) {
+    mem.add(&p->vvvo_res, nu * (nu + 1) / 2 * nu * no);
+    mem.add(&p->slabs, kSlabs * nu2 * d.KP);
+  } else {
+    mem.add(&p->E, no * nu2 * d.KP);
+  }
+  mem.add(&p->F, no * no * d.NP * d.KP);
+  mem.add(&p->X, (int64_t)p->group * p->nring * 3 * p->xsize);
+  mem.add(&p->xpart, p->group * d.ncta);
+  mem.add(&p->vpart, p->group * vpart_size(d));
+  mem.add(&p->tsum, p->group * tsum_size(d));
+  mem.add(&p->cta_table, d.ncta * 3);
+  mem.add(&p->acc, 5 + nu * no + 2 + kEmuMaxSlices + 1);
+  mem.add(&p->jobs, job_offset(p, ntup));
   if (p->emulated) {
     EmuOperands &e = p->emu;
     e.slices = o.emu_slices ? o.emu_slices : kEmuMaxSlices;
@@ -815,14 +864,19 @@ static int plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options
     e.tiles_m = (nu2 + kEmuBM - 1) / kEmuBM;
     const int64_t rowsE = no * nu2, rowsF = no * no * d.NP;
     const int64_t bytesE = e.slices * no * e.tiles_m * kEmuBM * e.KP8;  // row tiles padded to 128 rows
-    if ((s = dalloc(&e.E8, bytesE)) || (s = dalloc(&e.E8T, bytesE)) ||
-        (s = dalloc(&e.F8, e.slices * rowsF * e.KP8)) || (s = dalloc(&e.expE, rowsE)) ||
-        (s = dalloc(&e.expET, rowsE)) || (s = dalloc(&e.expF, rowsF)) || (s = dalloc(&e.expRowF, rowsF)) ||
-        (s = dalloc(&p->emu_jobs, job_offset(p, ntup))) ||
-        (s = dalloc(&e.tileExp, e.tiles_m + no * (d.NP / d.EBN) + 2)) ||
-        (s = dalloc(&e.slice_hist, kEmuMaxSlices + 1)))
-      return fail(s);
+    mem.add(&e.E8, bytesE);
+    mem.add(&e.E8T, bytesE);
+    mem.add(&e.F8, e.slices * rowsF * e.KP8);
+    mem.add(&e.expE, rowsE);
+    mem.add(&e.expET, rowsE);
+    mem.add(&e.expF, rowsF);
+    mem.add(&e.expRowF, rowsF);
+    mem.add(&p->emu_jobs, job_offset(p, ntup));
+    mem.add(&e.tileExp, e.tiles_m + no * (d.NP / d.EBN) + 2);
   }
+  if ((s = mem.allocate(&p->arena))) return fail(s);
+  p->flags = reinterpret_cast<int *>(p->acc + 5 + nu * no);
+  if (p->emulated) p->emu.slice_hist = reinterpret_cast<unsigned long long *>(p->acc + 5 + nu * no + 2);
   std::vector<int16_t> table(d.ncta * 3);
   int64_t idx = 0;
   for (int C = 0; C < d.nb; C++)
@@ -894,12 +948,17 @@ int ccT_set_inputs(ccT_plan *p, const double *eh, const double *ep, const double
     cuda(cudaMemcpyAsync(p->vvvo_res, vvvo, nvvvo * 8, kind, p->stream), "copy vvvo");
     vvvo_dev = p->vvvo_res;
   } else if (s == CCT_OK && mem == CCT_MEM_HOST) {
-    // the packed VVVO is only needed to build E; stage it in a transient
+    // the packed VVVO is only needed to build E; stage it in the X ring, which
+    // no forward is using now, or where that is too small in a transient
     // buffer.  Plain cudaMalloc/cudaFree: with the stream-ordered pool this
     // call took 0.12-0.21 s at no=24/nu=320 (3.2 GB staged), 0.08-0.10 s so.
-    cuda(cudaMalloc(reinterpret_cast<void **>(&staged), nvvvo * 8), "stage vvvo");
-    if (s == CCT_OK) cuda(cudaMemcpyAsync(staged, vvvo, nvvvo * 8, cudaMemcpyHostToDevice, p->stream), "copy vvvo");
-    vvvo_dev = staged;
+    double *dst = p->X;
+    if (nvvvo > (int64_t)p->group * p->nring * 3 * p->xsize) {
+      cuda(cudaMalloc(reinterpret_cast<void **>(&staged), nvvvo * 8), "stage vvvo");
+      dst = staged;
+    }
+    if (s == CCT_OK) cuda(cudaMemcpyAsync(dst, vvvo, nvvvo * 8, cudaMemcpyHostToDevice, p->stream), "copy vvvo");
+    vvvo_dev = dst;
   }
   if (s == CCT_OK && p->opt.check_inputs) {
     cuda(cudaMemsetAsync(p->flags, 0, 16, p->stream), "clear flags");
@@ -959,10 +1018,7 @@ int ccT_forward(ccT_plan *p, int64_t begin, int64_t end, double *ets, double *et
   DeviceGuard guard(p->device);
   const Dims &d = p->d;
   p->last_launches = 0;
-  CCT_CUDA(cudaMemsetAsync(p->acc, 0, (5 + (int64_t)d.nu * d.no) * 8, p->stream));
-  CCT_CUDA(cudaMemsetAsync(p->flags + 1, 0, 4, p->stream));
-  if (p->emulated)
-    CCT_CUDA(cudaMemsetAsync(p->emu.slice_hist, 0, (kEmuMaxSlices + 1) * sizeof(unsigned long long), p->stream));
+  CCT_TRY(clear_results(p));
   p->keep_begin = p->keep_end = -1;
   bool keep = false;
   if (p->opt.keep_w && !p->emulated && !p->packed && end > begin) CCT_TRY(prepare_keep(p, begin, end, &keep));
@@ -982,11 +1038,7 @@ int ccT_forward(ccT_plan *p, int64_t begin, int64_t end, double *ets, double *et
   CCT_CUDA(cudaEventRecord(p->ev1, p->stream));
   double out3[3];
   int werr = 0;
-  CCT_CUDA(cudaMemcpyAsync(&werr, p->flags + 1, 4, cudaMemcpyDeviceToHost, p->stream));
-  CCT_CUDA(cudaMemcpyAsync(out3, p->acc + 2, 3 * 8, cudaMemcpyDeviceToHost, p->stream));
-  if (v1_out)
-    CCT_CUDA(cudaMemcpyAsync(v1_out, v1_acc(p), (int64_t)d.nu * d.no * 8, cudaMemcpyDeviceToHost, p->stream));
-  CCT_CUDA(cudaStreamSynchronize(p->stream));
+  CCT_TRY(read_results(p, out3, v1_out, &werr));
   CCT_CUDA(cudaEventElapsedTime(&p->last_ms, p->ev0, p->ev1));
   CCT_TRY(prof_collect(p));
   if (ets) *ets = out3[0];
@@ -1327,19 +1379,10 @@ int ccT_plan_destroy(ccT_plan *p) {
   DeviceGuard guard(p->device);
   for (cudaStream_t st : {p->stream, p->gemm_stream, p->gemm_stream2, p->red_stream, p->bwd_stream, p->rec_stream})
     if (st) cudaStreamSynchronize(st);
-  double *bufs[] = {p->eh, p->ep, p->t1, p->t2, p->vm, p->voe, p->E, p->F, p->xpart, p->vpart, p->acc, p->stage,
-                    p->vvvo_res, p->slabs, p->X, p->tsum, p->vb};
-  for (double *b : bufs)
-    if (b) cudaFree(b);
-  if (p->cta_table) cudaFree(p->cta_table);
-  if (p->jobs) cudaFree(p->jobs);
+  if (p->arena) cudaFree(p->arena);
+  if (p->stage) cudaFree(p->stage);
   if (p->xkeep) cudaFree(p->xkeep);
   if (p->keep_jobs) cudaFree(p->keep_jobs);
-  if (p->flags) cudaFree(p->flags);
-  for (void *b : {(void *)p->emu.E8, (void *)p->emu.E8T, (void *)p->emu.F8, (void *)p->emu.expE,
-                  (void *)p->emu.expET, (void *)p->emu.expF, (void *)p->emu.expRowF, (void *)p->emu_jobs,
-                  (void *)p->emu.tileExp, (void *)p->emu.slice_hist})
-    if (b) cudaFree(b);
   adj_free(&p->adj);
   if (p->ev0) cudaEventDestroy(p->ev0);
   if (p->ev1) cudaEventDestroy(p->ev1);
