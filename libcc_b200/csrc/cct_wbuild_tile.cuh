@@ -2,6 +2,8 @@
 // kernel (cct_wbuild_f64.cu) and the persistent batch kernel (cct_batch.cu).
 // See cct_wbuild_f64.cu for the formulation and the reference lines.
 #pragma once
+#include <type_traits>
+
 #include "cct_internal.cuh"
 
 namespace cct {
@@ -36,7 +38,20 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem, int src_
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// cp.async of 16 bytes (zero-filled when !live) to a shared address plus a constant.
+template <int OFF>
+__device__ __forceinline__ void cp_async16_at(uint32_t smem, const void *gmem, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0+%1], [%2], 16, %3;\n" ::"r"(smem), "n"(OFF), "l"(gmem),
+               "r"(live ? 16 : 0));
+}
+template <int OFF>
+__device__ __forceinline__ double lds_at(uint32_t smem) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1+%2];\n" : "=d"(v) : "r"(smem), "n"(OFF));
+  return v;
 }
 
 __device__ __forceinline__ void dmma_16x8x4(double *d, double a0, double a1, double b0) {
@@ -88,23 +103,41 @@ __device__ __forceinline__ void wbuild_tile(const GemmJob &job, int nu, int64_t 
 
   const int ktiles_half = (int)(KP / BK);
   const int ktiles = ktiles_half * job.nhalves;
+  // Shared addresses are a per-thread base plus constants: the rows a thread
+  // copies are NT/8 apart and the rows of a fragment 8 apart, multiples of 4, so
+  // the XOR of a row (r & 3) is the same for all of them.  (Indexing the tiles
+  // through swz() for every copy and fragment, with a K check per step, took
+  // 464 instructions a warp and k-tile beside its 40 MMAs and kept the FP64 pipe
+  // at 0.84: one tuple took 708 us at no16-nu200 and 4.11 ms at no24-nu320, 631 us
+  // and 3.95 ms now.)
+  constexpr int RS = LDS * 8;               // bytes of a row
+  constexpr int A_ST = BM * RS, B_ST = BN * RS;  // bytes of a stage
+  const uint32_t sA = (uint32_t)__cvta_generic_to_shared(As), sB = (uint32_t)__cvta_generic_to_shared(Bs);
+  const int cr = tid >> 3, chunk = tid & 7;  // a thread copies 16-byte chunk `chunk` of rows cr, cr + NT/8, ...
+  const uint32_t cdst = (uint32_t)swz(cr, chunk * 2) * 8;
+  const uint32_t kp8 = (uint32_t)KP * 8;
 
   auto load_stage = [&](int stage, int kt) {
     const int h = kt >= ktiles_half;
     const int64_t k0 = (int64_t)(kt - h * ktiles_half) * BK;
     const double *abase = h ? job.a1 : job.a0;
     const double *bbase = h ? job.b1 : job.b0;
-    double *as = As + stage * BM * LDS;
-    double *bs = Bs + stage * BN * LDS;
-    const int chunk = tid & 7;  // 8 x 16 B per 16-double row
     if (!job.packed) {
-#pragma unroll
-      for (int rr = tid >> 3; rr < BM; rr += NT / 8) {
-        const int ro = rowoff[h * BM + rr];
-        const double *src = abase + (ro < 0 ? 0 : (int64_t)ro * KP) + k0 + chunk * 2;
-        cp_async16(as + swz(rr, chunk * 2), src, ro < 0 ? 0 : 16);
-      }
+      const uint32_t dst = sA + stage * A_ST + cdst;
+      const char *src0 = reinterpret_cast<const char *>(abase + k0 + chunk * 2);
+      const int *ro = rowoff + h * BM + cr;
+      auto rows = [&](auto self, auto ic) {
+        constexpr int I = decltype(ic)::value;
+        if constexpr (I < 8) {
+          const int r = ro[I * (NT / 8)];
+          cp_async16_at<I *(NT / 8) * RS>(dst, src0 + (uint64_t)(uint32_t)max(r, 0) * kp8, r >= 0);
+          self(self, std::integral_constant<int, I + 1>{});
+        }
+      };
+      static_assert(BM == NT, "eight passes of NT/8 rows");
+      rows(rows, std::integral_constant<int, 0>{});
     } else {
+      double *as = As + stage * BM * LDS;
       // the row's E values gathered one double at a time: the packed
       // triangle holds (k q | p x) at tri(k, q) of column p, the -T2 rows the
       // k >= nu part; past nu + no the row is zero
@@ -131,10 +164,19 @@ __device__ __forceinline__ void wbuild_tile(const GemmJob &job, int nu, int64_t 
         }
       }
     }
-#pragma unroll
-    for (int rr = tid >> 3; rr < BN; rr += NT / 8) {
-      const double *src = bbase + (int64_t)(n0 + rr) * KP + k0 + chunk * 2;
-      cp_async16(bs + swz(rr, chunk * 2), src, 16);
+    {
+      const uint32_t dst = sB + stage * B_ST + cdst;
+      const char *src = reinterpret_cast<const char *>(bbase + (int64_t)(n0 + cr) * KP + k0 + chunk * 2);
+      const int64_t step = (int64_t)(NT / 8) * kp8;
+      auto rows = [&](auto self, auto ic) {
+        constexpr int I = decltype(ic)::value;
+        if constexpr (I * (NT / 8) < BN) {
+          if (I * (NT / 8) + NT / 8 <= BN || cr < BN - I * (NT / 8))
+            cp_async16_at<I *(NT / 8) * RS>(dst, src + I * step, true);
+          self(self, std::integral_constant<int, I + 1>{});
+        }
+      };
+      rows(rows, std::integral_constant<int, 0>{});
     }
   };
 
@@ -155,34 +197,55 @@ __device__ __forceinline__ void wbuild_tile(const GemmJob &job, int nu, int64_t 
     cp_async_commit();
   }
 
+  // fragment bases of the four k4 steps: row g, column (4 s) ^ 4 (g & 3) + t
+  const uint32_t fA = sA + ((warp * WM + g) * LDS + t) * 8, fB = sB + (g * LDS + t) * 8;
+  const uint32_t gx = (uint32_t)(g & 3) * 32;
+  int stage = 0, fill = STAGES - 1;
   for (int kt = 0; kt < ktiles; kt++) {
     cp_async_wait<STAGES - 2>();
     __syncthreads();
     {
       const int nk = kt + STAGES - 1;
-      if (nk < ktiles) load_stage(nk % STAGES, nk);
+      if (nk < ktiles) load_stage(fill, nk);
       cp_async_commit();
+      if (++fill == STAGES) fill = 0;
     }
-    const double *as = As + (kt % STAGES) * BM * LDS + (warp * WM) * LDS;
-    const double *bs = Bs + (kt % STAGES) * BN * LDS;
-    // columns of this k-tile below nu + no; the k4 steps past them multiply zero padding
-    const int64_t kv = KV - (int64_t)(kt < ktiles_half ? kt : kt - ktiles_half) * BK;
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      if (kk >= kv) break;
+    auto step = [&](int s) {
+      const uint32_t pa = fA + stage * A_ST + ((uint32_t)(32 * s) ^ gx);
+      const uint32_t pb = fB + stage * B_ST + ((uint32_t)(32 * s) ^ gx);
       double af[MF][2], bf[NF];
-#pragma unroll
-      for (int i = 0; i < MF; i++) {
-        af[i][0] = as[swz(i * 16 + g, kk + t)];
-        af[i][1] = as[swz(i * 16 + g + 8, kk + t)];
-      }
-#pragma unroll
-      for (int j = 0; j < NF; j++) bf[j] = bs[swz(j * 8 + g, kk + t)];
+      auto fa = [&](auto self, auto ic) {
+        constexpr int I = decltype(ic)::value;
+        if constexpr (I < MF) {
+          af[I][0] = lds_at<I * 16 * RS>(pa);
+          af[I][1] = lds_at<(I * 16 + 8) * RS>(pa);
+          self(self, std::integral_constant<int, I + 1>{});
+        }
+      };
+      auto fb = [&](auto self, auto ic) {
+        constexpr int J = decltype(ic)::value;
+        if constexpr (J < NF) {
+          bf[J] = lds_at<J * 8 * RS>(pb);
+          self(self, std::integral_constant<int, J + 1>{});
+        }
+      };
+      fa(fa, std::integral_constant<int, 0>{});
+      fb(fb, std::integral_constant<int, 0>{});
 #pragma unroll
       for (int i = 0; i < MF; i++)
 #pragma unroll
         for (int j = 0; j < NF; j++) dmma_16x8x4(acc[i][j], af[i][0], af[i][1], bf[j]);
+    };
+    // columns of this k-tile below nu + no; the k4 steps past them multiply zero padding
+    const int kv = (int)(KV - (int64_t)(kt < ktiles_half ? kt : kt - ktiles_half) * BK);
+    if (kv > BK - 4) {
+#pragma unroll
+      for (int s = 0; s < BK / 4; s++) step(s);
+    } else {
+#pragma unroll 1
+      for (int s = 0; 4 * s < kv; s++) step(s);
     }
+    if (++stage == STAGES) stage = 0;
   }
   cp_async_wait<0>();
 
