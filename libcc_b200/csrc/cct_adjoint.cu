@@ -507,16 +507,11 @@ constexpr int BST = 3;                  // cp.async stages
 constexpr int LDA_KM = BBM + 4;         // dF A tile [k][m]
 template <int BN>
 constexpr int ldb_kn() { return BN + 4; }  // B tile [k][n]
-__device__ __forceinline__ int aswz(int r, int c) { return r * BBK + (c ^ ((r & 3) << 2)); }
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src_bytes) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 // D(16x8) += A(16x8) B(8x8).  Lane (g = lane/4, t = lane%4) holds
 // a = {A[g][t], A[g+8][t], A[g][t+4], A[g+8][t+4]}, b = {B[t][g], B[t+4][g]} and
@@ -526,6 +521,20 @@ __device__ __forceinline__ void dmma_16x8x8(double *d, const double *a, const do
       "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+// Both GEMMs address shared memory as a per-thread base plus constants (the
+// copies of a thread and the fragments of a lane are fixed distances apart);
+// indexing every copy and fragment anew held them at 0.73 and 0.76 of the
+// FP64 pipe.
+__device__ __forceinline__ uint32_t smem32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp_async16_to(uint32_t smem, const void *gmem, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(live ? 16 : 0));
+}
+// 64-bit shared load at base + OFF bytes, OFF a constant after unrolling
+__device__ __forceinline__ double lds_off(uint32_t base, int off) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v) : "r"(base + (uint32_t)off));
+  return v;
 }
 // Row m = p*nu + q of a nu^2 x . operand and its (p,q) <-> (q,p) partner, for
 // m < 2^24 (nu <= 4096): the float quotient is within one of p, then corrected.
@@ -591,28 +600,46 @@ __global__ void __launch_bounds__(BNT, BN == 64 ? 2 : 3) bwd_e_kernel(const BwdE
   }
   __syncthreads();
 
-  auto load_stage = [&](int stage, int kt) {
-    const int pi = p_begin + kt / kt_per;
-    const int64_t k0 = (int64_t)(kt % kt_per) * BBK;
-    const BwdPair &pr = args.pair[pi];
-    double *as = As + stage * BBM * BBK;
-    double *bs = Bs + stage * BBK * LDB_KN;
-    const int *rw = rows + pr.perm * BBM;
-    const int chunk = tid & 7;  // 8 x 16 B per 16-double row
-    const bool kok = k0 + chunk * 2 < NP;
-    for (int rr = tid >> 3; rr < BBM; rr += BNT / 8) {
-      const int row = rw[rr];
-      const bool ok = row >= 0 && kok;
-      const double *src = pr.A + (ok ? (int64_t)row * NP + k0 + chunk * 2 : 0);
-      cp_async16(as + aswz(rr, chunk * 2), src, ok ? 16 : 0);
+  constexpr int A_ST = BBM * BBK * 8, B_ST = BBK * LDB_KN * 8;  // bytes of a stage
+  const uint32_t sA = smem32(As), sB = smem32(Bs);
+  // A: 16-byte chunk (tid & 7) of rows tid/8 + 16 i (whose XOR is the same)
+  const int ar = tid >> 3, chunk = tid & 7;
+  const uint32_t adst = sA + (uint32_t)(ar * BBK + ((chunk * 2) ^ ((ar & 3) << 2))) * 8;
+  // B: chunks tid + 128 i of the 16 rows (s) x BN columns (n)
+  constexpr int NBC = BBK * (BBN / 2) / BNT;
+  static_assert(BBK * (BBN / 2) % BNT == 0, "whole passes over the B tile");
+  int brr[NBC], boff[NBC];
+  uint32_t bdst[NBC];
+#pragma unroll
+  for (int i = 0; i < NBC; i++) {
+    const int c = tid + i * BNT, rr = c / (BBN / 2), cc = c - rr * (BBN / 2), n = n0 + cc * 2;
+    brr[i] = n < KP ? rr : 1 << 30;  // past the last row: zero-filled
+    boff[i] = rr * (int)KP + n;
+    bdst[i] = sB + (uint32_t)(rr * LDB_KN + cc * 2) * 8;
+  }
+  const uint32_t np8 = (uint32_t)NP * 8;
+  int ld_pi = p_begin, ld_k0 = 0;  // the pair and first column of the next stage to load
+  auto load_stage = [&](int stage) {
+    const BwdPair &pr = args.pair[ld_pi];
+    const int *rw = rows + pr.perm * BBM + ar;
+    const bool kok = ld_k0 + chunk * 2 < NP;
+    const char *asrc = reinterpret_cast<const char *>(pr.A + (kok ? ld_k0 + chunk * 2 : 0));
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int row = rw[i * 16];
+      cp_async16_to(adst + stage * A_ST + i * 16 * BBK * 8, asrc + (uint64_t)(uint32_t)max(row, 0) * np8,
+                    row >= 0 && kok);
     }
-    // B tile: 16 rows (s) x BN columns (n)
-    for (int c = tid; c < BBK * (BBN / 2); c += BNT) {
-      const int rr = c / (BBN / 2), cc = c - rr * (BBN / 2);
-      const int n = n0 + cc * 2;
-      const bool ok = n < KP && k0 + rr < NP;
-      const double *src = pr.B + (ok ? (k0 + rr) * KP + n : 0);
-      cp_async16(bs + rr * LDB_KN + cc * 2, src, ok ? 16 : 0);
+    const double *bsrc = pr.B + (int64_t)ld_k0 * KP;
+#pragma unroll
+    for (int i = 0; i < NBC; i++) {
+      const bool ok = brr[i] < NP - ld_k0;
+      cp_async16_to(bdst[i] + stage * B_ST, bsrc + (ok ? boff[i] : 0), ok);
+    }
+    ld_k0 += BBK;
+    if (ld_k0 >= NP) {
+      ld_k0 = 0;
+      ld_pi++;
     }
   };
 
@@ -641,47 +668,50 @@ __global__ void __launch_bounds__(BNT, BN == 64 ? 2 : 3) bwd_e_kernel(const BwdE
 
 #pragma unroll
   for (int s = 0; s < BST - 1; s++) {
-    if (s < ktiles) load_stage(s, s);
+    if (s < ktiles) load_stage(s);
     cp_async_commit();
   }
   // NFR: n8 fragments computed; the tile's last one is skipped when all its
   // columns are padding (>= nu + no)
+  const uint32_t fA = sA + (uint32_t)((warp * BWM + g) * BBK + t) * 8, fB = sB + (uint32_t)(t * LDB_KN + g) * 8;
+  const uint32_t gx = (uint32_t)(g & 3) * 32;
   auto mainloop = [&](auto nfr_c) {
     constexpr int NFR = decltype(nfr_c)::value;
+    int stage = 0, fill = BST - 1, left = (int)NP;  // columns of the pair from this k-tile on
     for (int kt = 0; kt < ktiles; kt++) {
       cp_async_wait<BST - 2>();
       __syncthreads();
-      {
-        const int nk = kt + BST - 1;
-        if (nk < ktiles) load_stage(nk % BST, nk);
-        cp_async_commit();
-      }
-      const double *as = As + (kt % BST) * BBM * BBK;
-      const double *bs = Bs + (kt % BST) * BBK * LDB_KN;
+      if (kt + BST - 1 < ktiles) load_stage(fill);
+      cp_async_commit();
+      if (++fill == BST) fill = 0;
+      const uint32_t as = fA + stage * A_ST, bs = fB + stage * B_ST;
       // NP is a multiple of 8: the last k-tile of a pair may hold only 8 columns
-      const bool half_tile = NP - (int64_t)(kt % kt_per) * BBK <= BBK / 2;
+      const bool half_tile = left <= BBK / 2;
+      left -= BBK;
+      if (left <= 0) left = (int)NP;
 #pragma unroll
       for (int kk = 0; kk < BBK; kk += 8) {
         if (kk >= BBK / 2 && half_tile) break;
         double af[MF][4], bf[NF][2];
+        const uint32_t a0 = as + ((uint32_t)(kk * 8) ^ gx), a1 = as + ((uint32_t)((kk + 4) * 8) ^ gx);
 #pragma unroll
         for (int i = 0; i < MF; i++) {
-          const int r = warp * BWM + i * 16 + g;
-          af[i][0] = as[aswz(r, kk + t)];
-          af[i][1] = as[aswz(r + 8, kk + t)];
-          af[i][2] = as[aswz(r, kk + 4 + t)];
-          af[i][3] = as[aswz(r + 8, kk + 4 + t)];
+          af[i][0] = lds_off(a0, i * 16 * BBK * 8);
+          af[i][1] = lds_off(a0, (i * 16 + 8) * BBK * 8);
+          af[i][2] = lds_off(a1, i * 16 * BBK * 8);
+          af[i][3] = lds_off(a1, (i * 16 + 8) * BBK * 8);
         }
 #pragma unroll
         for (int j = 0; j < NFR; j++) {
-          bf[j][0] = bs[(kk + t) * LDB_KN + j * 8 + g];
-          bf[j][1] = bs[(kk + 4 + t) * LDB_KN + j * 8 + g];
+          bf[j][0] = lds_off(bs, (kk * LDB_KN + j * 8) * 8);
+          bf[j][1] = lds_off(bs, ((kk + 4) * LDB_KN + j * 8) * 8);
         }
 #pragma unroll
         for (int i = 0; i < MF; i++)
 #pragma unroll
           for (int j = 0; j < NFR; j++) dmma_16x8x8(acc[i][j], af[i], bf[j]);
       }
+      if (++stage == BST) stage = 0;
     }
   };
   if (full)
@@ -738,26 +768,43 @@ __global__ void __launch_bounds__(BNT, BN == 64 ? 2 : 3) bwd_f_kernel(const BwdF
   const int ktiles = kend > kbeg ? (int)((kend - kbeg + BBK - 1) / BBK) : 0;
   const int tid = threadIdx.x;
 
+  constexpr int A_ST = BBK * LDA_KM * 8, B_ST = BBK * LDB_KN * 8;  // bytes of a stage
+  const uint32_t sA = smem32(As), sB = smem32(Bs);
+  // A: chunk (tid & 63) of the 64 in a row, rows (m) tid/64 + 2 i
+  const int ar = tid >> 6, acol = (tid & 63) * 2;
+  const bool aok = s0 + acol < NP;
+  const uint32_t adst = sA + (uint32_t)(ar * LDA_KM + acol) * 8;
+  const double *asrc = pr.A + (aok ? (kbeg + ar) * NP + s0 + acol : 0);
+  // B: chunks tid + 128 i of the 16 rows (m) x BN columns (n)
+  constexpr int NBC = BBK * (BBN / 2) / BNT;
+  static_assert(BBK * (BBN / 2) % BNT == 0, "whole passes over the B tile");
+  int brr[NBC];
+  uint32_t bdst[NBC];
+  const double *bcol[NBC];
+#pragma unroll
+  for (int i = 0; i < NBC; i++) {
+    const int c = tid + i * BNT, rr = c / (BBN / 2), cc = c - rr * (BBN / 2), n = n0 + cc * 2;
+    brr[i] = n < KP ? rr : 1 << 30;
+    bcol[i] = pr.B + (n < KP ? n : 0);
+    bdst[i] = sB + (uint32_t)(rr * LDB_KN + cc * 2) * 8;
+  }
+  const bool perm = pr.perm != 0;
+  const int rows_left = (int)(kend - kbeg);
   auto load_stage = [&](int stage, int kt) {
-    const int64_t k0 = kbeg + (int64_t)kt * BBK;
-    double *as = As + stage * BBK * LDA_KM;
-    double *bs = Bs + stage * BBK * LDB_KN;
-    // A tile: 16 rows (m) x 128 columns (s): 64 chunks per row
-    for (int c = tid; c < BBK * (BBM / 2); c += BNT) {
-      const int rr = c / (BBM / 2), cc = c - rr * (BBM / 2);
-      const int64_t m = k0 + rr, s = s0 + cc * 2;
-      const bool ok = m < kend && s < NP;
-      const double *src = pr.A + (ok ? m * NP + s : 0);
-      cp_async16(as + rr * LDA_KM + cc * 2, src, ok ? 16 : 0);
+    const int left = rows_left - kt * BBK;  // rows of the split from this stage on
+    const double *asrc_k = asrc + (aok ? (int64_t)kt * BBK * NP : 0);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const bool ok = aok && ar + 2 * i < left;
+      cp_async16_to(adst + stage * A_ST + 2 * i * LDA_KM * 8, asrc_k + (ok ? 2 * i * NP : 0), ok);
     }
-    for (int c = tid; c < BBK * (BBN / 2); c += BNT) {
-      const int rr = c / (BBN / 2), cc = c - rr * (BBN / 2);
-      const int64_t m = k0 + rr;
-      const int n = n0 + cc * 2;
-      const bool ok = m < kend && n < KP;
-      const int64_t row = ok && pr.perm ? (int64_t)swap_row((int)m, nu, inv_nu) : m;
-      const double *src = pr.B + (ok ? row * KP + n : 0);
-      cp_async16(bs + rr * LDB_KN + cc * 2, src, ok ? 16 : 0);
+    const int m0 = (int)kbeg + kt * BBK;
+#pragma unroll
+    for (int i = 0; i < NBC; i++) {
+      const bool ok = brr[i] < left;
+      const int m = ok ? m0 + brr[i] : 0;
+      const int row = perm ? swap_row(m, nu, inv_nu) : m;
+      cp_async16_to(bdst[i] + stage * B_ST, bcol[i] + (int64_t)row * KP, ok);
     }
   };
 
@@ -777,38 +824,38 @@ __global__ void __launch_bounds__(BNT, BN == 64 ? 2 : 3) bwd_f_kernel(const BwdF
     if (s < ktiles) load_stage(s, s);
     cp_async_commit();
   }
+  const uint32_t fA = sA + (uint32_t)(t * LDA_KM + warp * BWM + g) * 8, fB = sB + (uint32_t)(t * LDB_KN + g) * 8;
   auto mainloop = [&](auto nfr_c) {  // NFR n8 fragments, as in bwd_e_kernel
     constexpr int NFR = decltype(nfr_c)::value;
+    int stage = 0, fill = BST - 1;
     for (int kt = 0; kt < ktiles; kt++) {
       cp_async_wait<BST - 2>();
       __syncthreads();
-      {
-        const int nk = kt + BST - 1;
-        if (nk < ktiles) load_stage(nk % BST, nk);
-        cp_async_commit();
-      }
-      const double *as = As + (kt % BST) * BBK * LDA_KM + warp * BWM;
-      const double *bs = Bs + (kt % BST) * BBK * LDB_KN;
+      if (kt + BST - 1 < ktiles) load_stage(fill, kt + BST - 1);
+      cp_async_commit();
+      if (++fill == BST) fill = 0;
+      const uint32_t as = fA + stage * A_ST, bs = fB + stage * B_ST;
 #pragma unroll
       for (int kk = 0; kk < BBK; kk += 8) {
         double af[MF][4], bf[NF][2];
 #pragma unroll
         for (int i = 0; i < MF; i++) {
-          af[i][0] = as[(kk + t) * LDA_KM + i * 16 + g];
-          af[i][1] = as[(kk + t) * LDA_KM + i * 16 + g + 8];
-          af[i][2] = as[(kk + 4 + t) * LDA_KM + i * 16 + g];
-          af[i][3] = as[(kk + 4 + t) * LDA_KM + i * 16 + g + 8];
+          af[i][0] = lds_off(as, (kk * LDA_KM + i * 16) * 8);
+          af[i][1] = lds_off(as, (kk * LDA_KM + i * 16 + 8) * 8);
+          af[i][2] = lds_off(as, ((kk + 4) * LDA_KM + i * 16) * 8);
+          af[i][3] = lds_off(as, ((kk + 4) * LDA_KM + i * 16 + 8) * 8);
         }
 #pragma unroll
         for (int j = 0; j < NFR; j++) {
-          bf[j][0] = bs[(kk + t) * LDB_KN + j * 8 + g];
-          bf[j][1] = bs[(kk + 4 + t) * LDB_KN + j * 8 + g];
+          bf[j][0] = lds_off(bs, (kk * LDB_KN + j * 8) * 8);
+          bf[j][1] = lds_off(bs, ((kk + 4) * LDB_KN + j * 8) * 8);
         }
 #pragma unroll
         for (int i = 0; i < MF; i++)
 #pragma unroll
           for (int j = 0; j < NFR; j++) dmma_16x8x8(acc[i][j], af[i], bf[j]);
       }
+      if (++stage == BST) stage = 0;
     }
   };
   if (full)

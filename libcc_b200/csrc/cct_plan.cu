@@ -109,7 +109,7 @@ struct ccT_plan {
   cudaEvent_t ev_bwdf[2] = {};
   // backward, per GX set: pointwise pass done / dE GEMM done / dF GEMM done reading it
   cudaEvent_t ev_gx_pw[kGXSets] = {}, ev_gx_e[kGXSets] = {}, ev_gx_f[kGXSets] = {};
-  std::vector<cudaEvent_t> ev_rec, ev_pw;  // per tuple of the X ring: W rebuilt / read by the pointwise pass
+  cudaEvent_t ev_rec[kNBuf] = {}, ev_pw[kNBuf] = {};  // per X ring group: W rebuilt / read by the pointwise pass
   int64_t fwd_begin = -1, fwd_end = -1;
   float last_bwd_ms = 0.f;
   // options.keep_w: the W-build output of the last forward, kept for the
@@ -203,7 +203,6 @@ int upload_emu_jobs(ccT_plan *p, const std::vector<GemmJob> &jobs, EmuJob *dst) 
   return CCT_OK;
 }
 
-int num_jobs(const Tuple &t) { return t.kind == kIJK ? 3 : 2; }
 // Position of tuple t's first job in the plan's job lists.
 int64_t job_offset(const ccT_plan *p, int64_t t) {
   const int64_t no = p->d.no, nijk = no * (no - 1) * (no - 2) / 6;
@@ -1109,17 +1108,15 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
     for (int g = 0; g < kGXSets; g++)
       for (cudaEvent_t *e : {&p->ev_gx_pw[g], &p->ev_gx_e[g], &p->ev_gx_f[g]})
         CCT_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-    for (std::vector<cudaEvent_t> *v : {&p->ev_rec, &p->ev_pw}) {
-      v->assign((size_t)p->group * p->nring, nullptr);
-      for (cudaEvent_t &e : *v) CCT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
+    for (int b = 0; b < kNBuf; b++)
+      for (cudaEvent_t *e : {&p->ev_rec[b], &p->ev_pw[b]})
+        CCT_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   }
-  const int64_t ring = (int64_t)p->group * p->nring;  // X buffers in flight, one tuple each
   CCT_CUDA(cudaEventRecord(p->ev0, p->stream));
   CCT_TRY(adj_zero(d, &p->adj, p->stream));
   // dT1 = 2 v1: an emulated plan's v1 is rebuilt from the FP64 W of this pass
   if (p->emulated) CCT_CUDA(cudaMemsetAsync(p->adj.v1, 0, (5 + (size_t)d.nu * d.no) * 8, p->stream));
-  // Four streams.  rec_stream rebuilds W of tuple t into its X ring buffer,
+  // Four streams.  rec_stream rebuilds W one X ring group of tuples per launch,
   // ahead of red_stream, which runs the pointwise adjoint kernels of tuple t
   // (dE/dW, dVOE, deps and dE/dX into GX set t mod 4); bwd_stream then runs
   // the dF GEMM of tuple t, and gemm_stream one dE GEMM for each pair of
@@ -1139,15 +1136,19 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
   for (int64_t t = begin; t < end; t++) {
     const Tuple &tu = p->tuples[t];
     const int set = (int)((t - begin) % kGXSets);
-    const int xb = (int)(t % ring);
+    const int64_t grp = t / p->group, grp_end = std::min(end, (grp + 1) * p->group);
+    const int xb = (int)(grp % p->nring);
     double *Xk[3] = {nullptr, nullptr, nullptr};
     if (kept) {
       for (int g = 0; g < 3; g++) Xk[g] = xkeep_at(p, t - begin, g);
     } else {
-      if (t - begin >= ring) CCT_CUDA(cudaStreamWaitEvent(sW, p->ev_pw[xb], 0));  // X buffer read by t - ring
-      CCT_TRY(launch_wbuild_f64(d, p->jobs + job_offset(p, t), num_jobs(tu), sW));
-      CCT_CUDA(cudaEventRecord(p->ev_rec[xb], sW));
-      CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_rec[xb], 0));
+      if (t == begin || t % p->group == 0) {  // the group's first tuple
+        // X buffers last read by the pointwise passes of nring groups before
+        if (grp - begin / p->group >= p->nring) CCT_CUDA(cudaStreamWaitEvent(sW, p->ev_pw[xb], 0));
+        CCT_TRY(wbuild_tuples(p, t, grp_end, true, sW, false));
+        CCT_CUDA(cudaEventRecord(p->ev_rec[xb], sW));
+        CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_rec[xb], 0));
+      }
       for (int g = 0; g < 3; g++) Xk[g] = xbuf(p, t, g);
     }
     if (t - begin >= kGXSets) {  // GX set last read by the GEMMs of tuple t - kGXSets
@@ -1162,7 +1163,7 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
       CCT_TRY(launch_reduce(d, g, false, p->eh, p->ep, p->vb, p->cta_table, p->xpart, p->vpart, p->flags + 1, sP));
       CCT_TRY(launch_finalize(d, g, p->xpart, p->vpart, p->tsum, p->adj.v1, p->adj.v1 + 5, sP));
     }
-    CCT_CUDA(cudaEventRecord(p->ev_pw[xb], sP));
+    if (t + 1 == grp_end) CCT_CUDA(cudaEventRecord(p->ev_pw[xb], sP));
     CCT_CUDA(cudaEventRecord(p->ev_gx_pw[set], sP));
     CCT_CUDA(cudaStreamWaitEvent(sF, p->ev_gx_pw[set], 0));
     CCT_TRY(adj_tuple_gemm_f(d, tu, p->E, &p->adj, set, sF));
@@ -1400,8 +1401,8 @@ int ccT_plan_destroy(ccT_plan *p) {
   if (p->pw_stream) cudaStreamDestroy(p->pw_stream);
   for (cudaEvent_t e : p->ev_bwdf)
     if (e) cudaEventDestroy(e);
-  for (std::vector<cudaEvent_t> *v : {&p->ev_rec, &p->ev_pw})
-    for (cudaEvent_t e : *v)
+  for (int b = 0; b < kNBuf; b++)
+    for (cudaEvent_t e : {p->ev_rec[b], p->ev_pw[b]})
       if (e) cudaEventDestroy(e);
   for (int g = 0; g < kGXSets; g++)
     for (cudaEvent_t e : {p->ev_gx_pw[g], p->ev_gx_e[g], p->ev_gx_f[g]})
