@@ -30,9 +30,10 @@
 //
 // A second executor (mode 1) runs the same items as grouped launches: per
 // tuple group, one launch of 128-row W-build tiles (three CTAs per SM) on one
-// stream, then one launch of its reduction blocks (two CTAs per SM, the last
-// block of a tuple finalizing it) on a second stream, the ring slots guarded
-// by stream events instead of counters.  Either forward (counter reset plus the
+// stream, then one launch of its reduction blocks (two CTAs per SM walking over
+// them) and one of its tuples' sums on a second stream, the ring slots
+// guarded by stream events instead of counters; the systems are summed at the
+// end.  Either forward (counter reset plus the
 // launches) is captured once in a CUDA graph and replayed.  The executor, the
 // W-build N tile (BN) and the tuple order are chosen by ccT_batch_tune, which
 // times every candidate on the loaded batch.
@@ -51,6 +52,7 @@
 #include <cstring>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cct_internal.cuh"
@@ -84,13 +86,28 @@ struct TupleRec {
   double *xpart, *vpart;
 };
 
+// What a reduction block of the grouped executors reads of its tuple and system:
+// one 128-byte record.
+struct alignas(16) RdTuple {
+  TupleDev t;
+  const double *eh, *ep, *vb;
+  double *xpart, *vpart;
+  int64_t NP;
+  int nu, no;
+  int64_t pad[3];
+};
+static_assert(sizeof(RdTuple) == 128, "eight 16-byte copies");
+
 struct BatchArgs {
-  const int4 *items;  // {kind 0 = W-build tile / 1 = reduction block, tuple, job slot | block, tile}
+  // {kind 0 = W-build tile / 1 = reduction block, tuple, job slot | block, tile | the blocks A + 1024 B + 1024^2 C}
+  const int4 *items;
   int64_t nitems;
   int *counters;      // [0] queue head, then wb_done[T], rd_done[T], group_rd[G], sys_done[S]
   int ntuple, ngroup;
   const int *group_rd_items;  // reduction blocks per group
   const TupleRec *tuples;
+  const RdTuple *rd;    // [tuple]
+  const int *group_tuples;  // tuples in group order
   const GemmJob *jobs;  // [tuple][3]
   const SysDev *sys;
   double *tuple_etd, *tuple_v1;  // per tuple: weight x3, and 3 nu v1 contributions
@@ -116,10 +133,13 @@ __device__ void spin_until(const int *p, int target, int *err, long limit) {
   atomicExch(err, 1);
 }
 
-// Sums of one tuple's reduction partials, in the order of tuple_sum_kernel.
-__device__ void finalize_tuple(const TupleRec &T, const SysDev &S, int t, const BatchArgs &A, double *red) {
+// Sums of one tuple's reduction partials, in the order of tuple_sum_kernel:
+// part `part` of nparts (part 0 the E[4] sum, every part its virtual indices).
+__device__ void finalize_tuple(const TupleRec &T, const SysDev &S, int t, const BatchArgs &A, double *red, int part,
+                               int nparts) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double weight = T.kind == kIJK ? 1.0 : 0.5;
+  if (part == 0) {
   double s = 0.0;
   for (int64_t c = tid; c < S.ncta; c += kBT) s += __ldcg(T.xpart + c);
   red[tid] = s;
@@ -129,9 +149,10 @@ __device__ void finalize_tuple(const TupleRec &T, const SysDev &S, int t, const 
     __syncthreads();
   }
   if (tid == 0) A.tuple_etd[t] = weight * red[0];
+  }
   const int64_t npairs = (int64_t)S.nb * (S.nb + 1) / 2;
   double *tv = A.tuple_v1 + A.tuple_v1_off[t];
-  for (int a = warp; a < S.nu; a += kBT / 32) {
+  for (int a = warp + kBT / 32 * part; a < S.nu; a += kBT / 32 * nparts) {
     const int X = a / red::RB, la = a - X * red::RB;
     const double *slab = T.vpart + ((int64_t)X * red::RB + la) * 3 * npairs;
 #pragma unroll
@@ -145,24 +166,12 @@ __device__ void finalize_tuple(const TupleRec &T, const SysDev &S, int t, const 
   }
 }
 
-// One system's etd (Neumaier over its tuples in order), v1 and ets -- the
-// arithmetic of tuple_sum_kernel, group_add_kernel and ets_kernel, in the same order.
-__device__ void system_sum(const SysDev &S, int s, const BatchArgs &A, double *red) {
-  const int tid = threadIdx.x;
+// v1 elements (a, x) of a system from e0 on, every `step`-th: the contributions
+// of the system's tuples in order, each tuple's columns i, j, k in that order
+// (as group_add_kernel adds them).
+__device__ void system_v1(const SysDev &S, const BatchArgs &A, int64_t e0, int64_t step) {
   const int nu = S.nu, no = S.no;
-  if (tid == 0) {
-    double sum = 0.0, comp = 0.0;
-    for (int64_t t = S.tuple_begin; t < S.tuple_begin + S.ntuples; t++) {
-      const double v = __ldcg(A.tuple_etd + t);
-      const double nsum = sum + v;
-      comp += fabs(sum) >= fabs(v) ? (sum - nsum) + v : (v - nsum) + sum;
-      sum = nsum;
-    }
-    red[kBT] = sum + comp;
-  }
-  // thread per v1 element (a, x): the contributions of the system's tuples in
-  // order, each tuple's columns i, j, k in that order (as group_add_kernel adds them)
-  for (int64_t e = tid; e < (int64_t)nu * no; e += kBT) {
+  for (int64_t e = e0; e < (int64_t)nu * no; e += step) {
     const int x = (int)(e / nu), a = (int)(e - (int64_t)x * nu);
     double v = 0.0;
     for (int64_t t = S.tuple_begin; t < S.tuple_begin + S.ntuples; t++) {
@@ -174,7 +183,25 @@ __device__ void system_sum(const SysDev &S, int s, const BatchArgs &A, double *r
     }
     S.v1[e] = v;
   }
-  __syncthreads();
+}
+
+// One system's etd (Neumaier over its tuples in order) and, from its v1, ets --
+// the arithmetic of tuple_sum_kernel, group_add_kernel and ets_kernel, in the
+// same order.
+__device__ void system_energy(const SysDev &S, int s, const BatchArgs &A, double *red) {
+  const int tid = threadIdx.x;
+  const int nu = S.nu, no = S.no;
+  if (tid == 0) {
+    double sum = 0.0, comp = 0.0;
+#pragma unroll 8
+    for (int64_t t = S.tuple_begin; t < S.tuple_begin + S.ntuples; t++) {
+      const double v = __ldcg(A.tuple_etd + t);
+      const double nsum = sum + v;
+      comp += fabs(sum) >= fabs(v) ? (sum - nsum) + v : (v - nsum) + sum;
+      sum = nsum;
+    }
+    red[kBT] = sum + comp;
+  }
   double sacc = 0.0;
   const int64_t n = (int64_t)no * nu;
   for (int64_t e = tid; e < n; e += kBT) {
@@ -244,16 +271,18 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
       td.weight = T.kind == kIJK ? 1.0 : 0.5;
       const int c = it.z;
       const int S0 = S.cta_table[3 * c], S1 = S.cta_table[3 * c + 1], S2 = S.cta_table[3 * c + 2];
-      double *dsm = reinterpret_cast<double *>(smem);
+      const red::Smem m(reinterpret_cast<double *>(smem));
+      auto block = [&](auto kind) {
+        constexpr int KIND = decltype(kind)::value;
+        red::fill_rows<KIND, red::kRowsCoherent>(S.nu, S.no, S.NP, td, S.vb, S0, S1, S2, m.Xs, m.Vs);
+        red::reduce_compute<KIND>(S.nu, td, S.eh, S.ep, S0, S1, S2, T.xpart + c, T.vpart, m, [] {});
+      };
       if (T.kind == kIJK)
-        red::reduce_block<kIJK, red::kRowsCoherent>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c,
-                                                      T.vpart, dsm, A.err);
+        block(std::integral_constant<int, kIJK>{});
       else if (T.kind == kIJJ)
-        red::reduce_block<kIJJ, red::kRowsCoherent>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c,
-                                                      T.vpart, dsm, A.err);
+        block(std::integral_constant<int, kIJJ>{});
       else
-        red::reduce_block<kIIJ, red::kRowsCoherent>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c,
-                                                      T.vpart, dsm, A.err);
+        block(std::integral_constant<int, kIIJ>{});
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -263,14 +292,16 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
       __syncthreads();
       if (s_flag) {  // last block of the tuple: finalize it
         __threadfence();
-        finalize_tuple(T, S, t, A, red);
+        finalize_tuple(T, S, t, A, red, 0, 1);
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) s_flag = atomicAdd(sys_done + T.sys, 1) == S.ntuples - 1;
         __syncthreads();
         if (s_flag) {  // last tuple of the system: sum the system
           __threadfence();
-          system_sum(S, T.sys, A, red);
+          system_v1(S, A, threadIdx.x, kBT);
+          __syncthreads();
+          system_energy(S, T.sys, A, red);
           __threadfence();
         }
       }
@@ -291,50 +322,77 @@ __global__ void __launch_bounds__(wb::NT, 3) batch_wb_kernel(const BatchArgs A, 
   wb::wbuild_tile<BN, wb::BM>(A.jobs[(int64_t)it.y * 3 + it.z], S.nu, S.KP, S.nu + S.no, S.NP, tile_m, tile_n, true, smem);
 }
 
-__global__ void __launch_bounds__(kBT, 2) batch_rd_kernel(const BatchArgs A, int64_t item0) {
+// Reduction blocks item0 .. item0 + count - 1, the blockIdx.x-th and every
+// gridDim.x-th after it.  The item after next and the next item's record are
+// read, and the next item's copies started, while a block is evaluated: with
+// one CTA per block, four dependent reads before its copies and a counter after
+// it, the launches took 67 ms of 24 systems' 128 (emulated), 27 ms now.
+__global__ void __launch_bounds__(kBT, 2) batch_rd_kernel(const BatchArgs A, int64_t item0, int count) {
   extern __shared__ __align__(16) double dsm[];
-  __shared__ double red[kBT + 1];
-  __shared__ int s_flag;
-  int *const rd_done = A.counters + 1 + A.ntuple;
-  int *const sys_done = rd_done + A.ntuple + A.ngroup;
-  const int4 it = A.items[item0 + blockIdx.x];
-  const int t = it.y;
+  __shared__ RdTuple desc[2];
+  const red::Smem m(dsm);
+  int i = blockIdx.x;
+  if (i >= count) return;
+  auto load_desc = [&](int b, int tuple) {
+    if (threadIdx.x < 8)
+      wb::cp_async16(reinterpret_cast<char *>(&desc[b]) + 16 * threadIdx.x,
+                     reinterpret_cast<const char *>(A.rd + tuple) + 16 * threadIdx.x, 16);
+    wb::cp_async_commit();
+  };
+  int4 it = A.items[item0 + i], it1 = it;
+  if (i + (int)gridDim.x < count) it1 = A.items[item0 + i + gridDim.x];
+  load_desc(0, it.y);
+  wb::cp_async_wait<0>();
+  red::init_copies(m);  // (a block barrier: the record is visible)
+  red::start_copies(desc[0].nu, desc[0].no, desc[0].NP, desc[0].t, desc[0].vb, it.w & 1023, (it.w >> 10) & 1023,
+                    it.w >> 20, m);
+  for (uint32_t round = 0;; round ^= 1) {
+    const bool more = i + (int)gridDim.x < count;
+    int4 it2 = it1;
+    if (more) load_desc(round ^ 1, it1.y);
+    if (i + 2 * (int)gridDim.x < count) it2 = A.items[item0 + i + 2 * gridDim.x];
+    if (!red::copies_landed(m, round, A.err)) return;
+    const RdTuple &T = desc[round];
+    auto next = [&]() {
+      if (!more) return;
+      wb::cp_async_wait<0>();
+      __syncthreads();
+      const RdTuple &N = desc[round ^ 1];
+      red::start_copies(N.nu, N.no, N.NP, N.t, N.vb, it1.w & 1023, (it1.w >> 10) & 1023, it1.w >> 20, m);
+    };
+    auto block = [&](auto kind) {
+      constexpr int KIND = decltype(kind)::value;
+      red::reduce_compute<KIND>(T.nu, T.t, T.eh, T.ep, it.w & 1023, (it.w >> 10) & 1023, it.w >> 20, T.xpart + it.z,
+                                T.vpart, m, next);
+    };
+    if (T.t.kind == kIJK)
+      block(std::integral_constant<int, kIJK>{});
+    else if (T.t.kind == kIJJ)
+      block(std::integral_constant<int, kIJJ>{});
+    else
+      block(std::integral_constant<int, kIIJ>{});
+    if (!more) break;
+    i += gridDim.x;
+    it = it1;
+    it1 = it2;
+  }
+}
+
+// Sums of the tuples of a group (grid: tuple of the group, part).
+constexpr int kSumParts = 8;
+__global__ void __launch_bounds__(kBT) batch_sum_kernel(const BatchArgs A, int first) {
+  __shared__ double red[kBT];
+  const int t = A.group_tuples[first + blockIdx.x];
   const TupleRec &T = A.tuples[t];
-  const SysDev &S = A.sys[T.sys];
-  TupleDev td;
-  td.x[0] = T.x[0];
-  td.x[1] = T.x[1];
-  td.x[2] = T.x[2];
-  td.kind = T.kind;
-  td.i = T.i;
-  td.j = T.j;
-  td.k = T.k;
-  td.weight = T.kind == kIJK ? 1.0 : 0.5;
-  const int c = it.z;
-  const int S0 = S.cta_table[3 * c], S1 = S.cta_table[3 * c + 1], S2 = S.cta_table[3 * c + 2];
-  if (T.kind == kIJK)
-    red::reduce_block<kIJK, red::kBulk>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c, T.vpart, dsm,
-                                          A.err);
-  else if (T.kind == kIJJ)
-    red::reduce_block<kIJJ, red::kBulk>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c, T.vpart, dsm,
-                                          A.err);
-  else
-    red::reduce_block<kIIJ, red::kBulk>(S.nu, S.no, S.NP, td, S.eh, S.ep, S.vb, S0, S1, S2, T.xpart + c, T.vpart, dsm,
-                                          A.err);
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_flag = atomicAdd(rd_done + t, 1) == T.rd_items - 1;
-  __syncthreads();
-  if (!s_flag) return;
-  __threadfence();
-  finalize_tuple(T, S, t, A, red);
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_flag = atomicAdd(sys_done + T.sys, 1) == S.ntuples - 1;
-  __syncthreads();
-  if (!s_flag) return;
-  __threadfence();
-  system_sum(S, T.sys, A, red);
+  finalize_tuple(T, A.sys[T.sys], t, A, red, blockIdx.y, kSumParts);
+}
+// v1, then the energies, of every system.
+__global__ void __launch_bounds__(kBT) batch_v1_kernel(const BatchArgs A) {
+  system_v1(A.sys[blockIdx.x], A, blockIdx.y * kBT + threadIdx.x, (int64_t)gridDim.y * kBT);
+}
+__global__ void __launch_bounds__(kBT) batch_energy_kernel(const BatchArgs A) {
+  __shared__ double red[kBT + 1];
+  system_energy(A.sys[blockIdx.x], blockIdx.x, A, red);
 }
 
 template <typename T>
@@ -355,6 +413,7 @@ struct BatchSystemHost {
   double *eh = nullptr, *ep = nullptr, *t1 = nullptr, *t2 = nullptr, *vm = nullptr, *voe = nullptr,
          *vvvo = nullptr, *E = nullptr, *F = nullptr, *v1 = nullptr, *vb = nullptr;
   int16_t *cta_table = nullptr;
+  void *arena = nullptr;  // all of the above but F
   int64_t f_np = 0;  // the N padding F was built for
   bool ready = false;
 };
@@ -398,11 +457,15 @@ struct ccT_batch {
   int64_t ncounters = 0;
   int *group_rd_items = nullptr;
   TupleRec *tuples = nullptr;
+  RdTuple *rd = nullptr;
+  int *group_tuples = nullptr;
+  std::vector<int> grp_first;             // per group: its first position in group_tuples (and the end)
   GemmJob *jobs = nullptr;
   SysDev *sysdev = nullptr;
   double *tuple_etd = nullptr, *tuple_v1 = nullptr, *sys_out = nullptr, *scratch = nullptr;
   int64_t *tuple_v1_off = nullptr;
   int *err = nullptr;
+  void *sched = nullptr;  // one allocation: items .. err above, but scratch
   cudaGraphExec_t graph = nullptr;
   float last_ms = 0.f;
 };
@@ -412,15 +475,16 @@ namespace {
 void free_schedule(ccT_batch *b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   b->graph = nullptr;
-  for (void *q : {(void *)b->items, (void *)b->counters, (void *)b->group_rd_items, (void *)b->tuples,
-                  (void *)b->jobs, (void *)b->sysdev, (void *)b->tuple_etd, (void *)b->tuple_v1, (void *)b->sys_out,
-                  (void *)b->scratch, (void *)b->tuple_v1_off, (void *)b->err, (void *)b->emu_jobs})
-    if (q) cudaFree(q);
+  if (b->sched) cudaFree(b->sched);
+  if (b->scratch) cudaFree(b->scratch);
+  b->sched = nullptr;
   b->emu_jobs = nullptr;
   b->items = nullptr;
   b->counters = nullptr;
   b->group_rd_items = nullptr;
   b->tuples = nullptr;
+  b->rd = nullptr;
+  b->group_tuples = nullptr;
   b->jobs = nullptr;
   b->sysdev = nullptr;
   b->tuple_etd = b->tuple_v1 = b->sys_out = b->scratch = nullptr;
@@ -667,7 +731,9 @@ int build_schedule(ccT_batch *b) {
   auto push_rd = [&](int g) {
     b->grp_rd_begin[g] = (int64_t)items.size();
     for (int u : groups[g])
-      for (int c = 0; c < th[u].rd_items; c++) items.push_back(make_int4(1, u, c, 0));
+      for (int c = 0, C = 0; c < th[u].rd_items; C++)  // the order of the reduction table
+        for (int B = 0; B <= C; B++)
+          for (int a = 0; a <= B; a++, c++) items.push_back(make_int4(1, u, c, a | B << 10 | C << 20));
     b->grp_rd_count[g] = (int64_t)items.size() - b->grp_rd_begin[g];
   };
   if (b->mode == 0) {
@@ -706,6 +772,33 @@ int build_schedule(ccT_batch *b) {
     v.v1 = S.v1;
     sd[s] = v;
   }
+  std::vector<RdTuple> rd(T);
+  for (int u = 0; u < T; u++) {
+    const BatchSystemHost &S = b->sys[th[u].sys];
+    RdTuple r{};
+    for (int g = 0; g < 3; g++) r.t.x[g] = rec[u].x[g];
+    r.t.kind = th[u].kind;
+    r.t.i = th[u].i;
+    r.t.j = th[u].j;
+    r.t.k = th[u].k;
+    r.t.weight = th[u].kind == kIJK ? 1.0 : 0.5;
+    r.eh = S.eh;
+    r.ep = S.ep;
+    r.vb = S.vb;
+    r.xpart = rec[u].xpart;
+    r.vpart = rec[u].vpart;
+    r.NP = S.d.NP;
+    r.nu = S.nu;
+    r.no = S.no;
+    rd[u] = r;
+  }
+  std::vector<int> gtuples;
+  b->grp_first.clear();
+  for (int g = 0; g < G; g++) {
+    b->grp_first.push_back((int)gtuples.size());
+    gtuples.insert(gtuples.end(), groups[g].begin(), groups[g].end());
+  }
+  b->grp_first.push_back((int)gtuples.size());
   std::vector<int> gnt(G, 0);
   for (int g = 0; g < G; g++)
     for (int u : groups[g]) gnt[g] += th[u].rd_items;
@@ -713,17 +806,26 @@ int build_schedule(ccT_batch *b) {
   b->ngroup = G;
   b->nitems = (int64_t)items.size();
   b->ncounters = 1 + 2 * (int64_t)T + G + nsys;
-  CCT_TRY(dmalloc(&b->items, items.size()));
-  CCT_TRY(dmalloc(&b->counters, (size_t)b->ncounters));
-  CCT_TRY(dmalloc(&b->group_rd_items, (size_t)G));
-  CCT_TRY(dmalloc(&b->tuples, (size_t)T));
-  CCT_TRY(dmalloc(&b->jobs, (size_t)T * 3));
-  CCT_TRY(dmalloc(&b->sysdev, (size_t)nsys));
-  CCT_TRY(dmalloc(&b->tuple_etd, (size_t)T));
-  CCT_TRY(dmalloc(&b->tuple_v1, (size_t)v1tot));
-  CCT_TRY(dmalloc(&b->tuple_v1_off, (size_t)T));
-  CCT_TRY(dmalloc(&b->sys_out, (size_t)3 * nsys));
-  CCT_TRY(dmalloc(&b->err, 1));
+  {
+    Arena mem;
+    mem.add(&b->items, (int64_t)items.size());
+    mem.add(&b->counters, b->ncounters);
+    mem.add(&b->group_rd_items, G);
+    mem.add(&b->tuples, T);
+    mem.add(&b->rd, T);
+    mem.add(&b->group_tuples, T);
+    mem.add(&b->jobs, (int64_t)T * 3);
+    mem.add(&b->sysdev, nsys);
+    mem.add(&b->tuple_etd, T);
+    mem.add(&b->tuple_v1, v1tot);
+    mem.add(&b->tuple_v1_off, T);
+    mem.add(&b->sys_out, 3 * (int64_t)nsys);
+    mem.add(&b->err, 1);
+    if (!ejobs.empty()) mem.add(&b->emu_jobs, (int64_t)ejobs.size());
+    CCT_TRY(mem.allocate(&b->sched));
+  }
+  CCT_CUDA(cudaMemcpy(b->rd, rd.data(), T * sizeof(RdTuple), cudaMemcpyHostToDevice));
+  CCT_CUDA(cudaMemcpy(b->group_tuples, gtuples.data(), T * sizeof(int), cudaMemcpyHostToDevice));
   CCT_CUDA(cudaMemcpy(b->items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
   CCT_CUDA(cudaMemcpy(b->group_rd_items, gnt.data(), G * sizeof(int), cudaMemcpyHostToDevice));
   CCT_CUDA(cudaMemcpy(b->tuples, rec.data(), T * sizeof(TupleRec), cudaMemcpyHostToDevice));
@@ -731,7 +833,6 @@ int build_schedule(ccT_batch *b) {
   CCT_CUDA(cudaMemcpy(b->sysdev, sd.data(), nsys * sizeof(SysDev), cudaMemcpyHostToDevice));
   CCT_CUDA(cudaMemcpy(b->tuple_v1_off, v1off.data(), T * sizeof(int64_t), cudaMemcpyHostToDevice));
   if (!ejobs.empty()) {
-    CCT_TRY(dmalloc(&b->emu_jobs, ejobs.size()));
     CCT_CUDA(cudaMemcpy(b->emu_jobs, ejobs.data(), ejobs.size() * sizeof(EmuJob), cudaMemcpyHostToDevice));
   }
   CCT_CUDA(cudaStreamSynchronize(b->stream));
@@ -748,6 +849,8 @@ BatchArgs batch_args(ccT_batch *b) {
   a.ngroup = b->ngroup;
   a.group_rd_items = b->group_rd_items;
   a.tuples = b->tuples;
+  a.rd = b->rd;
+  a.group_tuples = b->group_tuples;
   a.jobs = b->jobs;
   a.sys = b->sysdev;
   a.tuple_etd = b->tuple_etd;
@@ -785,6 +888,8 @@ int launch_wb_range(const BatchArgs &a, int64_t begin, int64_t count, cudaStream
 
 int launch_grouped(ccT_batch *b) {
   const BatchArgs a = batch_args(b);
+  int nsm = 0;
+  CCT_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device));
   CCT_CUDA(cudaMemsetAsync(b->counters, 0, (size_t)b->ncounters * sizeof(int), b->stream));
   CCT_CUDA(cudaMemsetAsync(b->err, 0, sizeof(int), b->stream));
   CCT_CUDA(cudaEventRecord(b->ev_fork, b->stream));
@@ -811,11 +916,21 @@ int launch_grouped(ccT_batch *b) {
     CCT_CUDA(cudaEventRecord(b->ev_wb[slot], b->stream));
     CCT_CUDA(cudaStreamWaitEvent(b->stream2, b->ev_wb[slot], 0));
     if (b->grp_rd_count[g] > 0) {
-      batch_rd_kernel<<<(unsigned)b->grp_rd_count[g], kBT, red::REDUCE_SMEM, b->stream2>>>(a, b->grp_rd_begin[g]);
+      const int64_t blocks = std::min<int64_t>(b->grp_rd_count[g], 2 * nsm);
+      batch_rd_kernel<<<(unsigned)blocks, kBT, red::REDUCE_SMEM, b->stream2>>>(a, b->grp_rd_begin[g],
+                                                                             (int)b->grp_rd_count[g]);
       CCT_CUDA(cudaGetLastError());
     }
     CCT_CUDA(cudaEventRecord(b->ev_ring[slot], b->stream2));
+    const int ntup = b->grp_first[g + 1] - b->grp_first[g];
+    batch_sum_kernel<<<dim3((unsigned)ntup, kSumParts), kBT, 0, b->stream2>>>(a, b->grp_first[g]);
+    CCT_CUDA(cudaGetLastError());
   }
+  const unsigned nsys = (unsigned)b->sys.size();
+  batch_v1_kernel<<<dim3(nsys, 8), kBT, 0, b->stream2>>>(a);
+  CCT_CUDA(cudaGetLastError());
+  batch_energy_kernel<<<nsys, kBT, 0, b->stream2>>>(a);
+  CCT_CUDA(cudaGetLastError());
   CCT_CUDA(cudaEventRecord(b->ev_join, b->stream2));
   CCT_CUDA(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
   return CCT_OK;
@@ -884,8 +999,8 @@ int configure_all(ccT_batch *b) {
   CCT_CUDA(cudaFuncSetAttribute(batch_wb_kernel<40>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 wb::smem_bytes<40, wb::BM>()));
   CCT_CUDA(cudaFuncSetAttribute(batch_rd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, red::REDUCE_SMEM));
-  CCT_CUDA(cudaFuncSetAttribute(batch_rd_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                cudaSharedmemCarveoutMaxShared));
+  for (const void *k : {(const void *)batch_rd_kernel, (const void *)batch_sum_kernel})  // the W builds' carveout
+    CCT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   (void)b;
   return CCT_OK;
 }
@@ -964,12 +1079,19 @@ int ccT_batch_create(ccT_batch **out, int64_t nsys, const int64_t *no, const int
     S.nu = (int)nu[s];
     S.d = batch_dims(S.no, S.nu, b->bn ? b->bn : choose_bn(S.nu));
     const int64_t n = S.no, v = S.nu, v2 = v * v;
-    if ((st = dmalloc(&S.eh, n)) || (st = dmalloc(&S.ep, v)) || (st = dmalloc(&S.t1, n * v)) ||
-        (st = dmalloc(&S.t2, v2 * n * n)) || (st = dmalloc(&S.vm, n * v * n * n)) ||
-        (st = dmalloc(&S.voe, v2 * n * n)) || (st = dmalloc(&S.vb, vb_size(S.d))) || (st = dmalloc(&S.vvvo, v * (v + 1) / 2 * v * n)) ||
-        (st = dmalloc(&S.E, n * v2 * S.d.KP)) || (st = dmalloc(&S.v1, v * n)) ||
-        (st = dmalloc(&S.cta_table, S.d.ncta * 3)))
-      return fail(st);
+    Arena mem;
+    mem.add(&S.eh, n);
+    mem.add(&S.ep, v);
+    mem.add(&S.t1, n * v);
+    mem.add(&S.t2, v2 * n * n);
+    mem.add(&S.vm, n * v * n * n);
+    mem.add(&S.voe, v2 * n * n);
+    mem.add(&S.vb, vb_size(S.d));
+    mem.add(&S.vvvo, v * (v + 1) / 2 * v * n);
+    mem.add(&S.E, n * v2 * S.d.KP);
+    mem.add(&S.v1, v * n);
+    mem.add(&S.cta_table, S.d.ncta * 3);
+    if ((st = mem.allocate(&S.arena))) return fail(st);
     std::vector<int16_t> table(S.d.ncta * 3);
     int64_t idx = 0;
     for (int C = 0; C < S.d.nb; C++)
@@ -1189,8 +1311,7 @@ int ccT_batch_destroy(ccT_batch *b) {
   for (ccT_plan *p : b->emu_plans)
     if (p) ccT_plan_destroy(p);
   for (BatchSystemHost &S : b->sys)
-    for (void *q : {(void *)S.eh, (void *)S.ep, (void *)S.t1, (void *)S.t2, (void *)S.vm, (void *)S.voe,
-                    (void *)S.vvvo, (void *)S.E, (void *)S.F, (void *)S.v1, (void *)S.cta_table, (void *)S.vb})
+    for (void *q : {S.arena, (void *)S.F})
       if (q) cudaFree(q);
   for (cudaEvent_t e : {b->ev0, b->ev1, b->ev_fork, b->ev_join})
     if (e) cudaEventDestroy(e);

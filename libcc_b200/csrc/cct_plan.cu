@@ -143,24 +143,6 @@ int dalloc(T **p, size_t count) {
 
 double *v1_acc(ccT_plan *p) { return p->acc + 5; }
 
-// Device buffers collected first and then cut from one allocation (256-byte
-// aligned pieces): some twenty cudaMalloc / cudaFree pairs took most of a small
-// plan's life (no8-nu72: create and destroy 5.0 ms, 1.6 ms as one).
-struct Arena {
-  std::vector<std::pair<void **, size_t>> parts;
-  size_t bytes = 0;
-  template <typename T>
-  void add(T **p, int64_t count) {
-    parts.push_back({reinterpret_cast<void **>(p), bytes});
-    bytes += (std::max<size_t>((size_t)count * sizeof(T), 1) + 255) / 256 * 256;
-  }
-  int allocate(void **block) {
-    CCT_CUDA(cudaMalloc(block, bytes));
-    for (auto &q : parts) *q.first = static_cast<char *>(*block) + q.second;
-    return CCT_OK;
-  }
-};
-
 // The accumulators, flags and digit histogram of a forward, zeroed.
 int clear_results(ccT_plan *p) {
   const size_t n = 5 + (size_t)p->d.nu * p->d.no;

@@ -17,6 +17,7 @@
 // once.  Per-CTA partials are summed by
 // tuple_sum_kernel and group_add_kernel in a fixed order, so results are bitwise reproducible.
 #include <algorithm>
+#include <type_traits>
 
 #include "cct_internal.cuh"
 #include "cct_reduce_block.cuh"
@@ -26,27 +27,65 @@ namespace {
 
 using namespace red;
 
-// Grid (block triple, tuple of the group); a group may mix tuple kinds, the
-// branch is uniform over a CTA.
+// Block triples of every tuple of the group, blockIdx.x-th and each
+// gridDim.x-th after it; a group may mix tuple kinds, the branch is uniform over
+// a CTA.
 template <Fill FILL>
-__global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t NP, int64_t vsize,
+__global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t NP, int ncta, int64_t vsize,
                                                       const __grid_constant__ TupleGroup grp,
                                                       const double *__restrict__ eh, const double *__restrict__ ep,
                                                       const double *__restrict__ vb,
                                                       const int16_t *__restrict__ table, double *__restrict__ xpart,
                                                       double *__restrict__ vpart, int *err) {
   extern __shared__ __align__(16) double dyn_smem[];
-  const int64_t cta = blockIdx.x;
-  const int u = blockIdx.y;
-  const TupleDev &t = grp.t[u];
-  const int S0 = table[3 * cta], S1 = table[3 * cta + 1], S2 = table[3 * cta + 2];
-  double *xp = xpart + (int64_t)u * gridDim.x + cta, *vp = vpart + u * vsize;
-  if (t.kind == kIJK)
-    reduce_block<kIJK, FILL>(nu, no, NP, t, eh, ep, vb, S0, S1, S2, xp, vp, dyn_smem, err);
-  else if (t.kind == kIJJ)
-    reduce_block<kIJJ, FILL>(nu, no, NP, t, eh, ep, vb, S0, S1, S2, xp, vp, dyn_smem, err);
-  else
-    reduce_block<kIIJ, FILL>(nu, no, NP, t, eh, ep, vb, S0, S1, S2, xp, vp, dyn_smem, err);
+  const Smem m(dyn_smem);
+  int u = blockIdx.x / ncta, c = blockIdx.x - u * ncta;
+  if (u >= grp.n) return;
+  int S0 = table[3 * c], S1 = table[3 * c + 1], S2 = table[3 * c + 2];
+  if (FILL == kBulk) {
+    init_copies(m);
+    start_copies(nu, no, NP, grp.t[u], vb, S0, S1, S2, m);
+  }
+  for (uint32_t round = 0;; round ^= 1) {
+    int u1 = u, c1 = c + gridDim.x;
+    while (c1 >= ncta) {
+      c1 -= ncta;
+      u1++;
+    }
+    const bool more = u1 < grp.n;
+    int T0 = 0, T1 = 0, T2 = 0;
+    if (more) {
+      T0 = table[3 * c1];
+      T1 = table[3 * c1 + 1];
+      T2 = table[3 * c1 + 2];
+    }
+    if (FILL == kBulk && !copies_landed(m, round, err)) return;
+    auto next = [&]() {
+      if (FILL == kBulk && more) {
+        __syncthreads();
+        start_copies(nu, no, NP, grp.t[u1], vb, T0, T1, T2, m);
+      }
+    };
+    const TupleDev &t = grp.t[u];
+    double *xp = xpart + (int64_t)u * ncta + c, *vp = vpart + u * vsize;
+    auto block = [&](auto kind) {
+      constexpr int KIND = decltype(kind)::value;
+      if constexpr (FILL != kBulk) fill_rows<KIND, FILL>(nu, no, NP, t, vb, S0, S1, S2, m.Xs, m.Vs);
+      reduce_compute<KIND>(nu, t, eh, ep, S0, S1, S2, xp, vp, m, next);
+    };
+    if (t.kind == kIJK)
+      block(std::integral_constant<int, kIJK>{});
+    else if (t.kind == kIJJ)
+      block(std::integral_constant<int, kIJJ>{});
+    else
+      block(std::integral_constant<int, kIIJ>{});
+    if (!more) break;
+    u = u1;
+    c = c1;
+    S0 = T0;
+    S1 = T1;
+    S2 = T2;
+  }
 }
 
 // Sums of one tuple's partials, weighted: tsum[0] = its E[4], then the v1
@@ -220,8 +259,13 @@ int launch_reduce_fill(const Dims &d, const TupleGroup &g, const double *eh, con
                                   cudaSharedmemCarveoutMaxShared));
     configured_device = dev;
   }
-  reduce_kernel<FILL><<<dim3((unsigned)d.ncta, (unsigned)g.n), RT, smem, s>>>(
-      d.nu, d.no, d.NP, vpart_size(d), g, eh, ep, vb, cta_table, xpart, vpart, err);
+  static int nsm = 0;
+  if (nsm == 0) CCT_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  // up to two rounds of two CTAs per SM: a CTA per triple (no4-nu36: 79 us a
+  // forward, 80 with every CTA taking two)
+  const int64_t total = d.ncta * g.n, blocks = total <= 4 * nsm ? total : 2 * nsm;
+  reduce_kernel<FILL><<<(unsigned)blocks, RT, smem, s>>>(d.nu, d.no, d.NP, (int)d.ncta, vpart_size(d), g, eh, ep, vb,
+                                                         cta_table, xpart, vpart, err);
   CCT_CUDA(cudaGetLastError());
   return CCT_OK;
 }

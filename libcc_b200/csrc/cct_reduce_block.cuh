@@ -101,13 +101,13 @@ __device__ __forceinline__ int64_t voe_tile(int c, int no, int nb, const TupleDe
 }
 
 constexpr int kReduceWaitLimit = 1 << 22;
-__device__ __forceinline__ bool wait_landed(uint32_t bar, int *err) {
+__device__ __forceinline__ bool wait_landed(uint32_t bar, uint32_t parity, int *err) {
   for (int it = 0; it < kReduceWaitLimit; it++) {
     uint32_t ok;
     asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0; selp.u32 %0, 1, 0, p; }"
+        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
         : "=r"(ok)
-        : "r"(bar)
+        : "r"(bar), "r"(parity)
         : "memory");
     if (ok) return true;
   }
@@ -115,64 +115,100 @@ __device__ __forceinline__ bool wait_landed(uint32_t bar, int *err) {
   return false;
 }
 
-// Fills X and V; false when the bounded wait for the copies ran out (the error
-// word is then set and the CTA must write nothing).
-template <int KIND, Fill FILL>
-__device__ __forceinline__ bool fill_block(int nu, int no, int64_t NP, const TupleDev &t,
-                                           const double *__restrict__ vb, int S0, int S1, int S2, const int slot[6],
-                                           double *Xs, double *Vs, uint64_t *bar, int *err) {
-  constexpr int NG = KIND == kIJK ? 3 : 2;  // GEMM outputs of the tuple
+// Shared memory of a reduction CTA.
+struct Smem {
+  double *Xs, *Vs;
+  double (*part)[RT / 32][RB][3];  // [axis][warp][l][col]
+  double *red;
+  uint64_t *bar;
+  __device__ __forceinline__ explicit Smem(double *dyn) {
+    Xs = dyn;
+    Vs = Xs + kXBlocks * SL;
+    part = reinterpret_cast<double (*)[RT / 32][RB][3]>(Vs + 3 * VPAIR);
+    red = Vs + 3 * VPAIR + 3 * (RT / 32) * RB * 3;
+    bar = reinterpret_cast<uint64_t *>(red + RT / 32);
+  }
+};
+
+// kBulk: the barrier of the copies, once per CTA (ends with a block barrier).
+__device__ __forceinline__ void init_copies(const Smem &m) {
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(m.bar)));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  __syncthreads();
+}
+// kBulk: starts the copies of a block triple into X and V.  Every thread has read
+// what it needs of the blocks before (a block barrier lies between).  One
+// copy per thread, spread over the warps: X block c = 6 g + q, then the VOE
+// tiles.
+__device__ __forceinline__ void start_copies(int nu, int no, int64_t NP, const TupleDev &t,
+                                             const double *__restrict__ vb, int S0, int S1, int S2, const Smem &m) {
   const int tid = threadIdx.x, nb = nb_of(nu);
-  auto Sm = [&](int m) { return sel3(m, S0, S1, S2); };
-  if (FILL == kBulk) {
-    const uint32_t sbar = (uint32_t)__cvta_generic_to_shared(bar);
+  const int nx = t.kind == kIJK ? 18 : 12;  // X blocks: three GEMM outputs, or a degenerate tuple's two
+  const uint32_t sbar = (uint32_t)__cvta_generic_to_shared(m.bar);
+  int slot[6];
+  orbit_slots(S0, S1, S2, slot);
+  auto Sm = [&](int q) { return sel3(q, S0, S1, S2); };
+  if (tid == 0) {
     int nq = 0;
 #pragma unroll
     for (int q = 0; q < 6; q++) nq += slot[q] == q;
-    if (tid == 0) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar));
-      asm volatile("fence.mbarrier_init.release.cluster;");
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sbar),
-                   "r"((uint32_t)(NG * nq * SL * 8 + kVTiles * VTILE * 8))
-                   : "memory");
-    }
-    __syncthreads();
-    // one copy per thread, spread over the warps: X block c = 6 g + q, then the VOE tiles
-    const int c = (tid >> 5) + (tid & 31) * (RT / 32);
-    if (c < 6 * NG) {
-      const int q = c % 6;
-      int sq = 0, O0 = 0, O1 = 0, O2 = 0;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sbar),
+                 "r"((uint32_t)(nx / 6 * nq * SL * 8 + kVTiles * VTILE * 8))
+                 : "memory");
+  }
+  const int c = (tid >> 5) + (tid & 31) * (RT / 32);
+  if (c < nx) {
+    const int q = c % 6;
+    int sq = 0, O0 = 0, O1 = 0, O2 = 0;
 #pragma unroll
-      for (int p = 0; p < 6; p++)
-        if (p == q) {
-          sq = slot[p];
-          O0 = Sm(pm(p, 0));
-          O1 = Sm(pm(p, 1));
-          O2 = Sm(pm(p, 2));
-        }
-      if (sq == q) {
-        const double *src = t.x[c / 6] + xblock_base(O0, O1, O2, nu, NP);
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                (uint32_t)__cvta_generic_to_shared(Xs + c * SL)),
-            "l"(src), "r"(SL * 8), "r"(sbar)
-            : "memory");
+    for (int p = 0; p < 6; p++)
+      if (p == q) {
+        sq = slot[p];
+        O0 = Sm(pm(p, 0));
+        O1 = Sm(pm(p, 1));
+        O2 = Sm(pm(p, 2));
       }
-    } else if (c < 6 * NG + kVTiles) {
-      const int v = c - 6 * NG;
+    if (sq == q) {
+      const double *src = sel3(c / 6, t.x[0], t.x[1], t.x[2]) + xblock_base(O0, O1, O2, nu, NP);
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-              (uint32_t)__cvta_generic_to_shared(Vs + v * VTILE)),
-          "l"(vb + voe_tile(v, no, nb, t, S0, S1, S2)), "r"(VTILE * 8), "r"(sbar)
+              (uint32_t)__cvta_generic_to_shared(m.Xs + c * SL)),
+          "l"(src), "r"(SL * 8), "r"(sbar)
           : "memory");
     }
-    bool ok = wait_landed(sbar, err);
-    if (!__syncthreads_and(ok)) {
-      wait_landed(sbar, err);
-      return false;
-    }
-    return true;
+  } else if (c < nx + kVTiles) {
+    const int v = c - nx;
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+            (uint32_t)__cvta_generic_to_shared(m.Vs + v * VTILE)),
+        "l"(vb + voe_tile(v, no, nb, t, S0, S1, S2)), "r"(VTILE * 8), "r"(sbar)
+        : "memory");
   }
+}
+// kBulk: waits for the copies of the parity's round.  False (for the whole CTA)
+// when the bounded wait ran out: the error word is set, the copies have had a
+// second limit to land, and the CTA must return.
+__device__ __forceinline__ bool copies_landed(const Smem &m, uint32_t parity, int *err) {
+  const uint32_t sbar = (uint32_t)__cvta_generic_to_shared(m.bar);
+  const bool ok = wait_landed(sbar, parity, err);
+  if (__syncthreads_and(ok)) return true;
+  wait_landed(sbar, parity, err);
+  return false;
+}
+
+// kRows, kRowsCoherent: X and V by the threads; block barriers before and after.
+template <int KIND, Fill FILL>
+__device__ __forceinline__ void fill_rows(int nu, int no, int64_t NP, const TupleDev &t,
+                                          const double *__restrict__ vb, int S0, int S1, int S2, double *Xs,
+                                          double *Vs) {
+  constexpr int NG = KIND == kIJK ? 3 : 2;  // GEMM outputs of the tuple
+  const int tid = threadIdx.x, nb = nb_of(nu);
+  auto Sm = [&](int m) { return sel3(m, S0, S1, S2); };
+  int slot[6];
+  orbit_slots(S0, S1, S2, slot);
+  __syncthreads();
 #pragma unroll
   for (int g = 0; g < NG; g++) {
     const double *X = t.x[g];
@@ -196,13 +232,13 @@ __device__ __forceinline__ bool fill_block(int nu, int no, int64_t NP, const Tup
   for (int e = tid; e < kVTiles * VTILE; e += RT)
     Vs[e] = __ldg(vb + voe_tile(e / VTILE, no, nb, t, S0, S1, S2) + e % VTILE);
   __syncthreads();
-  return true;
 }
 
-// One CTA per unordered block triple {A<=B<=C}.  Each thread evaluates two
-// orbits -- the six index permutations of one (a,b,c) of block (A,B,C) share
-// six W values and one denominator -- and accumulates E[4] and the v1 updates
-// of all six elements; fixed-order sums over the CTA follow.
+// One unordered block triple {A<=B<=C}, its X and V in shared memory.  Each thread
+// evaluates two orbits -- the six index permutations of one (a,b,c) of block
+// (A,B,C) share six W values and one denominator -- and accumulates E[4] and
+// the v1 updates of all six elements; next() runs once every read of X and V
+// is done (it may hold block barriers), then the fixed-order sums over the CTA.
 //
 // Entries of indices >= nu are whatever lies in the padding of the X blocks:
 // only elements whose three indices are < nu are evaluated.
@@ -210,25 +246,22 @@ __device__ __forceinline__ bool fill_block(int nu, int no, int64_t NP, const Tup
 // What bounds it: the X traffic (3 nu^3 doubles a tuple).  The blocks reach
 // shared memory by bulk copies in the order they lie in memory, so no thread
 // spends an instruction on them; W is summed from them in registers as it is
-// used.  Two CTAs per SM (97 KB each): one's copies run under the other's
-// arithmetic.  At no24-nu320 (3-digit X) a launch took 245 us when threads
-// staged W through registers term by term (four CTAs per SM, 1740
-// instructions a warp), 203 us now.
-template <int KIND, Fill FILL>
-__device__ __forceinline__ void reduce_block(int nu, int no, int64_t NP, const TupleDev &t,
-                                             const double *__restrict__ eh, const double *__restrict__ ep,
-                                             const double *__restrict__ vb, const int S0, const int S1, const int S2,
-                                             double *__restrict__ xpart_slot, double *__restrict__ vpart,
-                                             double *__restrict__ dyn_smem, int *err) {
+// used.  Two CTAs per SM (97 KB each) walk over the block triples, the next
+// triple's copies started before the sums of the last.  At no24-nu320 (3-digit X)
+// a launch took 245 us when threads staged W through registers term by term
+// (four CTAs per SM, 1740 instructions a warp), 203 us with one CTA per block
+// triple on bulk copies, 181 us now.
+template <int KIND, class Next>
+__device__ __forceinline__ void reduce_compute(int nu, const TupleDev &t, const double *__restrict__ eh,
+                                               const double *__restrict__ ep, const int S0, const int S1,
+                                               const int S2, double *__restrict__ xpart_slot,
+                                               double *__restrict__ vpart, const Smem &m, Next next) {
   constexpr int NTERM = KIND == kIJK ? 3 : 4, NG = KIND == kIJK ? 3 : 2;
-  double *Xs = dyn_smem, *Vs = Xs + kXBlocks * SL;
-  double(*part)[RT / 32][RB][3] = reinterpret_cast<double(*)[RT / 32][RB][3]>(Vs + 3 * VPAIR);  // [axis][warp][l][col]
-  double *red = Vs + 3 * VPAIR + 3 * (RT / 32) * RB * 3;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(red + RT / 32);
+  double *Xs = m.Xs, *Vs = m.Vs, *red = m.red;
+  auto part = m.part;
   const int tid = threadIdx.x;
   int slot[6];
   orbit_slots(S0, S1, S2, slot);
-  if (!fill_block<KIND, FILL>(nu, no, NP, t, vb, S0, S1, S2, slot, Xs, Vs, bar, err)) return;
 
   const double dijk = eh[t.i] + eh[t.j] + eh[t.k];
   double x3 = 0.0;
@@ -327,6 +360,7 @@ __device__ __forceinline__ void reduce_block(int nu, int no, int64_t NP, const T
       }
     }
   }
+  next();
   // ---- fixed-order sums: over the lanes of equal l0 / l1 / l2 (orbit_coords),
   // then over the warps, each of which holds all eight values of every axis
   const int warp = tid >> 5, lane = tid & 31;
