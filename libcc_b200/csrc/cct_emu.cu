@@ -48,6 +48,12 @@
 // bound by its shared-memory operand reads (A 4 KB + B 2.5 KB); a wide one
 // reads A once for up to three B slices.
 //
+// The last column tile covers only what is left of nu: where 16 or 32 columns
+// do, its B blocks hold that many rows and every A slice meets all its B slices
+// in one MMA (7 x 32 <= 256 columns).  A 16-column item of a 7-digit no16-nu200
+// launch (200 = 3 x 64 + 8) takes some 0.55 of a full item's MMA time and stores a
+// quarter of it; the tuple went from 311 to 285 us.
+//
 // Persistent kernel, one CTA of 64 + 32 NDW threads per SM (NDW = 16 drain
 // warps at 80 registers a thread: the drain is latency-bound, and 16 warps
 // took a 3-digit tuple from 0.54 to 0.46 ms against 8 warps at 128
@@ -70,6 +76,7 @@
 // timeout sets the error word, the producer waits for its copies in flight,
 // the issuer for its MMAs, and the CTA frees its tensor memory and returns.
 #include <algorithm>
+#include <numeric>
 #include <type_traits>
 
 #include "cct_internal.cuh"
@@ -231,6 +238,10 @@ struct EmuArgs {
   const int *tileExp;  // adaptive plans: see EmuOperands::tileExp; nullptr: every item runs S digits
   unsigned long long *slice_hist;
   int nu, no, njobs, kchunks, tiles_m, tiles_n;
+  int nl;   // rows per B block of the last column tile (EmuOperands::nl)
+  // a CTA's n-th item is n G + (b + rot n) mod G (G CTAs): from one item to the
+  // next G + rot items on, or rot where the place wraps, each as row and column tiles
+  int rot, step_m[2], step_n[2];
   int sop;  // digit slices stored per K chunk in the operands (>= the S of the launch)
   int64_t NP;   // X row stride; columns at or past it (a partial last N tile) are not stored
   int64_t NPe;  // rows per (y,z) of the B digits and expF: tiles_n * EBN
@@ -241,21 +252,24 @@ struct EmuArgs {
 constexpr int kNoRowExp = -30000;  // exponent of an all-zero row: never the maximum
 
 // A CTA's work items, one after the other: (job, row tile, column tile), the
-// column tile fastest, every gridDim.x-th.
+// column tile fastest.  rot keeps a CTA from meeting the same column tile every
+// time when that one is narrow (148 CTAs and four column tiles: always).
 struct ItemCursor {
-  int jb, tm, tn, step_m, step_n;
+  int jb, tm, tn, pos;
   __device__ __forceinline__ explicit ItemCursor(const EmuArgs &a) {
-    step_m = (int)gridDim.x / a.tiles_n;
-    step_n = (int)gridDim.x - step_m * a.tiles_n;
-    tm = (int)blockIdx.x / a.tiles_n;
-    tn = (int)blockIdx.x - tm * a.tiles_n;
+    pos = (int)blockIdx.x;
+    tm = pos / a.tiles_n;
+    tn = pos - tm * a.tiles_n;
     jb = tm / a.tiles_m;
     tm -= jb * a.tiles_m;
   }
   __device__ __forceinline__ bool valid(const EmuArgs &a) const { return jb < a.njobs; }
   __device__ __forceinline__ void next(const EmuArgs &a) {
-    tn += step_n;
-    tm += step_m;
+    pos += a.rot;
+    const int wrap = pos >= (int)gridDim.x;
+    if (wrap) pos -= (int)gridDim.x;
+    tn += a.step_n[wrap];
+    tm += a.step_m[wrap];
     if (tn >= a.tiles_n) {
       tn -= a.tiles_n;
       tm++;
@@ -293,7 +307,8 @@ __device__ __forceinline__ double pow2(int e) {
   return (e >= -1022 && e <= 1023) ? __longlong_as_double((long long)(e + 1023) << 52) : ldexp(1.0, e);
 }
 
-template <int S, int EBN>
+// NAR: the last column tile is narrow (nl < EBN).
+template <int S, int EBN, bool NAR>
 __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs args) {
   static_assert(S * EBN <= 512 && EBN % 16 == 0, "S diagonals of EBN columns must fit the tensor memory");
   constexpr int B_BLK = EBN * kEmuKC;
@@ -375,6 +390,9 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
           if (nx2.valid(args)) job2 = args.jobs[nx2.jb];
         }
         const bool run = sl == S && whole;  // a stage's chunks are one contiguous run per operand
+        const uint32_t bblk = NAR && tn == args.tiles_n - 1 ? (uint32_t)args.nl * kEmuKC : (uint32_t)B_BLK;
+        const uint32_t cb = S * bblk;                   // bytes of a B chunk here and in HBM
+        const int64_t gb = (int64_t)args.sop * bblk;
         for (int h = 0; h < job.nhalves && ok; h++) {
           const int8_t *A = (h == 0 ? args.E8 + job.x1 * aslab : args.E8T + job.x2 * aslab) + (int64_t)tm * KC * GA;
           const int8_t *B = args.F8 + job.fyz[h] * bslab + (int64_t)tn * KC * GB;
@@ -386,18 +404,18 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
             }
             const uint32_t bar = full0 + 8 * st, da = a0 + st * SA, db = b0 + st * SB;
             if (run) {
-              mbar_expect_tx_at(bar, nch * (CA + CB));
+              mbar_expect_tx_at(bar, nch * (CA + cb));
               bulk_load_at(da, A, nch * CA, bar);
-              bulk_load_at(db, B, nch * CB, bar);
+              bulk_load_at(db, B, nch * cb, bar);
             } else {  // the leading sl digit slices of each chunk
-              mbar_expect_tx_at(bar, nch * (uint32_t)sl * (A_BLK + B_BLK));
+              mbar_expect_tx_at(bar, nch * (uint32_t)sl * (A_BLK + bblk));
               for (uint32_t c = 0; c < nch; c++) {
                 bulk_load_at(da + c * CA, A + c * GA, (uint32_t)sl * A_BLK, bar);
-                bulk_load_at(db + c * CB, B + c * GB, (uint32_t)sl * B_BLK, bar);
+                bulk_load_at(db + c * cb, B + c * gb, (uint32_t)sl * bblk, bar);
               }
             }
             A += KS * GA;
-            B += KS * GB;
+            B += KS * gb;
             if (++st == ST) {
               st = 0;
               ph ^= 1;
@@ -484,7 +502,7 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
         };
         // A slice t meets n = s - t B slices, taken as MMAs of at most MPS
         // slices whose sizes differ by one.
-        auto row = [&](uint32_t loA, uint32_t loB, int s, int t, uint32_t accumulate) {
+        auto row_full = [&](uint32_t loA, uint32_t loB, int s, int t, uint32_t accumulate) {
           const int n = s - t;
           const int parts = (n + MPS - 1) / MPS;
           const int base = n / parts, extra = n - base * parts;
@@ -492,11 +510,27 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
           for (int q = 0; q < parts; q++)
             mma(loA, loB, t, q * base + (q < extra ? q : extra), base + (q < extra ? 1 : 0), accumulate);
         };
+        // The same in a narrow last column tile: one MMA of s - t slices of nl.
+        auto row_narrow = [&](uint32_t loA, uint32_t loB, int s, int t, uint32_t accumulate) {
+          const uint32_t idesc = idesc0 | ((uint32_t)((s - t) * args.nl >> 3) << 17);
+          asm volatile(
+              "{ .reg .pred p; .reg .b64 a, b; setp.ne.b32 p, %6, 0; mov.b64 a, {%1, %2}; mov.b64 b, {%3, %4}; "
+              "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %5, p; }" ::"r"(acc + (uint32_t)(t * args.nl)),
+              "r"(loA + (uint32_t)(t * (A_BLK >> 4))), "r"(hiA), "r"(loB), "r"(hiB), "r"(idesc), "r"(accumulate));
+        };
         const int stages = (KC + KS - 1) / KS * nh;
-        // The stages of the item at a digit count fixed at compile time:
-        // straight-line MMAs with constant shapes and offsets.
-        auto run_item = [&](auto slc) {
+        // The stages of the item at a digit count (and tile form) fixed at
+        // compile time: straight-line MMAs with constant shapes and offsets.
+        auto run_item = [&](auto slc, auto narrow) {
           constexpr int SLC = decltype(slc)::value;
+          constexpr bool NARROW = decltype(narrow)::value;
+          auto row = [&](uint32_t loA, uint32_t loB, int s, int t, uint32_t accumulate) {
+            if constexpr (NARROW)
+              row_narrow(loA, loB, s, t, accumulate);
+            else
+              row_full(loA, loB, s, t, accumulate);
+          };
+          const uint32_t cb4 = NARROW ? (uint32_t)(S * kEmuKC * args.nl) >> 4 : (uint32_t)(CB >> 4);
           int left = KC;  // chunks of the half
           for (int q = 0; q < stages; q++) {
             if (!ready && !mbar_wait(&full[st], ph, args.err, abort_flag)) {
@@ -537,19 +571,29 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
             }
             if (two) {
 #pragma unroll
-              for (int t = SLC - 1; t >= 0; t--) row(loA + (CA >> 4), loB + (CB >> 4), SLC, t, 1u);
+              for (int t = SLC - 1; t >= 0; t--) row(loA + (CA >> 4), loB + cb4, SLC, t, 1u);
             }
             if (!kLate) mma_commit(slot);
           }
         };
-        switch (sl) {
-          case 1: run_item(std::integral_constant<int, 1>{}); break;
-          case 2: if constexpr (S >= 2) run_item(std::integral_constant<int, 2>{}); break;
-          case 3: if constexpr (S >= 3) run_item(std::integral_constant<int, 3>{}); break;
-          case 4: if constexpr (S >= 4) run_item(std::integral_constant<int, 4>{}); break;
-          case 5: if constexpr (S >= 5) run_item(std::integral_constant<int, 5>{}); break;
-          case 6: if constexpr (S >= 6) run_item(std::integral_constant<int, 6>{}); break;
-          default: if constexpr (S >= 7) run_item(std::integral_constant<int, 7>{}); break;
+        auto run = [&](auto narrow) {
+          switch (sl) {
+            case 1: run_item(std::integral_constant<int, 1>{}, narrow); break;
+            case 2: if constexpr (S >= 2) run_item(std::integral_constant<int, 2>{}, narrow); break;
+            case 3: if constexpr (S >= 3) run_item(std::integral_constant<int, 3>{}, narrow); break;
+            case 4: if constexpr (S >= 4) run_item(std::integral_constant<int, 4>{}, narrow); break;
+            case 5: if constexpr (S >= 5) run_item(std::integral_constant<int, 5>{}, narrow); break;
+            case 6: if constexpr (S >= 6) run_item(std::integral_constant<int, 6>{}, narrow); break;
+            default: if constexpr (S >= 7) run_item(std::integral_constant<int, 7>{}, narrow); break;
+          }
+        };
+        if constexpr (NAR) {
+          if (cur.tn == args.tiles_n - 1)
+            run(std::true_type{});
+          else
+            run(std::false_type{});
+        } else {
+          run(std::false_type{});
         }
         if (!ok) break;
         mma_commit(su32(&acc_full[ab]));
@@ -599,6 +643,8 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
       const uint32_t m = (uint32_t)cur.tm * EBM + row;
       const bool live = m < (uint32_t)M;
       const int n0 = cur.tn * EBN + cbase;
+      // columns of the tile, which are also its diagonals' distance in the tensor memory
+      const int cols = NAR && cur.tn == args.tiles_n - 1 ? args.nl : EBN;
       // The diagonals are summed exactly in int64, acc = sum_d D_d 2^(7(sl-1-d)): |D_d| <= 2 (d+1) K 64^2, so below 2^63 for six
       // digits and K <= 32000; a seventh is added in FP64.  One conversion
       // and one power-of-two scaling per element follow.
@@ -633,6 +679,7 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
       // warp-uniform decision: the tcgen05.ld below are .sync.aligned
       if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[ab], use & 1, args.err, abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
+      if (cbase < cols) {  // (a narrow tile leaves the last warps without columns)
       // Pairs of diagonals first, D_d 128 + D_d+1 (one widening multiply-add
       // each), then the pairs.  (Loading every diagonal before one wait, to
       // hold the tensor memory for less, spilled at 96 registers: 7 digits
@@ -643,7 +690,7 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
         const int w = CW - c0 >= 16 ? 16 : (CW - c0 >= 8 ? 8 : 4);  // chunk widths 16, then 8 or 4
         uint32_t v[2][16];
         auto load = [&](int d) {
-          const uint32_t addr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((ab * S + d) * EBN + cbase + c0);
+          const uint32_t addr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * S * EBN + d * cols + cbase + c0);
           if (w == 16)
             tmem_ld16(addr, v[d & 1]);
           else if (w == 8)
@@ -694,6 +741,7 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
       // wrote half a sector each and doubled the write traffic); a quad of
       // columns stays inside one block.  NP is a multiple of 4: a quad is
       // stored whole or not at all.
+      const int send = min((int)args.NP, cur.tn * EBN + cols);
       auto store = [&](auto scale) {
 #pragma unroll
         for (int j = 0; j < CW; j += 4) {
@@ -701,7 +749,7 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
 #pragma unroll
           for (int u = 0; u < 4; u++) x[u] = value(j + u) * scale(__shfl_sync(0xffffffffu, eBl, j + u));
           const int sc = n0 + j;
-          if (live && sc < (int)args.NP)
+          if (live && sc < send)
             st_global_v4(xrow + (args.xblocked ? (sc >> 3) * 512 + (sc & 7) : sc), x[0], x[1], x[2], x[3]);
         }
       };
@@ -709,6 +757,11 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
         store([&](int e) { return __hiloint2double((e0 + 1023 + e) << 20, 0); });
       else
         store([&](int e) { return pow2(e0 + e); });
+      } else {
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[ab]);
+      }
       dig = dig1;
       sl = dig.digits<S>(args);
       out = out1;
@@ -880,24 +933,26 @@ __global__ void digits_e_kernel(const double *__restrict__ E, int no, int nu, in
 }
 
 __global__ void digits_f_kernel(const double *__restrict__ F, int no, int nu, int64_t NP, int64_t NPe, int64_t KP,
-                                int64_t KP8, int S, int ebn, const int16_t *__restrict__ expF,
+                                int64_t KP8, int S, int ebn, int nl, const int16_t *__restrict__ expF,
                                 int8_t *__restrict__ F8) {
   const int64_t rows = (int64_t)no * no * NP;
   const int64_t KC = KP8 / kEmuKC, tiles_n = NPe / ebn;
-  const int64_t bblk = (int64_t)ebn * kEmuKC;
   const int lane = threadIdx.x & 31;
   int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (; row < rows; row += stride) {
     const int64_t yz = row / NP, n = row - yz * NP;
     const int64_t z = yz % no;
+    const bool last = n / ebn == tiles_n - 1;  // its blocks hold nl rows
+    if (last && n % ebn >= nl) continue;
+    const int64_t bblk = (int64_t)(last ? nl : ebn) * kEmuKC;
     const int e = expF[z * NPe + n];
     for (int64_t k = 4 * lane; k < KP8; k += 128) {
       uint32_t w[kEmuDigitCap];
       digits4(F + row * KP, k, nu + no, e, S, w);
       const int64_t kc = k / kEmuKC;
       const int kb = (int)(k - kc * kEmuKC);
-      const int64_t b = ((yz * tiles_n + n / ebn) * KC + kc) * S * bblk + blk_off((int)(n % ebn), kb);
+      const int64_t b = (yz * tiles_n + n / ebn) * KC * S * ebn * kEmuKC + kc * S * bblk + blk_off((int)(n % ebn), kb);
       for (int t = 0; t < S; t++) *reinterpret_cast<uint32_t *>(F8 + b + (int64_t)t * bblk) = w[t];
     }
   }
@@ -905,16 +960,16 @@ __global__ void digits_f_kernel(const double *__restrict__ F, int no, int nu, in
 
 int g_num_sms[64] = {0};
 
-template <int S, int EBN>
-int launch_emu_s(const EmuOperands &o, const Dims &d, const EmuJob *jobs_dev, int njobs, int *err, cudaStream_t s,
+template <int S, int EBN, bool NAR>
+int launch_emu_n(const EmuOperands &o, const Dims &d, const EmuJob *jobs_dev, int njobs, int *err, cudaStream_t s,
                  bool blocked) {
   constexpr int smem = emu_stages<S, EBN>() * KS * S * (A_BLK + EBN * kEmuKC) + 1024;
   static int configured_device = -1;
   int dev = 0;
   CCT_CUDA(cudaGetDevice(&dev));
   if (configured_device != dev) {
-    CCT_CUDA(cudaFuncSetAttribute(wbuild_emu_kernel<S, EBN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CCT_CUDA(cudaFuncSetAttribute(wbuild_emu_kernel<S, EBN>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    CCT_CUDA(cudaFuncSetAttribute(wbuild_emu_kernel<S, EBN, NAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CCT_CUDA(cudaFuncSetAttribute(wbuild_emu_kernel<S, EBN, NAR>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   cudaSharedmemCarveoutMaxShared));
     configured_device = dev;
   }
@@ -958,9 +1013,25 @@ int launch_emu_s(const EmuOperands &o, const Dims &d, const EmuJob *jobs_dev, in
     return CCT_ERR_INVALID;
   }
   const int grid = (int)(items < g_num_sms[dev] ? items : g_num_sms[dev]);
-  wbuild_emu_kernel<S, EBN><<<grid, EMU_THREADS, smem, s>>>(a);
+  a.nl = o.nl;
+  a.rot = 0;
+  if (NAR)  // spread the narrow tiles: G + rot and the column tiles without a common factor
+    while (a.rot + 1 < grid && std::gcd(grid + a.rot, a.tiles_n) != 1) a.rot++;
+  for (int w = 0; w < 2; w++) {
+    const int step = w ? a.rot : grid + a.rot;
+    a.step_m[w] = step / a.tiles_n;
+    a.step_n[w] = step % a.tiles_n;
+  }
+  wbuild_emu_kernel<S, EBN, NAR><<<grid, EMU_THREADS, smem, s>>>(a);
   CCT_CUDA(cudaGetLastError());
   return CCT_OK;
+}
+
+template <int S, int EBN>
+int launch_emu_s(const EmuOperands &o, const Dims &d, const EmuJob *jobs_dev, int njobs, int *err, cudaStream_t s,
+                 bool blocked) {
+  return o.nl < EBN ? launch_emu_n<S, EBN, true>(o, d, jobs_dev, njobs, err, s, blocked)
+                    : launch_emu_n<S, EBN, false>(o, d, jobs_dev, njobs, err, s, blocked);
 }
 
 }  // namespace
@@ -975,6 +1046,10 @@ int emu_build_operands(const Dims &d, const double *E, const double *F, EmuOpera
     set_error("emulated operands need NPe >= NP a multiple of their N tile, KP8 a multiple of 32 and "
               "slices x N <= 512");
     return CCT_ERR_INVALID;
+  }
+  {
+    const int64_t left = d.nu - (o->NPe / o->ebn - 1) * o->ebn;  // columns of the last N tile
+    o->nl = left <= 16 ? 16 : (left <= 32 ? 32 : o->ebn);
   }
   const int64_t rowsE = (int64_t)d.no * d.nu * d.nu, rowsF = (int64_t)d.no * d.no * d.NP;
   auto grid_rows = [](int64_t rows) {
@@ -1004,7 +1079,7 @@ int emu_build_operands(const Dims &d, const double *E, const double *F, EmuOpera
   if (o->NPe > d.NP)  // the padding rows of a partial last N tile stay zero
     CCT_CUDA(cudaMemsetAsync(o->F8, 0, (size_t)o->slices * d.no * d.no * o->NPe * o->KP8, s));
   digits_f_kernel<<<grid_rows(rowsF), 256, 0, s>>>(F, d.no, d.nu, d.NP, o->NPe, d.KP, o->KP8, o->slices, o->ebn,
-                                                   o->expF, o->F8);
+                                                   o->nl, o->expF, o->F8);
   CCT_CUDA(cudaGetLastError());
   if (o->adaptive) {
     const int tiles_n = (int)(o->NPe / o->ebn), nbt = d.no * tiles_n;

@@ -180,6 +180,9 @@ struct EmuOperands {
   int slices = kEmuMaxSlices;                // digit slices stored per K chunk
   int run_slices = kEmuMaxSlices;            // digits the W build runs (<= slices; the calibrated count)
   int ebn = 0;                               // N tile of F8 (rows per B block)
+  // Rows per B block of the last N tile: 16 or 32 where that covers what is left
+  // of nu, else ebn.  Its K chunks are nl rows a slice, at the tile's usual place.
+  int nl = 0;
   int64_t NPe = 0;                           // rows per (y,z) in F8 and expF: NP rounded up to ebn
   int64_t KP8 = 0;                           // digit row length: round_up(nu+no, 32)
   int64_t tiles_m = 0;                       // ceil(nu^2 / 128) row tiles per occupied index
