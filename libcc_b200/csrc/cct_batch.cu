@@ -519,7 +519,7 @@ int ensure_emu_plans(ccT_batch *b) {
     o.precision = CCT_PREC_INT8_EMU;
     o.device = b->device;
     o.vvvo_mode = CCT_VVVO_EXPANDED;
-    CCT_TRY(ccT_plan_create(&b->emu_plans[s], S.no, S.nu, &o));
+    CCT_TRY(plan_create(&b->emu_plans[s], S.no, S.nu, &o, 1));  // it runs single tuples: one X set a group
     CCT_TRY(ccT_set_inputs(b->emu_plans[s], S.eh, S.ep, S.t1, S.t2, S.vm, S.voe, S.vvvo, CCT_MEM_DEVICE));
     double ets = 0.0, etd = 0.0;
     CCT_TRY(ccT_forward(b->emu_plans[s], 0, 1, &ets, &etd, nullptr));

@@ -297,6 +297,10 @@ int assemble_w_fortran(const Dims &d, const Tuple &t, double *const X[3], double
 
 // cct_plan.cu: the dimensions and split-integer operands of an emulated plan,
 // for the batched executor that runs many plans' W builds in grouped launches
+// ccT_plan_create; group_cap bounds the tuples per group, and with them the X
+// ring (the legacy driver hook hands tuples over one at a time, in any order;
+// a batch's emulated plans calibrate on single tuples).
+int plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *opt, int group_cap);
 const Dims &plan_dims(const ccT_plan *p);
 const EmuOperands &plan_emu(const ccT_plan *p);
 

@@ -693,9 +693,7 @@ int64_t ccT_num_tuples(int64_t no) {
 
 }  // extern "C"
 
-// ccT_plan_create; group_cap bounds the tuples per group (the legacy driver
-// hook hands tuples over one at a time, in any order).
-static int plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *opt, int group_cap) {
+int cct::plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *opt, int group_cap) {
   if (!out) {
     set_error("plan pointer is NULL");
     return CCT_ERR_INVALID;
