@@ -26,7 +26,11 @@
 // own waits point further back, so the queue cannot deadlock; each wait is
 // also bounded (on timeout the error word is set and the item proceeds).
 // Data produced inside the kernel is read through L2 (ld.global.cg /
-// cp.async.cg), never through the incoherent L1.
+// cp.async.cg / bulk copies), never through the incoherent L1.  A reduction
+// block is one CTA on its SM, so nothing hides its copies: X lies in 8 x 8 x 8
+// blocks and a block triple's 18 blocks and its VOE tiles come as bulk copies
+// in flight together, where reading rows of X with one load a thread and element
+// took 1181 ms on 96 uneven systems (no 3-12, nu 24-140) against 954 ms.
 //
 // A second executor (mode 1) runs the same items as grouped launches: per
 // tuple group, one launch of 128-row W-build tiles (three CTAs per SM) on one
@@ -233,6 +237,11 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
   __shared__ double red[kBT + 1];
   __shared__ int64_t s_item;
   __shared__ int s_flag;
+  __shared__ uint64_t s_bar;  // the reduction's copies (the dynamic memory is the W tiles' too)
+  red::Smem m(reinterpret_cast<double *>(smem));
+  m.bar = &s_bar;
+  red::init_copies(m);
+  uint32_t round = 0;
   int *const wb_done = A.counters + 1;
   int *const rd_done = wb_done + A.ntuple;
   int *const group_rd = rd_done + A.ntuple;
@@ -252,7 +261,7 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
         spin_until(group_rd + (T.group - kRing), A.group_rd_items[T.group - kRing], A.err, A.spin_limit);
       __syncthreads();
       const int tile_m = it.w / S.tiles_n, tile_n = it.w - tile_m * S.tiles_n;
-      wb::wbuild_tile<BN, kBTM>(A.jobs[(int64_t)t * 3 + it.z], S.nu, S.KP, S.nu + S.no, S.NP, tile_m, tile_n, false, smem);
+      wb::wbuild_tile<BN, kBTM>(A.jobs[(int64_t)t * 3 + it.z], S.nu, S.KP, S.nu + S.no, S.NP, tile_m, tile_n, true, smem);
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) atomicAdd(wb_done + t, 1);
@@ -271,18 +280,25 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
       td.weight = T.kind == kIJK ? 1.0 : 0.5;
       const int c = it.z;
       const int S0 = S.cta_table[3 * c], S1 = S.cta_table[3 * c + 1], S2 = S.cta_table[3 * c + 2];
-      const red::Smem m(reinterpret_cast<double *>(smem));
-      auto block = [&](auto kind) {
-        constexpr int KIND = decltype(kind)::value;
-        red::fill_rows<KIND, red::kRowsCoherent>(S.nu, S.no, S.NP, td, S.vb, S0, S1, S2, m.Xs, m.Vs);
-        red::reduce_compute<KIND>(S.nu, td, S.eh, S.ep, S0, S1, S2, T.xpart + c, T.vpart, m, [] {});
-      };
-      if (T.kind == kIJK)
-        block(std::integral_constant<int, kIJK>{});
-      else if (T.kind == kIJJ)
-        block(std::integral_constant<int, kIJJ>{});
-      else
-        block(std::integral_constant<int, kIIJ>{});
+      // X was written by other CTAs of this kernel and shared memory by this
+      // one, both through the generic proxy; the copies are the async proxy's
+      asm volatile("fence.proxy.async;" ::: "memory");
+      __syncthreads();
+      red::start_copies(S.nu, S.no, S.NP, td, S.vb, S0, S1, S2, m);
+      const bool landed = red::copies_landed(m, round, A.err);
+      if (landed) {
+        auto block = [&](auto kind) {
+          constexpr int KIND = decltype(kind)::value;
+          red::reduce_compute<KIND>(S.nu, td, S.eh, S.ep, S0, S1, S2, T.xpart + c, T.vpart, m, [] {});
+        };
+        if (T.kind == kIJK)
+          block(std::integral_constant<int, kIJK>{});
+        else if (T.kind == kIJJ)
+          block(std::integral_constant<int, kIJJ>{});
+        else
+          block(std::integral_constant<int, kIIJ>{});
+      }
+      round ^= 1;
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -305,6 +321,7 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
           __threadfence();
         }
       }
+      if (!landed) return;  // the error word is set; the other CTAs take the queue's rest
     }
   }
 }
@@ -573,7 +590,7 @@ int build_schedule(ccT_batch *b) {
       h.j = t.j;
       h.k = t.k;
       h.njobs = t.kind == kIJK ? 3 : 2;
-      const int64_t xs = b->mode == 0 ? nu2 * d.NP : round_up(S.nu, kRB) * round_up(S.nu, kRB) * d.NP;  // X: rows / blocks
+      const int64_t xs = round_up(S.nu, kRB) * round_up(S.nu, kRB) * d.NP;  // X in blocks
       h.xsize = xs;
       h.cost = (double)h.njobs * nu2 * d.NP * d.KP;
       // X, then the reduction partials; rounded to 256 B so every X buffer of

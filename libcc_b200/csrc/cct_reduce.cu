@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t N
     double *xp = xpart + (int64_t)u * ncta + c, *vp = vpart + u * vsize;
     auto block = [&](auto kind) {
       constexpr int KIND = decltype(kind)::value;
-      if constexpr (FILL != kBulk) fill_rows<KIND, FILL>(nu, no, NP, t, vb, S0, S1, S2, m.Xs, m.Vs);
+      if constexpr (FILL != kBulk) fill_rows<KIND>(nu, no, NP, t, vb, S0, S1, S2, m.Xs, m.Vs);
       reduce_compute<KIND>(nu, t, eh, ep, S0, S1, S2, xp, vp, m, next);
     };
     if (t.kind == kIJK)

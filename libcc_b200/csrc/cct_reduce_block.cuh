@@ -55,9 +55,8 @@ constexpr int REDUCE_SMEM = (kXBlocks * SL + 3 * VPAIR + kPartDoubles + 1) * 8;
 
 // Where the X blocks come from: kBulk, 8 x 8 x 8 blocks (xblock_base), each one
 // contiguous 4 KB bulk copy; kRows, rows of NP (a forward that keeps W for the
-// backward, the backward itself); kRowsCoherent, rows written by other CTAs of
-// the same persistent kernel, so read through L2.
-enum Fill { kBulk, kRows, kRowsCoherent };
+// backward, the backward itself).
+enum Fill { kBulk, kRows };
 
 __device__ __forceinline__ int nb_of(int nu) { return (nu + RB - 1) / RB; }
 
@@ -198,8 +197,8 @@ __device__ __forceinline__ bool copies_landed(const Smem &m, uint32_t parity, in
   return false;
 }
 
-// kRows, kRowsCoherent: X and V by the threads; block barriers before and after.
-template <int KIND, Fill FILL>
+// kRows: X and V by the threads; block barriers before and after.
+template <int KIND>
 __device__ __forceinline__ void fill_rows(int nu, int no, int64_t NP, const TupleDev &t,
                                           const double *__restrict__ vb, int S0, int S1, int S2, double *Xs,
                                           double *Vs) {
@@ -222,8 +221,7 @@ __device__ __forceinline__ void fill_rows(int nu, int no, int64_t NP, const Tupl
         const int xp = RB * O0 + (idx >> 6), xq = RB * O1 + ((idx >> 3) & 7), xs = RB * O2 + (idx & 7);
         double v = 0.0;
         if (xp < nu && xq < nu && xs < nu) {
-          const double *src = X + ((int64_t)xp * nu + xq) * NP + xs;
-          v = FILL == kRowsCoherent ? __ldcg(src) : __ldg(src);
+          v = __ldg(X + ((int64_t)xp * nu + xq) * NP + xs);
         }
         Xs[(6 * g + q) * SL + idx] = v;
       }
