@@ -191,16 +191,21 @@ double *xbuf(const ccT_plan *p, int64_t t, int g) {
   return p->X + (t % ((int64_t)p->group * p->nring) * 3 + g) * p->xsize;
 }
 
-// Tuples per group.  A launch of a small system's tuple leaves most SMs idle:
-// group until a launch has about kGroupTiles W-build tiles (eight waves of
-// three FP64 CTAs, or 24 tiles of an emulated CTA, on 148 SMs; four FP64 waves
-// took 32.2 ms where eight take 31.2, at no12-nu120), within kMaxGroup tuples and kGroupBytes of X per group; a
-// tuple that has the tiles by itself stays alone (nu >= ~200, where one launch
-// a tuple and groups time the same).  A forward with one tuple a launch
-// against groups: no4-nu36 (16 tuples a group) 302 -> 109 us, no9-nu83
-// emulated (11) 6.11 -> 3.12 ms, no12-nu120 (4) 36.6 -> 34.7 ms.
-constexpr int64_t kGroupTiles = 3552;
-constexpr int64_t kGroupBytes = (int64_t)256 << 20;
+// Tuples per group.  A launch of a small system's tuple leaves most SMs idle, and
+// every launch ends in a wave that is partly empty and hands the SMs from the W
+// build to the reduction: group until a launch has about kGroupTiles W-build tiles
+// (64 waves of three FP64 CTAs, or 192 tiles of an emulated CTA, on 148 SMs) within
+// kMaxGroup tuples and kGroupBytes of X.  A forward with one tuple a launch
+// against groups of an eighth of the tiles and 256 MB, and these: no4-nu36 302 ->
+// 109 us (one group either way), no12-nu120 36.6 -> 34.7 ms then and 28.4 -> 27.0
+// now, no9-nu83 emulated 6.11 -> 3.12 then and 2.35 -> 2.11 now (3 digits 1.68 ->
+// 1.44), 3-digit no12-nu130 15.3 -> 14.2, no12-nu200 54.8 -> 50.3, no8-nu320
+// (two tuples a group) 63.8 -> 63.1 ms.  Twice the bytes gave at most 1% more.
+constexpr int64_t kGroupTiles = 28416;
+constexpr int64_t kGroupBytes = (int64_t)1536 << 20;
+// Groups of more X than this keep a ring of two instead of kNBuf (the same times
+// at no9-nu83 and up; a third less memory to allocate).
+constexpr int64_t kRing2Bytes = (int64_t)256 << 20;
 int choose_group(int64_t tiles_per_tuple, int64_t xbytes_per_tuple, int64_t ntuples) {
   int64_t g = (kGroupTiles + tiles_per_tuple - 1) / tiles_per_tuple;
   g = std::min(g, std::max<int64_t>(1, kGroupBytes / xbytes_per_tuple));
@@ -800,60 +805,71 @@ int cct::plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *
   if (cudaEventCreate(&p->ev0) != cudaSuccess || cudaEventCreate(&p->ev1) != cudaSuccess) return fail(CCT_ERR_CUDA);
   const int64_t nu2 = nu * nu, ntup = (int64_t)p->tuples.size();
   p->xsize = round_up(nu, kRB) * round_up(nu, kRB) * d.NP;  // blocked; rows of NP fit
+  auto set_ring = [&] {
+    const int64_t most = p->group > 1 && p->group * 3 * p->xsize * 8 > kRing2Bytes ? 2 : kNBuf;
+    p->nring = (int)std::min<int64_t>(most, (ntup + p->group - 1) / p->group);
+  };
   {
     const int64_t bm = p->emulated ? kEmuBM : 128, bn = p->emulated ? d.EBN : d.BN;
     // packed plans: a group could need more slabs than the cache holds
     p->group = p->packed ? 1
                          : choose_group(3 * ((nu2 + bm - 1) / bm) * (d.NP / bn), 3 * p->xsize * 8, ntup);
     p->group = std::min(p->group, group_cap);
-    p->nring = (int)std::min<int64_t>(kNBuf, (ntup + p->group - 1) / p->group);
+    set_ring();
   }
-  Arena mem;
-  mem.add(&p->eh, no);
-  mem.add(&p->ep, nu);
-  mem.add(&p->t1, no * nu);
-  mem.add(&p->t2, nu2 * no * no);
-  mem.add(&p->vm, no * nu * no * no);
-  mem.add(&p->voe, nu2 * no * no);
-  mem.add(&p->vb, vb_size(d));
-  if (p->packed) {
-    mem.add(&p->vvvo_res, nu * (nu + 1) / 2 * nu * no);
-    mem.add(&p->slabs, kSlabs * nu2 * d.KP);
-  } else {
-    mem.add(&p->E, no * nu2 * d.KP);
+  for (;;) {  // smaller groups where the device has no room for the ring
+    Arena mem;
+    mem.add(&p->eh, no);
+    mem.add(&p->ep, nu);
+    mem.add(&p->t1, no * nu);
+    mem.add(&p->t2, nu2 * no * no);
+    mem.add(&p->vm, no * nu * no * no);
+    mem.add(&p->voe, nu2 * no * no);
+    mem.add(&p->vb, vb_size(d));
+    if (p->packed) {
+      mem.add(&p->vvvo_res, nu * (nu + 1) / 2 * nu * no);
+      mem.add(&p->slabs, kSlabs * nu2 * d.KP);
+    } else {
+      mem.add(&p->E, no * nu2 * d.KP);
+    }
+    mem.add(&p->F, no * no * d.NP * d.KP);
+    mem.add(&p->X, (int64_t)p->group * p->nring * 3 * p->xsize);
+    mem.add(&p->xpart, p->group * d.ncta);
+    mem.add(&p->vpart, p->group * vpart_size(d));
+    mem.add(&p->tsum, p->group * tsum_size(d));
+    mem.add(&p->cta_table, d.ncta * 3);
+    mem.add(&p->acc, 5 + nu * no + 2 + kEmuMaxSlices + 1);
+    mem.add(&p->jobs, job_offset(p, ntup));
+    if (p->emulated) {
+      EmuOperands &e = p->emu;
+      e.slices = o.emu_slices ? o.emu_slices : kEmuMaxSlices;
+      e.run_slices = e.slices;         // an automatic plan lowers it at calibration
+      e.ebn = d.EBN;
+      e.NPe = d.NP;
+      e.adaptive = o.emu_slices == 0;  // automatic: the calibrated count is the maximum, each tile takes what it needs
+      p->emu_auto = o.emu_slices == 0;
+      p->emu_base_ebn = d.EBN;
+      e.KP8 = round_up(nu + no, kEmuKC);
+      e.tiles_m = (nu2 + kEmuBM - 1) / kEmuBM;
+      const int64_t rowsE = no * nu2, rowsF = no * no * d.NP;
+      const int64_t bytesE = e.slices * no * e.tiles_m * kEmuBM * e.KP8;  // row tiles padded to 128 rows
+      mem.add(&e.E8, bytesE);
+      mem.add(&e.E8T, bytesE);
+      mem.add(&e.F8, e.slices * rowsF * e.KP8);
+      mem.add(&e.expE, rowsE);
+      mem.add(&e.expET, rowsE);
+      mem.add(&e.expF, rowsF);
+      mem.add(&e.expRowF, rowsF);
+      mem.add(&p->emu_jobs, job_offset(p, ntup));
+      mem.add(&e.tileExp, e.tiles_m + no * (d.NP / d.EBN) + 2);
+    }
+    s = mem.allocate(&p->arena);
+    if (s == CCT_OK) break;
+    if (s != CCT_ERR_NOMEM || p->group == 1) return fail(s);
+    cudaGetLastError();
+    p->group = (p->group + 1) / 2;
+    set_ring();
   }
-  mem.add(&p->F, no * no * d.NP * d.KP);
-  mem.add(&p->X, (int64_t)p->group * p->nring * 3 * p->xsize);
-  mem.add(&p->xpart, p->group * d.ncta);
-  mem.add(&p->vpart, p->group * vpart_size(d));
-  mem.add(&p->tsum, p->group * tsum_size(d));
-  mem.add(&p->cta_table, d.ncta * 3);
-  mem.add(&p->acc, 5 + nu * no + 2 + kEmuMaxSlices + 1);
-  mem.add(&p->jobs, job_offset(p, ntup));
-  if (p->emulated) {
-    EmuOperands &e = p->emu;
-    e.slices = o.emu_slices ? o.emu_slices : kEmuMaxSlices;
-    e.run_slices = e.slices;         // an automatic plan lowers it at calibration
-    e.ebn = d.EBN;
-    e.NPe = d.NP;
-    e.adaptive = o.emu_slices == 0;  // automatic: the calibrated count is the maximum, each tile takes what it needs
-    p->emu_auto = o.emu_slices == 0;
-    p->emu_base_ebn = d.EBN;
-    e.KP8 = round_up(nu + no, kEmuKC);
-    e.tiles_m = (nu2 + kEmuBM - 1) / kEmuBM;
-    const int64_t rowsE = no * nu2, rowsF = no * no * d.NP;
-    const int64_t bytesE = e.slices * no * e.tiles_m * kEmuBM * e.KP8;  // row tiles padded to 128 rows
-    mem.add(&e.E8, bytesE);
-    mem.add(&e.E8T, bytesE);
-    mem.add(&e.F8, e.slices * rowsF * e.KP8);
-    mem.add(&e.expE, rowsE);
-    mem.add(&e.expET, rowsE);
-    mem.add(&e.expF, rowsF);
-    mem.add(&e.expRowF, rowsF);
-    mem.add(&p->emu_jobs, job_offset(p, ntup));
-    mem.add(&e.tileExp, e.tiles_m + no * (d.NP / d.EBN) + 2);
-  }
-  if ((s = mem.allocate(&p->arena))) return fail(s);
   p->flags = reinterpret_cast<int *>(p->acc + 5 + nu * no);
   if (p->emulated) p->emu.slice_hist = reinterpret_cast<unsigned long long *>(p->acc + 5 + nu * no + 2);
   std::vector<int16_t> table(d.ncta * 3);
