@@ -536,10 +536,16 @@ int ensure_emu_plans(ccT_batch *b) {
     o.precision = CCT_PREC_INT8_EMU;
     o.device = b->device;
     o.vvvo_mode = CCT_VVVO_EXPANDED;
-    CCT_TRY(plan_create(&b->emu_plans[s], S.no, S.nu, &o, 1));  // it runs single tuples: one X set a group
-    CCT_TRY(ccT_set_inputs(b->emu_plans[s], S.eh, S.ep, S.t1, S.t2, S.vm, S.voe, S.vvvo, CCT_MEM_DEVICE));
+    ccT_plan *p = nullptr;
+    CCT_TRY(plan_create(&p, S.no, S.nu, &o, 1));  // it runs single tuples: one X set a group
     double ets = 0.0, etd = 0.0;
-    CCT_TRY(ccT_forward(b->emu_plans[s], 0, 1, &ets, &etd, nullptr));
+    int st = ccT_set_inputs(p, S.eh, S.ep, S.t1, S.t2, S.vm, S.voe, S.vvvo, CCT_MEM_DEVICE);
+    if (st == CCT_OK) st = ccT_forward(p, 0, 1, &ets, &etd, nullptr);
+    if (st != CCT_OK) {  // rejected inputs: its digit operands are not built, so no schedule may name it
+      ccT_plan_destroy(p);
+      return st;
+    }
+    b->emu_plans[s] = p;
   }
   return CCT_OK;
 }
