@@ -221,6 +221,14 @@ int ccT_batch_tune(ccT_batch *batch, int32_t *best_mode, int32_t *best_bn, int32
  * counterpart (the reference's only failure handling is stop,
  * program.F90:221-222). */
 int ccT_batch_debug_stall(ccT_batch *batch, int64_t tuple, int64_t spin_limit);
+/* Testing hooks: a reduction block polls at most `polls` times (negative: the
+ * default limit) for the bulk copies of its inputs.  With 0 every wait runs
+ * out: the block waits once more, with the default limit, for its copies to
+ * land, leaves without its sums, and the forward returns CCT_ERR_TIMEOUT with
+ * the context intact.  A NULL plan is the one of ijk_gpu_init_
+ * (CCT_ERR_STATE where there is none).  No reference counterpart. */
+int ccT_debug_wait_limit(ccT_plan *plan, int64_t polls);
+int ccT_batch_debug_wait_limit(ccT_batch *batch, int64_t polls);
 /* Device milliseconds of the last batch forward (CUDA events around the graph). */
 double ccT_batch_last_ms(const ccT_batch *batch);
 /* Work items (W-build tiles + reduction blocks) in the current schedule. */

@@ -119,6 +119,7 @@ struct BatchArgs {
   double *sys_out;               // [sys][3] = ets, etd, ets+etd
   int *err;
   long spin_limit;               // iterations of a bounded counter wait
+  int copy_limit;                // ... and of a reduction block's wait for its copies
 };
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
       asm volatile("fence.proxy.async;" ::: "memory");
       __syncthreads();
       red::start_copies(S.nu, S.no, S.NP, td, S.vb, S0, S1, S2, m);
-      const bool landed = red::copies_landed(m, round, A.err);
+      const bool landed = red::copies_landed(m, round, A.err, A.copy_limit);
       if (landed) {
         auto block = [&](auto kind) {
           constexpr int KIND = decltype(kind)::value;
@@ -368,7 +369,10 @@ __global__ void __launch_bounds__(kBT, 2) batch_rd_kernel(const BatchArgs A, int
     int4 it2 = it1;
     if (more) load_desc(round ^ 1, it1.y);
     if (i + 2 * (int)gridDim.x < count) it2 = A.items[item0 + i + 2 * gridDim.x];
-    if (!red::copies_landed(m, round, A.err)) return;
+    if (!red::copies_landed(m, round, A.err, A.copy_limit)) {
+      wb::cp_async_wait<0>();  // the next record, in flight
+      return;
+    }
     const RdTuple &T = desc[round];
     auto next = [&]() {
       if (!more) return;
@@ -464,6 +468,7 @@ struct ccT_batch {
   // (position in queue order) wait for one W-build tile more than it has
   int64_t stall_tuple = -1;
   long spin_limit = kSpinLimit;
+  int copy_limit = kReduceWaitLimit;  // testing hook (ccT_batch_debug_wait_limit)
   bool tuned = false;
   // schedule (device)
   bool scheduled = false;
@@ -882,6 +887,7 @@ BatchArgs batch_args(ccT_batch *b) {
   a.sys_out = b->sys_out;
   a.err = b->err;
   a.spin_limit = b->spin_limit;
+  a.copy_limit = b->copy_limit;
   return a;
 }
 
@@ -1307,6 +1313,16 @@ int ccT_batch_debug_stall(ccT_batch *b, int64_t tuple, int64_t spin_limit) {
   }
   b->stall_tuple = tuple < 0 ? -1 : tuple;
   b->spin_limit = spin_limit > 0 ? (long)spin_limit : kSpinLimit;
+  free_schedule(b);  // the next forward rebuilds the schedule and its graph
+  return CCT_OK;
+}
+
+int ccT_batch_debug_wait_limit(ccT_batch *b, int64_t polls) {
+  if (!b) {
+    set_error("batch is NULL");
+    return CCT_ERR_INVALID;
+  }
+  b->copy_limit = polls < 0 ? kReduceWaitLimit : (int)std::min<int64_t>(polls, kReduceWaitLimit);
   free_schedule(b);  // the next forward rebuilds the schedule and its graph
   return CCT_OK;
 }

@@ -122,6 +122,8 @@ struct TupleDev {
 // The tuples of one reduction launch, passed by value (the constant bank):
 // at most kMaxGroup consecutive tuples of the list.
 constexpr int kMaxGroup = 32;
+// Polls of a reduction CTA's wait for its bulk copies (some seconds).
+constexpr int kReduceWaitLimit = 1 << 22;
 struct TupleGroup {
   int n = 0;
   TupleDev t[kMaxGroup];
@@ -239,7 +241,8 @@ int launch_wbuild_f64(const Dims &d, const GemmJob *jobs_dev, int njobs, cudaStr
 inline int64_t vpart_size(const Dims &d) { return (int64_t)12 * d.nb * d.nb * (d.nb + 1); }
 inline int64_t tsum_size(const Dims &d) { return 1 + 3 * (int64_t)d.nu; }
 int launch_reduce(const Dims &d, const TupleGroup &g, bool blocked, const double *eh, const double *ep,
-                  const double *vb, const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s);
+                  const double *vb, const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s,
+                  int wait_limit = kReduceWaitLimit);
 // 2 VOE(a,b,y,z) - VOE(a,b,z,y) in 8 x 8 tiles, [y][z][nb][nb][64], entry
 // (8 A + u, 8 B + v) of tile (A, B) at u + 8 v; zero past nu.
 inline int64_t vb_size(const Dims &d) { return (int64_t)d.no * d.no * d.nb * d.nb * 64; }

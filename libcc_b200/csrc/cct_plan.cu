@@ -61,6 +61,7 @@ struct ccT_plan {
   cudaEvent_t ev_gemm[kNBuf] = {}, ev_red[kNBuf] = {};
   int group = 1;                      // tuples per group (choose_group)
   int nring = 1;                      // groups in the X ring (<= kNBuf)
+  int wait_limit = kReduceWaitLimit;  // testing hook (ccT_debug_wait_limit)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // inputs (device copies, reference layouts)
   double *eh = nullptr, *ep = nullptr, *t1 = nullptr, *t2 = nullptr, *vm = nullptr, *voe = nullptr;
@@ -500,7 +501,8 @@ int run_group(ccT_plan *p, int64_t t0, int64_t t1, bool fp64 = false, int64_t ke
   }
   CCT_TRY(prof_mark(p, CCT_KERNEL_REDUCE, rs));
   if (rs != p->red_stream && !alone) CCT_CUDA(cudaStreamWaitEvent(rs, p->ev_sum, 0));  // the partials of the group before are summed
-  CCT_TRY(launch_reduce(p->d, g, keep < 0, p->eh, p->ep, p->vb, p->cta_table, p->xpart, p->vpart, p->flags + 1, rs));
+  CCT_TRY(launch_reduce(p->d, g, keep < 0, p->eh, p->ep, p->vb, p->cta_table, p->xpart, p->vpart, p->flags + 1, rs,
+                        p->wait_limit));
   CCT_CUDA(cudaEventRecord(p->ev_red[slot], rs));
   cudaStream_t fs = p->profiling || alone ? rs : p->red_stream;
   if (rs != fs) CCT_CUDA(cudaStreamWaitEvent(fs, p->ev_red[slot], 0));
@@ -1421,6 +1423,17 @@ double ccT_measure_int8_peak(int32_t device) { return measure_int8_peak(device);
 static ccT_plan *g_hook = nullptr;
 static double *g_hook_v1 = nullptr;
 static std::mutex g_hook_mutex;
+
+int ccT_debug_wait_limit(ccT_plan *p, int64_t polls) {
+  std::lock_guard<std::mutex> lock(g_hook_mutex);
+  if (!p) p = g_hook;
+  if (!p) {
+    set_error("no plan, and no ijk_gpu_init before");
+    return CCT_ERR_STATE;
+  }
+  p->wait_limit = polls < 0 ? kReduceWaitLimit : (int)std::min<int64_t>(polls, kReduceWaitLimit);
+  return CCT_OK;
+}
 
 void ijk_gpu_init_(const int64_t *no, const int64_t *nu, const double *eh, const double *ep, double *v1,
                    const double *t2, const double *vm, const double *voe) {

@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t N
                                                       const double *__restrict__ eh, const double *__restrict__ ep,
                                                       const double *__restrict__ vb,
                                                       const int16_t *__restrict__ table, double *__restrict__ xpart,
-                                                      double *__restrict__ vpart, int *err) {
+                                                      double *__restrict__ vpart, int *err, int wait_limit) {
   extern __shared__ __align__(16) double dyn_smem[];
   const Smem m(dyn_smem);
   int u = blockIdx.x / ncta, c = blockIdx.x - u * ncta;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t N
       T1 = table[3 * c1 + 1];
       T2 = table[3 * c1 + 2];
     }
-    if (FILL == kBulk && !copies_landed(m, round, err)) return;
+    if (FILL == kBulk && !copies_landed(m, round, err, wait_limit)) return;
     auto next = [&]() {
       if (FILL == kBulk && more) {
         __syncthreads();
@@ -248,7 +248,8 @@ int launch_build_vb(const Dims &d, const double *voe, double *vb, cudaStream_t s
 
 template <Fill FILL>
 int launch_reduce_fill(const Dims &d, const TupleGroup &g, const double *eh, const double *ep, const double *vb,
-                       const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s) {
+                       const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s,
+                       int wait_limit) {
   constexpr int smem = REDUCE_SMEM;
   static int configured_device = -1;
   int dev = 0;
@@ -265,21 +266,22 @@ int launch_reduce_fill(const Dims &d, const TupleGroup &g, const double *eh, con
   // forward, 80 with every CTA taking two)
   const int64_t total = d.ncta * g.n, blocks = total <= 4 * nsm ? total : 2 * nsm;
   reduce_kernel<FILL><<<(unsigned)blocks, RT, smem, s>>>(d.nu, d.no, d.NP, (int)d.ncta, vpart_size(d), g, eh, ep, vb,
-                                                         cta_table, xpart, vpart, err);
+                                                         cta_table, xpart, vpart, err, wait_limit);
   CCT_CUDA(cudaGetLastError());
   return CCT_OK;
 }
 
 int launch_reduce(const Dims &d, const TupleGroup &g, bool blocked, const double *eh, const double *ep,
-                  const double *vb, const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s) {
+                  const double *vb, const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s,
+                  int wait_limit) {
   if (blocked) {
     if (d.NP % RB) {
       set_error("blocked X needs NP a multiple of 8 (NP = " + std::to_string(d.NP) + ")");
       return CCT_ERR_INVALID;
     }
-    return launch_reduce_fill<kBulk>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s);
+    return launch_reduce_fill<kBulk>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s, wait_limit);
   }
-  return launch_reduce_fill<kRows>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s);
+  return launch_reduce_fill<kRows>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s, wait_limit);
 }
 
 int launch_finalize(const Dims &d, const TupleGroup &g, const double *xpart, const double *vpart, double *tsum,

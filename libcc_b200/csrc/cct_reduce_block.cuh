@@ -99,9 +99,8 @@ __device__ __forceinline__ int64_t voe_tile(int c, int no, int nb, const TupleDe
   return ((((int64_t)(pl & 1 ? z : y) * no + (pl & 1 ? y : z)) * nb + B1) * nb + B2) * VTILE;
 }
 
-constexpr int kReduceWaitLimit = 1 << 22;
-__device__ __forceinline__ bool wait_landed(uint32_t bar, uint32_t parity, int *err) {
-  for (int it = 0; it < kReduceWaitLimit; it++) {
+__device__ __forceinline__ bool wait_landed(uint32_t bar, uint32_t parity, int *err, int limit) {
+  for (int it = 0; it < limit; it++) {
     uint32_t ok;
     asm volatile(
         "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
@@ -187,13 +186,13 @@ __device__ __forceinline__ void start_copies(int nu, int no, int64_t NP, const T
   }
 }
 // kBulk: waits for the copies of the parity's round.  False (for the whole CTA)
-// when the bounded wait ran out: the error word is set, the copies have had a
-// second limit to land, and the CTA must return.
-__device__ __forceinline__ bool copies_landed(const Smem &m, uint32_t parity, int *err) {
+// when `limit` polls ran out: the error word is set, the copies have had the
+// full limit to land, and the CTA must return.
+__device__ __forceinline__ bool copies_landed(const Smem &m, uint32_t parity, int *err, int limit) {
   const uint32_t sbar = (uint32_t)__cvta_generic_to_shared(m.bar);
-  const bool ok = wait_landed(sbar, parity, err);
+  const bool ok = wait_landed(sbar, parity, err, limit);
   if (__syncthreads_and(ok)) return true;
-  wait_landed(sbar, parity, err);
+  wait_landed(sbar, parity, err, kReduceWaitLimit);
   return false;
 }
 
