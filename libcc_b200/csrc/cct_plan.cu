@@ -1462,7 +1462,7 @@ void ijk_gpu_init_(const int64_t *no, const int64_t *nu, const double *eh, const
   if ((s = launch_build_f(p->d, p->t2, p->vm, p->F, p->stream))) legacy_stop("ijk_gpu_init", s);
   if ((s = launch_build_vb(p->d, p->voe, p->vb, p->stream))) legacy_stop("ijk_gpu_init", s);
   if ((s = dalloc(&p->stage, n_u * (n_u + 1) / 2 * n_u))) legacy_stop("ijk_gpu_init", s);
-  if (cudaMemsetAsync(p->acc, 0, (5 + n_u * n_o) * 8, p->stream) != cudaSuccess) legacy_stop("ijk_gpu_init", CCT_ERR_CUDA);
+  if ((s = clear_results(p))) legacy_stop("ijk_gpu_init", s);
   p->host_eh.assign(eh, eh + n_o);
   p->host_ep.assign(ep, ep + n_u);
   std::fill(p->e_built.begin(), p->e_built.end(), 0);
@@ -1515,11 +1515,17 @@ void ijk_gpu_finalize_(const int64_t *no, const int64_t *nu, double *etd) {
   const int64_t n = (int64_t)p->d.nu * p->d.no;
   std::vector<double> v1(n);
   double e[2];
+  int hflags[4];
   if (join_streams(p) != CCT_OK ||
       cudaMemcpyAsync(e, p->acc, 16, cudaMemcpyDeviceToHost, p->stream) != cudaSuccess ||
       cudaMemcpyAsync(v1.data(), v1_acc(p), n * 8, cudaMemcpyDeviceToHost, p->stream) != cudaSuccess ||
+      cudaMemcpyAsync(hflags, p->flags, 16, cudaMemcpyDeviceToHost, p->stream) != cudaSuccess ||
       cudaStreamSynchronize(p->stream) != cudaSuccess)
     legacy_stop("ijk_gpu_finalize", CCT_ERR_CUDA);
+  if (hflags[1]) {
+    set_error("a kernel ran out its bounded wait and unwound");
+    legacy_stop("ijk_gpu_finalize", CCT_ERR_TIMEOUT);
+  }
   *etd += e[0] + e[1];
   for (int64_t q = 0; q < n; q++) g_hook_v1[q] += v1[q];
   ccT_plan_destroy(p);
