@@ -302,9 +302,16 @@ struct ItemDigits {
   }
 };
 
-__device__ __forceinline__ double pow2(int e) {
-  // exact 2^e for normal exponents; ldexp covers the subnormal range
-  return (e >= -1022 && e <= 1023) ? __longlong_as_double((long long)(e + 1023) << 52) : ldexp(1.0, e);
+// 2^e for -1022 <= e <= 1023
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+// v 2^e with one rounding, for integers |v| < 2^63 and any e, in two normal
+// factors.  One factor would be zero, or subnormal, for products that are not: a
+// 7-digit sum carries 2^54 of its product's size, so 2^e is out of range
+// from products of 2^-1020 down.  (The clamps only meet a result that is zero or
+// infinite either way.)
+__device__ __forceinline__ double scaled(double v, int e) {
+  const int h = max(-1022, min(1023, e >> 1)), r = max(-1022, min(1023, e - h));
+  return v * pow2(h) * pow2(r);
 }
 
 // NAR: the last column tile is narrow (nl < EBN).
@@ -747,16 +754,16 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
         for (int j = 0; j < CW; j += 4) {
           double x[4];
 #pragma unroll
-          for (int u = 0; u < 4; u++) x[u] = value(j + u) * scale(__shfl_sync(0xffffffffu, eBl, j + u));
+          for (int u = 0; u < 4; u++) x[u] = scale(value(j + u), __shfl_sync(0xffffffffu, eBl, j + u));
           const int sc = n0 + j;
           if (live && sc < send)
             st_global_v4(xrow + (args.xblocked ? (sc >> 3) * 512 + (sc & 7) : sc), x[0], x[1], x[2], x[3]);
         }
       };
       if (normal)
-        store([&](int e) { return __hiloint2double((e0 + 1023 + e) << 20, 0); });
+        store([&](double v, int e) { return v * pow2(e0 + e); });
       else
-        store([&](int e) { return pow2(e0 + e); });
+        store([&](double v, int e) { return scaled(v, e0 + e); });
       } else {
         asm volatile("tcgen05.fence::before_thread_sync;");
         __syncwarp();
