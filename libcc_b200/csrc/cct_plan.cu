@@ -106,7 +106,8 @@ struct ccT_plan {
   cudaEvent_t ev_bwdf[2] = {};
   // backward, per GX set: pointwise pass done / dE GEMM done / dF GEMM done reading it
   cudaEvent_t ev_gx_pw[kGXSets] = {}, ev_gx_e[kGXSets] = {}, ev_gx_f[kGXSets] = {};
-  cudaEvent_t ev_rec[kNBuf] = {}, ev_pw[kNBuf] = {};  // per X ring group: W rebuilt / read by the pointwise pass
+  cudaEvent_t ev_rec[kNBuf] = {};  // W of tuple t rebuilt (t mod kNBuf)
+  cudaEvent_t ev_pw[kNBuf] = {};   // per X ring group: read by the pointwise passes
   int64_t fwd_begin = -1, fwd_end = -1;
   float last_bwd_ms = 0.f;
   // options.keep_w: the W-build output of the last forward, kept for the
@@ -1118,15 +1119,14 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
   CCT_TRY(adj_zero(d, &p->adj, p->stream));
   // dT1 = 2 v1: an emulated plan's v1 is rebuilt from the FP64 W of this pass
   if (p->emulated) CCT_CUDA(cudaMemsetAsync(p->adj.v1, 0, (5 + (size_t)d.nu * d.no) * 8, p->stream));
-  // Four streams.  rec_stream rebuilds W one X ring group of tuples per launch,
-  // ahead of red_stream, which runs the pointwise adjoint kernels of tuple t
-  // (dE/dW, dVOE, deps and dE/dX into GX set t mod 4); bwd_stream then runs
-  // the dF GEMM of tuple t, and gemm_stream one dE GEMM for each pair of
-  // consecutive tuples (twice the K per output slab, one read-modify-write of
-  // dE per pair).  So the latency-bound pointwise chain overlaps the GEMMs of
-  // earlier tuples and the recompute of later ones.  Every accumulator is
-  // written by one stream only, in tuple order, so the results stay bitwise
-  // reproducible.
+  // Four streams.  rec_stream rebuilds W, ahead of red_stream, which runs the
+  // pointwise adjoint kernels of tuple t (dE/dW, dVOE, deps and dE/dX into GX
+  // set t mod 4); bwd_stream then runs the dF GEMM of tuple t, and gemm_stream
+  // one dE GEMM for each pair of consecutive tuples (twice the K per output
+  // slab, one read-modify-write of dE per pair).  So the latency-bound pointwise
+  // chain overlaps the GEMMs of earlier tuples and the recompute of later ones.
+  // Every accumulator is written by one stream only, in tuple order, so the
+  // results stay bitwise reproducible.
   CCT_TRY(fork_streams(p));
   cudaStream_t sW = p->rec_stream, sP = p->pw_stream ? p->pw_stream : p->red_stream, sG = p->gemm_stream,
                sF = p->bwd_stream;
@@ -1135,22 +1135,31 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
   if (sP != p->red_stream) CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_fork, 0));
   // W kept by the forward (options.keep_w): no recompute, X read from there
   const bool kept = p->keep_begin == begin && p->keep_end == end;
+  // W of tuple t + 1 is issued before the pointwise passes of tuple t.  One tuple
+  // a launch: the first pass waits for one tuple's W build alone, and no
+  // launch fills every SM ahead of the passes and GEMMs it is to run beside.  With
+  // a ring group per launch no10-nu96 took 32.3 ms, 30.3 so; no12-nu120 emulated
+  // 124 and 117.
+  auto rebuild = [&](int64_t t) -> int {
+    const int64_t grp = t / p->group;
+    // X buffers last read by the pointwise passes of nring groups before, all
+    // issued already (with nring >= 2 that group ends before tuple t - 1)
+    if (t % p->group == 0 && grp - begin / p->group >= p->nring)
+      CCT_CUDA(cudaStreamWaitEvent(sW, p->ev_pw[grp % p->nring], 0));
+    CCT_TRY(wbuild_tuples(p, t, t + 1, true, sW, false));
+    CCT_CUDA(cudaEventRecord(p->ev_rec[t % kNBuf], sW));
+    return CCT_OK;
+  };
+  if (!kept && end > begin) CCT_TRY(rebuild(begin));
   for (int64_t t = begin; t < end; t++) {
     const Tuple &tu = p->tuples[t];
     const int set = (int)((t - begin) % kGXSets);
-    const int64_t grp = t / p->group, grp_end = std::min(end, (grp + 1) * p->group);
-    const int xb = (int)(grp % p->nring);
     double *Xk[3] = {nullptr, nullptr, nullptr};
     if (kept) {
       for (int g = 0; g < 3; g++) Xk[g] = xkeep_at(p, t - begin, g);
     } else {
-      if (t == begin || t % p->group == 0) {  // the group's first tuple
-        // X buffers last read by the pointwise passes of nring groups before
-        if (grp - begin / p->group >= p->nring) CCT_CUDA(cudaStreamWaitEvent(sW, p->ev_pw[xb], 0));
-        CCT_TRY(wbuild_tuples(p, t, grp_end, true, sW, false));
-        CCT_CUDA(cudaEventRecord(p->ev_rec[xb], sW));
-        CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_rec[xb], 0));
-      }
+      if (t + 1 < end) CCT_TRY(rebuild(t + 1));
+      CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_rec[t % kNBuf], 0));
       for (int g = 0; g < 3; g++) Xk[g] = xbuf(p, t, g);
     }
     if (t - begin >= kGXSets) {  // GX set last read by the GEMMs of tuple t - kGXSets
@@ -1165,7 +1174,7 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
       CCT_TRY(launch_reduce(d, g, false, p->eh, p->ep, p->vb, p->cta_table, p->xpart, p->vpart, p->flags + 1, sP));
       CCT_TRY(launch_finalize(d, g, p->xpart, p->vpart, p->tsum, p->adj.v1, p->adj.v1 + 5, sP));
     }
-    if (t + 1 == grp_end) CCT_CUDA(cudaEventRecord(p->ev_pw[xb], sP));
+    if ((t + 1) % p->group == 0) CCT_CUDA(cudaEventRecord(p->ev_pw[t / p->group % p->nring], sP));
     CCT_CUDA(cudaEventRecord(p->ev_gx_pw[set], sP));
     CCT_CUDA(cudaStreamWaitEvent(sF, p->ev_gx_pw[set], 0));
     CCT_TRY(adj_tuple_gemm_f(d, tu, p->E, &p->adj, set, sF));
