@@ -1129,7 +1129,7 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
   // results stay bitwise reproducible.
   CCT_TRY(fork_streams(p));
   cudaStream_t sW = p->rec_stream, sP = p->pw_stream ? p->pw_stream : p->red_stream, sG = p->gemm_stream,
-               sF = p->bwd_stream;
+               sF = p->bwd_stream, sV = p->gemm_stream2;
   CCT_CUDA(cudaStreamWaitEvent(sF, p->ev_fork, 0));
   CCT_CUDA(cudaStreamWaitEvent(sW, p->ev_fork, 0));
   if (sP != p->red_stream) CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_fork, 0));
@@ -1140,14 +1140,32 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
   // launch fills every SM ahead of the passes and GEMMs it is to run beside.  With
   // a ring group per launch no10-nu96 took 32.3 ms, 30.3 so; no12-nu120 emulated
   // 124 and 117.
+  // An emulated plan's v1 is summed from these X by the forward's reduction, on
+  // gemm_stream2, beside the passes: in the passes' chain it made every tuple's
+  // chain longer (no8-nu72 11.9 ms, 9.9 so).  Tuples of one launch: as many as
+  // fill two CTAs per SM once (no4-nu36: eight, 1.05 -> 0.84 ms; every launch costs
+  // the host too).
+  TupleGroup v1g;
+  const int v1_tuples = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxGroup, 2 * 148 / d.ncta));
   auto rebuild = [&](int64_t t) -> int {
     const int64_t grp = t / p->group;
     // X buffers last read by the pointwise passes of nring groups before, all
     // issued already (with nring >= 2 that group ends before tuple t - 1)
+    const int slot = (int)(grp % p->nring);
     if (t % p->group == 0 && grp - begin / p->group >= p->nring)
-      CCT_CUDA(cudaStreamWaitEvent(sW, p->ev_pw[grp % p->nring], 0));
+      for (cudaEvent_t e : {p->ev_pw[slot], p->ev_red[slot]}) CCT_CUDA(cudaStreamWaitEvent(sW, e, 0));
     CCT_TRY(wbuild_tuples(p, t, t + 1, true, sW, false));
     CCT_CUDA(cudaEventRecord(p->ev_rec[t % kNBuf], sW));
+    if (!p->emulated) return CCT_OK;
+    double *const X[3] = {xbuf(p, t, 0), xbuf(p, t, 1), xbuf(p, t, 2)};
+    v1g.t[v1g.n++] = tuple_dev(p->tuples[t], X);
+    const bool last = (t + 1) % p->group == 0;
+    if (v1g.n < v1_tuples && !last && t + 1 < end) return CCT_OK;
+    CCT_CUDA(cudaStreamWaitEvent(sV, p->ev_rec[t % kNBuf], 0));
+    CCT_TRY(launch_reduce(d, v1g, false, p->eh, p->ep, p->vb, p->cta_table, p->xpart, p->vpart, p->flags + 1, sV));
+    CCT_TRY(launch_finalize(d, v1g, p->xpart, p->vpart, p->tsum, p->adj.v1, p->adj.v1 + 5, sV));
+    if (last) CCT_CUDA(cudaEventRecord(p->ev_red[slot], sV));
+    v1g.n = 0;
     return CCT_OK;
   };
   if (!kept && end > begin) CCT_TRY(rebuild(begin));
@@ -1167,13 +1185,6 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
       CCT_CUDA(cudaStreamWaitEvent(sP, p->ev_gx_f[set], 0));
     }
     CCT_TRY(adj_tuple_pointwise(d, tu, Xk, p->eh, p->ep, p->t1, p->voe, &p->adj, set, sP));
-    if (p->emulated) {
-      TupleGroup g;
-      g.n = 1;
-      g.t[0] = tuple_dev(tu, Xk);
-      CCT_TRY(launch_reduce(d, g, false, p->eh, p->ep, p->vb, p->cta_table, p->xpart, p->vpart, p->flags + 1, sP));
-      CCT_TRY(launch_finalize(d, g, p->xpart, p->vpart, p->tsum, p->adj.v1, p->adj.v1 + 5, sP));
-    }
     if ((t + 1) % p->group == 0) CCT_CUDA(cudaEventRecord(p->ev_pw[t / p->group % p->nring], sP));
     CCT_CUDA(cudaEventRecord(p->ev_gx_pw[set], sP));
     CCT_CUDA(cudaStreamWaitEvent(sF, p->ev_gx_pw[set], 0));
@@ -1193,6 +1204,10 @@ int ccT_backward(ccT_plan *p, int64_t begin, int64_t end, double *d_eh, double *
     }
   }
   // p->stream after every stream (red_stream already waited for rec_stream)
+  if (p->emulated) {
+    CCT_CUDA(cudaEventRecord(p->ev_sum, sV));
+    CCT_CUDA(cudaStreamWaitEvent(p->stream, p->ev_sum, 0));
+  }
   CCT_CUDA(cudaEventRecord(p->ev_join, sP));
   CCT_CUDA(cudaStreamWaitEvent(p->stream, p->ev_join, 0));
   CCT_CUDA(cudaEventRecord(p->ev_fork, sG));
