@@ -42,10 +42,14 @@ __global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t N
   int u = blockIdx.x / ncta, c = blockIdx.x - u * ncta;
   if (u >= grp.n) return;
   int S0 = table[3 * c], S1 = table[3 * c + 1], S2 = table[3 * c + 2];
-  if (FILL == kBulk) {
-    init_copies(m);
-    start_copies(nu, no, NP, grp.t[u], vb, S0, S1, S2, m);
-  }
+  auto start = [&](const TupleDev &t, int A, int B, int C) {
+    if (FILL == kBulk)
+      start_copies(nu, no, NP, t, vb, A, B, C, m);
+    else
+      start_rows(nu, no, NP, t, vb, A, B, C, m);
+  };
+  if (FILL == kBulk) init_copies(m);
+  start(grp.t[u], S0, S1, S2);
   for (uint32_t round = 0;; round ^= 1) {
     int u1 = u, c1 = c + gridDim.x;
     while (c1 >= ncta) {
@@ -59,18 +63,19 @@ __global__ void __launch_bounds__(RT, 2) reduce_kernel(int nu, int no, int64_t N
       T1 = table[3 * c1 + 1];
       T2 = table[3 * c1 + 2];
     }
-    if (FILL == kBulk && !copies_landed(m, round, err, wait_limit)) return;
+    if (FILL == kRows)
+      rows_landed();
+    else if (!copies_landed(m, round, err, wait_limit))
+      return;
     auto next = [&]() {
-      if (FILL == kBulk && more) {
-        __syncthreads();
-        start_copies(nu, no, NP, grp.t[u1], vb, T0, T1, T2, m);
-      }
+      if (!more) return;
+      __syncthreads();
+      start(grp.t[u1], T0, T1, T2);
     };
     const TupleDev &t = grp.t[u];
     double *xp = xpart + (int64_t)u * ncta + c, *vp = vpart + u * vsize;
     auto block = [&](auto kind) {
       constexpr int KIND = decltype(kind)::value;
-      if constexpr (FILL != kBulk) fill_rows<KIND>(nu, no, NP, t, vb, S0, S1, S2, m.Xs, m.Vs);
       reduce_compute<KIND>(nu, t, eh, ep, S0, S1, S2, xp, vp, m, next);
     };
     if (t.kind == kIJK)
@@ -274,13 +279,11 @@ int launch_reduce_fill(const Dims &d, const TupleGroup &g, const double *eh, con
 int launch_reduce(const Dims &d, const TupleGroup &g, bool blocked, const double *eh, const double *ep,
                   const double *vb, const int16_t *cta_table, double *xpart, double *vpart, int *err, cudaStream_t s,
                   int wait_limit) {
-  if (blocked) {
-    if (d.NP % RB) {
-      set_error("blocked X needs NP a multiple of 8 (NP = " + std::to_string(d.NP) + ")");
-      return CCT_ERR_INVALID;
-    }
-    return launch_reduce_fill<kBulk>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s, wait_limit);
+  if (d.NP % RB) {
+    set_error("the reduction needs NP a multiple of 8 (NP = " + std::to_string(d.NP) + ")");
+    return CCT_ERR_INVALID;
   }
+  if (blocked) return launch_reduce_fill<kBulk>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s, wait_limit);
   return launch_reduce_fill<kRows>(d, g, eh, ep, vb, cta_table, xpart, vpart, err, s, wait_limit);
 }
 

@@ -196,38 +196,39 @@ __device__ __forceinline__ bool copies_landed(const Smem &m, uint32_t parity, in
   return false;
 }
 
-// kRows: X and V by the threads; block barriers before and after.
-template <int KIND>
-__device__ __forceinline__ void fill_rows(int nu, int no, int64_t NP, const TupleDev &t,
-                                          const double *__restrict__ vb, int S0, int S1, int S2, double *Xs,
-                                          double *Vs) {
-  constexpr int NG = KIND == kIJK ? 3 : 2;  // GEMM outputs of the tuple
-  const int tid = threadIdx.x, nb = nb_of(nu);
-  auto Sm = [&](int m) { return sel3(m, S0, S1, S2); };
+// kRows: starts the copies of a block triple into X and V, 16 bytes a thread at a
+// time: a row (p,q) of an X block is 64 contiguous bytes (NP is a multiple of 8),
+// so an X block is one copy of every thread.  Rows of indices >= nu become zero.
+// The barriers as for start_copies; rows_landed waits.  With one plain load a thread
+// and element before each triple's arithmetic a kept-W forward took 33.2 ms at
+// no12-nu120 and 54.0 at no10-nu160, 28.0 and 47.4 so.
+__device__ __forceinline__ void start_rows(int nu, int no, int64_t NP, const TupleDev &t,
+                                           const double *__restrict__ vb, int S0, int S1, int S2, const Smem &m) {
+  static_assert(RT == 4 * RB * RB, "a thread per 16 bytes of an X block");
+  const int tid = threadIdx.x, nb = nb_of(nu), ng = t.kind == kIJK ? 3 : 2;
+  const int u0 = tid >> 5, u1 = (tid >> 2) & 7, off = 8 * (tid >> 2) + 2 * (tid & 3);
+  auto cp16 = [](double *dst, const double *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(ok ? 16 : 0)
+                 : "memory");
+  };
   int slot[6];
   orbit_slots(S0, S1, S2, slot);
-  __syncthreads();
 #pragma unroll
-  for (int g = 0; g < NG; g++) {
-    const double *X = t.x[g];
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-      if (slot[q] != q) continue;
-      const int O0 = Sm(pm(q, 0)), O1 = Sm(pm(q, 1)), O2 = Sm(pm(q, 2));
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int idx = tid + RT * e;
-        const int xp = RB * O0 + (idx >> 6), xq = RB * O1 + ((idx >> 3) & 7), xs = RB * O2 + (idx & 7);
-        double v = 0.0;
-        if (xp < nu && xq < nu && xs < nu) {
-          v = __ldg(X + ((int64_t)xp * nu + xq) * NP + xs);
-        }
-        Xs[(6 * g + q) * SL + idx] = v;
-      }
-    }
+  for (int q = 0; q < 6; q++) {
+    if (slot[q] != q) continue;
+    const int O0 = sel3(pm(q, 0), S0, S1, S2), O1 = sel3(pm(q, 1), S0, S1, S2), O2 = sel3(pm(q, 2), S0, S1, S2);
+    const int xp = RB * O0 + u0, xq = RB * O1 + u1;
+    const bool ok = xp < nu && xq < nu;
+    const int64_t e = ok ? ((int64_t)xp * nu + xq) * NP + RB * O2 + 2 * (tid & 3) : 0;
+    for (int g = 0; g < ng; g++) cp16(m.Xs + (6 * g + q) * SL + off, t.x[g] + e, ok);
   }
-  for (int e = tid; e < kVTiles * VTILE; e += RT)
-    Vs[e] = __ldg(vb + voe_tile(e / VTILE, no, nb, t, S0, S1, S2) + e % VTILE);
+  for (int c = tid; c < kVTiles * VTILE / 2; c += RT)
+    cp16(m.Vs + 2 * c, vb + voe_tile(c / (VTILE / 2), no, nb, t, S0, S1, S2) + 2 * (c % (VTILE / 2)), true);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void rows_landed() {
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 }
 
