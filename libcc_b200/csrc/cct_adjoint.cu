@@ -1008,6 +1008,31 @@ int launch_bwd_f(const BwdFArgs &a, int tiles_m, cudaStream_t s) {
 
 }  // namespace
 
+// dF GEMM split-K: about CCT_BWD_F_CTAS_PER_SM CTAs per SM for the 6 pairs of an
+// i>j>k tuple, rounded to whole k-tiles.
+static void bwd_f_split(const Dims &d, AdjBuffers *b) {
+  int sms = 148, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t nu2 = (int64_t)d.nu * d.nu;
+  const int bn = bwd_bn(d.KP);
+  const int64_t tiles = ((d.NP + BBM - 1) / BBM) * ((d.KP + bn - 1) / bn) * 6;
+  int64_t ns = (int64_t)(CCT_BWD_F_CTAS_PER_SM * sms) / tiles;
+  ns = ns < 1 ? 1 : (ns > (nu2 + BBK - 1) / BBK ? (nu2 + BBK - 1) / BBK : ns);
+  b->kchunk = round_up((nu2 + ns - 1) / ns, BBK);
+  b->nsplit = (nu2 + b->kchunk - 1) / b->kchunk;
+}
+
+int64_t adj_bytes(const Dims &d) {
+  AdjBuffers b;
+  bwd_f_split(d, &b);
+  const int64_t no = d.no, nu = d.nu, nu2 = nu * nu;
+  const int64_t inputs = 2 * nu2 * no * no + no * nu * no * no + nu * (nu + 1) / 2 * nu * no;  // their gradients
+  const int64_t work = 2 * nu2 * nu + 3 * kGXSets * nu2 * d.NP + 6 * b.nsplit * d.NP * d.KP +
+                       (9 + (nu + kAChunk - 1) / kAChunk * 6) * nu2;
+  return 8 * (no * nu2 * d.KP + no * no * d.NP * d.KP + work + inputs);
+}
+
 int adj_alloc(const Dims &d, AdjBuffers *b) {
   const int64_t no = d.no, nu = d.nu, nu2 = nu * nu, nu3 = nu2 * nu;
   auto al = [](double **p, int64_t n) -> int {
@@ -1015,19 +1040,7 @@ int adj_alloc(const Dims &d, AdjBuffers *b) {
     CCT_CUDA(cudaMalloc(reinterpret_cast<void **>(p), (size_t)(n < 1 ? 1 : n) * 8));
     return CCT_OK;
   };
-  {
-    // dF GEMM split-K: about CCT_BWD_F_CTAS_PER_SM CTAs per SM for the 6 pairs
-    // of an i>j>k tuple, rounded to whole k-tiles
-    int sms = 148, dev = 0;
-    CCT_CUDA(cudaGetDevice(&dev));
-    CCT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int bn = bwd_bn(d.KP);
-    const int64_t tiles = ((d.NP + BBM - 1) / BBM) * ((d.KP + bn - 1) / bn) * 6;
-    int64_t ns = (int64_t)(CCT_BWD_F_CTAS_PER_SM * sms) / tiles;
-    ns = ns < 1 ? 1 : (ns > (nu2 + BBK - 1) / BBK ? (nu2 + BBK - 1) / BBK : ns);
-    b->kchunk = round_up((nu2 + ns - 1) / ns, BBK);
-    b->nsplit = (nu2 + b->kchunk - 1) / b->kchunk;
-  }
+  bwd_f_split(d, b);
   CCT_TRY(al(&b->dE, no * nu2 * d.KP));
   CCT_TRY(al(&b->dF, no * no * d.NP * d.KP));
   CCT_TRY(al(&b->Wf, nu3));

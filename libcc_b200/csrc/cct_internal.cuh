@@ -280,6 +280,7 @@ struct AdjBuffers {
   double *g_eh = nullptr, *g_ep = nullptr, *g_t1 = nullptr, *g_t2 = nullptr, *g_vm = nullptr, *g_voe = nullptr,
          *g_vvvo = nullptr;                            // gradients in the input layouts
 };
+int64_t adj_bytes(const Dims &d);  // what adj_alloc takes, but for vectors
 int adj_alloc(const Dims &d, AdjBuffers *b);
 void adj_free(AdjBuffers *b);
 int adj_configure(int device);

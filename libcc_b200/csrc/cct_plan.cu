@@ -208,6 +208,9 @@ constexpr int64_t kGroupBytes = (int64_t)1536 << 20;
 // Groups of more X than this keep a ring of two instead of kNBuf (the same times
 // at no9-nu83 and up; a third less memory to allocate).
 constexpr int64_t kRing2Bytes = (int64_t)256 << 20;
+// Groups shrink where what they add to the ring would be more than this part of the
+// free memory: at most 3 GB, so from 96 GB of free memory up they never do.
+constexpr int64_t kRingShare = 32;
 int choose_group(int64_t tiles_per_tuple, int64_t xbytes_per_tuple, int64_t ntuples) {
   int64_t g = (kGroupTiles + tiles_per_tuple - 1) / tiles_per_tuple;
   g = std::min(g, std::max<int64_t>(1, kGroupBytes / xbytes_per_tuple));
@@ -776,15 +779,12 @@ int cct::plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *
   d.nb = (int)((nu + kRB - 1) / kRB);
   d.ncta = (int64_t)d.nb * (d.nb + 1) * (d.nb + 2) / 6;
   p->tuples = tuple_list((int)no);
+  size_t free_b = 0, total_b = 0;
+  const bool know_free = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
   if (!p->emulated) {
-    if (o.vvvo_mode == CCT_VVVO_PACKED) {
-      p->packed = true;
-    } else if (o.vvvo_mode == CCT_VVVO_AUTO) {
-      // packed when the expanded operand would take more than half of the free memory
-      size_t free_b = 0, total_b = 0;
-      if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
-        p->packed = (double)no * nu * nu * d.KP * 8.0 > 0.5 * (double)free_b;
-    }
+    // automatic: packed when the expanded operand would take more than half of the free memory
+    p->packed = o.vvvo_mode == CCT_VVVO_PACKED ||
+                (o.vvvo_mode == CCT_VVVO_AUTO && know_free && (double)no * nu * nu * d.KP * 8.0 > 0.5 * (double)free_b);
   }
   auto fail = [&](int s) {
     ccT_plan_destroy(p);
@@ -808,20 +808,11 @@ int cct::plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *
   if (cudaEventCreate(&p->ev0) != cudaSuccess || cudaEventCreate(&p->ev1) != cudaSuccess) return fail(CCT_ERR_CUDA);
   const int64_t nu2 = nu * nu, ntup = (int64_t)p->tuples.size();
   p->xsize = round_up(nu, kRB) * round_up(nu, kRB) * d.NP;  // blocked; rows of NP fit
-  auto set_ring = [&] {
-    const int64_t most = p->group > 1 && p->group * 3 * p->xsize * 8 > kRing2Bytes ? 2 : kNBuf;
-    p->nring = (int)std::min<int64_t>(most, (ntup + p->group - 1) / p->group);
-  };
-  {
-    const int64_t bm = p->emulated ? kEmuBM : 128, bn = p->emulated ? d.EBN : d.BN;
-    // packed plans: a group could need more slabs than the cache holds
-    p->group = p->packed ? 1
-                         : choose_group(3 * ((nu2 + bm - 1) / bm) * (d.NP / bn), 3 * p->xsize * 8, ntup);
-    p->group = std::min(p->group, group_cap);
-    set_ring();
-  }
-  for (;;) {  // smaller groups where the device has no room for the ring
-    Arena mem;
+  // every buffer of the plan, with an X ring of groups of `group` tuples
+  auto lay_out = [&](int group, Arena &mem) {
+    const int64_t most = group > 1 && group * 3 * p->xsize * 8 > kRing2Bytes ? 2 : kNBuf;
+    p->group = group;
+    p->nring = (int)std::min<int64_t>(most, (ntup + group - 1) / group);
     mem.add(&p->eh, no);
     mem.add(&p->ep, nu);
     mem.add(&p->t1, no * nu);
@@ -866,12 +857,25 @@ int cct::plan_create(ccT_plan **out, int64_t no, int64_t nu, const ccT_options *
       mem.add(&p->emu_jobs, job_offset(p, ntup));
       mem.add(&e.tileExp, e.tiles_m + no * (d.NP / d.EBN) + 2);
     }
-    s = mem.allocate(&p->arena);
-    if (s == CCT_OK) break;
-    if (s != CCT_ERR_NOMEM || p->group == 1) return fail(s);
-    cudaGetLastError();
-    p->group = (p->group + 1) / 2;
-    set_ring();
+  };
+  {
+    const int64_t bm = p->emulated ? kEmuBM : 128, bn = p->emulated ? d.EBN : d.BN;
+    // packed plans: a group could need more slabs than the cache holds
+    int group = p->packed ? 1 : choose_group(3 * ((nu2 + bm - 1) / bm) * (d.NP / bn), 3 * p->xsize * 8, ntup);
+    group = std::min(group, group_cap);
+    Arena one;
+    lay_out(1, one);
+    // What groups add to the ring of single tuples is at most kRingShare of the
+    // memory that the plan and its backward leave free: this and other plans'
+    // later allocations, and their choice of a VVVO form, then find what they would.
+    const int64_t left = (know_free ? (int64_t)free_b : 0) - (int64_t)one.bytes - (p->packed ? 0 : adj_bytes(d));
+    for (;; group = (group + 1) / 2) {
+      Arena mem;
+      lay_out(group, mem);
+      if (group > 1 && (int64_t)(mem.bytes - one.bytes) > left / kRingShare) continue;
+      if ((s = mem.allocate(&p->arena))) return fail(s);
+      break;
+    }
   }
   p->flags = reinterpret_cast<int *>(p->acc + 5 + nu * no);
   if (p->emulated) p->emu.slice_hist = reinterpret_cast<unsigned long long *>(p->acc + 5 + nu * no + 2);
