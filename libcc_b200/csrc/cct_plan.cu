@@ -477,12 +477,12 @@ int run_group(ccT_plan *p, int64_t t0, int64_t t1, bool fp64 = false, int64_t ke
   // last one leaves it (no9-nu83 2.41 -> 2.36 ms, no16-nu200 281 -> 279 ms against
   // one stream; no24-nu320 the same).  The sums of a group's partials need little
   // of an SM and run on the reduction stream under a W build.  Packed plans
-  // refill the slab cache in W-build order, and profiled launches should not
-  // overlap: one GEMM stream.
+  // refill the slab cache in W-build order: one GEMM stream.  Profiled launches
+  // go one after the other on that stream, so that each one's time is its own.
   const bool emu = p->emulated && !fp64;
   cudaStream_t gs = p->packed || p->profiling || (grp & 1) == 0 ? p->gemm_stream : p->gemm_stream2;
   if (alone) gs = p->stream;
-  cudaStream_t rs = emu || alone ? gs : p->red_stream;
+  cudaStream_t rs = emu || alone || p->profiling ? gs : p->red_stream;
   CCT_CUDA(cudaStreamWaitEvent(gs, p->ev_red[slot], 0));
   CCT_TRY(prof_mark(p, CCT_KERNEL_WBUILD, gs));
   if (keep >= 0) {
