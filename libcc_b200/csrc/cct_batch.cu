@@ -919,7 +919,6 @@ int launch_grouped(ccT_batch *b) {
   const BatchArgs a = batch_args(b);
   int nsm = 0;
   CCT_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device));
-  CCT_CUDA(cudaMemsetAsync(b->counters, 0, (size_t)b->ncounters * sizeof(int), b->stream));
   CCT_CUDA(cudaMemsetAsync(b->err, 0, sizeof(int), b->stream));
   CCT_CUDA(cudaEventRecord(b->ev_fork, b->stream));
   CCT_CUDA(cudaStreamWaitEvent(b->stream2, b->ev_fork, 0));
