@@ -30,14 +30,14 @@
 // block is one CTA on its SM, so nothing hides its copies: X lies in 8 x 8 x 8
 // blocks and a block triple's 18 blocks and its VOE tiles come as bulk copies
 // in flight together, where reading rows of X with one load a thread and element
-// took 1181 ms on 96 uneven systems (no 3-12, nu 24-140) against 954 ms.
+// took 1181 ms on 96 uneven systems (no 3-12, nu 24-140) against 955 ms.
 //
 // A second executor (mode 1) runs the same items as grouped launches: per
 // tuple group, one launch of 128-row W-build tiles (three CTAs per SM) on one
 // stream, then one launch of its reduction blocks (two CTAs per SM walking over
 // them) and one of its tuples' sums on a second stream, the ring slots
 // guarded by stream events instead of counters; the systems are summed at the
-// end.  Either forward (counter reset plus the
+// end.  Either forward (the error word's and the queue counters' reset and the
 // launches) is captured once in a CUDA graph and replayed.  The executor, the
 // W-build N tile (BN) and the tuple order are chosen by ccT_batch_tune, which
 // times every candidate on the loaded batch.
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kBT, 1) batch_kernel(const BatchArgs A) {
 }
 
 // ---- grouped executor: per tuple group, one launch of W-build tiles (128-row
-// tiles, three CTAs per SM) and one launch of reduction blocks (several CTAs per
+// tiles, three CTAs per SM) and one launch of reduction blocks (two CTAs per
 // SM); ordering between the launches comes from the stream, so no item waits.
 template <int BN>
 __global__ void __launch_bounds__(wb::NT, 3) batch_wb_kernel(const BatchArgs A, int64_t item0) {

@@ -14,9 +14,9 @@
 // keeping digit products with t+u <= S+1 (the dropped tail is below
 // 2^(-7(S+1)) of |A||B| per term).  Each D_d is an exact int32 accumulation
 // (|D_d| <= 2 S K 64^2 < 2^31 for K <= 4096).  The epilogue combines the
-// diagonals exactly in int64 (up to five of them) and enters FP64 with one
-// conversion and one power-of-two scaling per element; the sixth and
-// seventh diagonals of 6- and 7-digit launches are added in FP64.  Rounded digits leave an
+// diagonals exactly in int64 (up to six of them) and enters FP64 with one
+// conversion and one power-of-two scaling per element; the seventh diagonal
+// of a 7-digit item is added in FP64.  Rounded digits leave an
 // unbiased remainder: truncated digits (remainder of the value's own sign)
 // shrink every product the same way, and that bias adds up over the K sum,
 // the a,b,c sum and the tuples into the energy.  On seeded systems the
@@ -55,7 +55,7 @@
 // quarter of it; the tuple went from 311 to 285 us.
 //
 // Persistent kernel, one CTA of 64 + 32 NDW threads per SM (NDW = 16 drain
-// warps at 80 registers a thread: the drain is latency-bound, and 16 warps
+// warps at 96 registers a thread: the drain is latency-bound, and 16 warps
 // took a 3-digit tuple from 0.54 to 0.46 ms against 8 warps at 128
 // registers), work items (job,
 // row tile, column tile) taken round-robin with the column tile fastest, so
@@ -66,7 +66,7 @@
 //   warp 1      TMEM owner + MMA issuer (one thread): per chunk and A slice t,
 //               merged MMAs over the B slices 0..s-1-t into the s diagonal
 //               accumulators (N int32 columns each)
-//   warps 2..   drain (NDW warps): tcgen05.ld one diagonal at a time, sum in
+//   warps 2..   drain (NDW warps): tcgen05.ld two diagonals at a time, sum in
 //               int64, hand the tensor memory back to the issuer, then convert,
 //               scale and store X in 32-byte stores.  When two accumulator sets fit
 //               the tensor memory (2 S N <= 512) the issuer alternates between
@@ -375,7 +375,7 @@ __global__ void __maxnreg__(CCT_EMU_MAXNREG) wbuild_emu_kernel(const EmuArgs arg
       // Every role reads an item's job one item ahead and what the job's
       // values address one item ahead of its use, so no item starts by
       // waiting for a chain of loads (that chain, with 64-bit divisions for
-      // the item's place, took some 2 us an item in each role): CCT_EMU_ITEM
+      // the item's place, took some 2 us an item in each role)
       ItemCursor cur(args), nxt = cur;
       ItemDigits dig(args);
       EmuJob job{}, job1{};
@@ -1095,7 +1095,7 @@ int emu_build_operands(const Dims &d, const double *E, const double *F, EmuOpera
     CCT_CUDA(cudaGetLastError());
     tile_exp_top_kernel<<<1, 256, 0, s>>>((int)o->tiles_m, nbt, o->tileExp);
     CCT_CUDA(cudaGetLastError());
-    // item_slices runs S - floor(gap / 7) digits, gap = top - (ea + eb) >= 0:
+    // ItemDigits::digits gives S - floor(gap / 7) digits, gap = top - (ea + eb) >= 0:
     // all S everywhere iff no tile is all zero and the smallest pair is within 7
     std::vector<int> te((size_t)o->tiles_m + nbt + 2);
     CCT_CUDA(cudaMemcpyAsync(te.data(), o->tileExp, te.size() * sizeof(int), cudaMemcpyDeviceToHost, s));

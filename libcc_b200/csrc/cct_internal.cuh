@@ -128,7 +128,8 @@ struct TupleGroup {
   int n = 0;
   TupleDev t[kMaxGroup];
 };
-// X(p,q,s) of a blocked X buffer (the forward's; the backward reads rows of NP): block (p/8, q/8, s/8) of 512 doubles at
+// X(p,q,s) of a blocked X buffer (the forward's, unless it keeps W; the backward
+// reads rows of NP): block (p/8, q/8, s/8) of 512 doubles at
 // ((p/8) nbk + q/8) NP/8 + s/8, element ((p%8) 8 + q%8) 8 + s%8, nbk = ceil(nu/8)
 __host__ __device__ __forceinline__ int64_t xblock_base(int64_t P, int64_t Q, int64_t S, int nu, int64_t NP) {
   return ((P * ((nu + 7) / 8) + Q) * (NP / 8) + S) * 512;

@@ -55,7 +55,9 @@ struct ccT_plan {
   cudaStream_t stream = nullptr;      // stream the kernels run on
   cudaStream_t own_stream = nullptr;  // the plan's own stream (ordering, ets)
   cudaStream_t gemm_stream = nullptr; // W-build GEMMs
-  cudaStream_t gemm_stream2 = nullptr; // FP64 W builds alternate between the two, so one's tail overlaps the next's start
+  // consecutive groups' W builds alternate between the two, so one's tail overlaps
+  // the next's start; an emulated plan's backward sums its v1 on the second
+  cudaStream_t gemm_stream2 = nullptr;
   cudaStream_t red_stream = nullptr;  // reductions
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_sum = nullptr;
   cudaEvent_t ev_gemm[kNBuf] = {}, ev_red[kNBuf] = {};
