@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kXW * 32, 2)
       double v = 0.0;
 #pragma unroll
       for (int w = 0; w < kXW; w++) v += xsm[w * (kNoTile * NT * 8) + e];
-      (&ps[0][0])[e] = -v;
+      (&ps[0][0])[e] = e < no * NT * 8 ? -v : 0.0;  // (a row k >= no is 0 x O1: NaN where O1 is infinite)
     }
     __syncthreads();
   }
@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(256, 2)
     for (int n = 0; n < NT; n++)
 #pragma unroll
       for (int r = 0; r < 4; r++)
-        qz[(16 * m + g + 8 * (r >> 1)) * kNoTile + 8 * n + 2 * t + (r & 1)] = -acc[m][n][r];
+        qz[(16 * m + g + 8 * (r >> 1)) * kNoTile + 8 * n + 2 * t + (r & 1)] =
+            16 * m + g + 8 * (r >> 1) < no ? -acc[m][n][r] : 0.0;
   __syncwarp();
   double b[2 * NT][NT];
 #pragma unroll
